@@ -36,13 +36,29 @@ __device__ __forceinline__ unsigned long long warp_reserve(unsigned long long* c
 // reports overflow and the solve is repeated with a larger table.
 constexpr uint32_t kMaxProbe = 256;
 
-__device__ __forceinline__ uint32_t ht_insert(HashTable t, unsigned long long key, unsigned* ov,
+// A key, its home slot and what that slot held when the probe was begun: a
+// caller with several inserts begins them all before it finishes the first.
+struct HashProbe {
+  unsigned long long key, first;
+  uint32_t slot;
+};
+__device__ __forceinline__ HashProbe ht_probe(HashTable t, unsigned long long key) {
+  HashProbe p;
+  p.key = key;
+  p.slot = uint32_t(mix64(key)) & t.mask;
+  p.first = *reinterpret_cast<volatile unsigned long long*>(&t.keys[p.slot]);
+  return p;
+}
+
+__device__ __forceinline__ uint32_t ht_insert(HashTable t, const HashProbe& p, unsigned* ov,
                                               unsigned bit, unsigned long long* used,
                                               unsigned long long* lost, bool* fresh = nullptr) {
-  uint32_t h = uint32_t(mix64(key)) & t.mask;
+  uint32_t h = p.slot;
+  const unsigned long long key = p.key;
   const uint32_t lim = min(kMaxProbe, t.mask + 1);
   for (uint32_t i = 0; i < lim; ++i) {
-    unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&t.keys[h]);
+    const unsigned long long k =
+        i == 0 ? p.first : *reinterpret_cast<volatile unsigned long long*>(&t.keys[h]);
     if (k == key) return h;
     if (k == kEmptyKey) {
       unsigned long long old = atomicCAS(&t.keys[h], kEmptyKey, key);
@@ -58,6 +74,11 @@ __device__ __forceinline__ uint32_t ht_insert(HashTable t, unsigned long long ke
   atomicOr(ov, bit);
   atomicAdd(lost, 1ull);
   return 0xFFFFFFFFu;
+}
+__device__ __forceinline__ uint32_t ht_insert(HashTable t, unsigned long long key, unsigned* ov,
+                                              unsigned bit, unsigned long long* used,
+                                              unsigned long long* lost, bool* fresh = nullptr) {
+  return ht_insert(t, ht_probe(t, key), ov, bit, used, lost, fresh);
 }
 
 // Find or claim key's slot in a table that may fill up: the slot, or

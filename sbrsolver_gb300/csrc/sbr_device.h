@@ -57,16 +57,7 @@ constexpr int kEmptyChild = INT_MIN;
 struct RefNode {
   double bb[6];
   float fb[6];
-  int c0, c1, first, count, parent, flat;
-};
-
-// One box on a reference leaf's path to the root (leaf first), stored
-// contiguously per leaf so the reachability check of a hit reads one run
-// instead of chasing parent links.  node < 0 ends a leaf's run.
-struct __align__(16) AncBox {
-  float fb[6];
-  int flat;  // RefNode::flat
-  int node;  // RefNode index (its FP64 box decides cases the FP32 test cannot)
+  int flat, c0, c1, first, count, parent;
 };
 
 // Triangle, depth-first leaf order (index == closest-hit tie rank).
@@ -106,10 +97,9 @@ struct DevScene {
   const Node4* snode4;
   const Tri32* stri;    // triangles in search leaf order
   const int* srank;     // their depth-first ranks
-  const AncBox* anc;    // per reference leaf: its boxes up to the root
-  const int* anc_off;   // start of a leaf's run in anc (by node index)
   int n_tri, n_nodes, n_mats;
   int root_leaf;
+  int soft;          // every triangle is in soft64's range
   float box_margin;  // absolute FP32 box expansion (metres)
 };
 
@@ -130,9 +120,8 @@ struct __align__(16) RayRec {
 
 // FP32 copy of a ray, made by the candidate search when it loads the ray
 // (it converts the FP64 origin and direction anyway), for the FP32 checks and
-// the node record of the ray's resolution, which then convert nothing (an
-// FP64 -> FP32 conversion costs an FP64 pipe slot): origin (o.w unused) and
-// unit direction (d.w unused).
+// the node record of the ray's resolution, which then convert nothing: origin
+// (o.w unused) and unit direction (d.w unused).
 struct __align__(16) RayF32 {
   float4 o, d;
 };

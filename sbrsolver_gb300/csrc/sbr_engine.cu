@@ -244,7 +244,7 @@ struct Workspace {
 struct Tuning {
   int find_steps = 0, find_refill = 0, find_bps = 0, trace_bps = 0, capture_bps = 0;
   int chunk_log2 = 0;
-  int trace_kernel = 0;  // FP64 resolution: 1 = k_trace (a ray per lane), 2 = k_trace_pool
+  int trace_kernel = 0;  // FP64 resolution: 1 or 2, both k_trace
   int graph = 0;         // pipeline as a CUDA graph on repeat: 1 (0 = default), -1 = never
   int find_tris = 0;     // FP32 search: leaf triangles per step, 1 or 2 (0 = default)
 };
@@ -279,8 +279,6 @@ struct SceneImpl {
   DBuf<Node4> snode4;
   DBuf<Tri32> stri;
   DBuf<int> srank;
-  DBuf<AncBox> anc;
-  DBuf<int> anc_off;
   DBuf<CorrTri> corr;
   DBuf<Tri32> corr32;
   DBuf<Material> mats;
@@ -399,7 +397,9 @@ static void upload_scene(SceneImpl& S) {
   std::vector<Tri32> t32(nt);
   std::vector<Tri64> t64(nt);
   std::vector<int> cop(nt), r2i(nt);
+  std::atomic<bool> soft{true};
   host_parallel(size_t(nt), [&](size_t b, size_t e) {
+    bool ok = true;
     for (int r = int(b); r < int(e); ++r) {
       const HostTri& t = H.tris[H.dfs_tris[r]];
       Tri64& d = t64[r];
@@ -412,6 +412,8 @@ static void upload_scene(SceneImpl& S) {
         f.v1[a] = float(d.v1[a]);
         f.e1[a] = float(d.e1[a]);
         f.e2[a] = float(d.e2[a]);
+        ok &= soft64::safe(d.v1[a]) && soft64::safe(d.e1[a]) && soft64::safe(d.e2[a]) &&
+              soft64::safe(d.n[a]);
       }
       f.nv1 = float(std::sqrt(d.v1[0] * d.v1[0] + d.v1[1] * d.v1[1] + d.v1[2] * d.v1[2])) * 1.0001f;
       f.ne1 = float(std::sqrt(d.e1[0] * d.e1[0] + d.e1[1] * d.e1[1] + d.e1[2] * d.e1[2])) * 1.0001f;
@@ -423,6 +425,7 @@ static void upload_scene(SceneImpl& S) {
       cop[r] = t.cop;
       r2i[r] = t.id;
     }
+    if (!ok) soft = false;
   });
   host_parallel(size_t(nn), [&](size_t b, size_t e) {
     for (int i = int(b); i < int(e); ++i)
@@ -517,26 +520,6 @@ static void upload_scene(SceneImpl& S) {
     S.dev.srank = S.srank.p;
     CK(cudaStreamSynchronize(st));  // the host vectors above go out of scope
   }
-  {  // every reference leaf's boxes up to the root, one run per leaf
-    // (the leaf, its ancestors to the root, then an end marker), written on
-    // the device from the reference nodes uploaded above
-    std::vector<int> off(nn, -1);
-    size_t total = 0;
-    for (int i = 0; i < nn; ++i) {
-      if (H.nodes[i].c0 >= 0) continue;
-      off[i] = int(total);
-      total += size_t(H.nodes[i].depth) + 2;
-    }
-    if (total > size_t(INT_MAX)) throw std::string("reference BVH too deep for the ancestor table");
-    S.anc.ensure(std::max<size_t>(1, total));
-    S.anc_off.upload(off.data(), off.size(), st);
-    prep::k_anc_fill<<<std::max(1, std::min(4096, (nn + 255) / 256)), 256, 0, st>>>(
-        S.ref.p, nn, S.anc_off.p, S.anc.p);
-    CK(cudaGetLastError());
-    S.dev.anc = S.anc.p;
-    S.dev.anc_off = S.anc_off.p;
-    CK(cudaStreamSynchronize(st));
-  }
   S.tri_cop.upload(cop.data(), cop.size(), st);
   S.rank_to_id.upload(r2i.data(), r2i.size(), st);
   S.dev.node32 = S.node32.p;
@@ -549,13 +532,13 @@ static void upload_scene(SceneImpl& S) {
   S.dev.n_nodes = nn;
   S.dev.n_mats = int(mats.size());
   S.dev.root_leaf = H.nodes[0].c0 < 0 ? 1 : 0;
+  S.dev.soft = soft.load() ? 1 : 0;
   S.dev.box_margin = float(margin_m);
   S.dev_bytes = (long long)(n32.size() * sizeof(Node32) + ref.size() * sizeof(RefNode) +
                             t32.size() * sizeof(Tri32) + t64.size() * sizeof(Tri64) +
                             2 * nt * sizeof(int) + nt * sizeof(CorrTri) +
                             S.snode4.n * sizeof(Node4) + S.stri.n * sizeof(Tri32) +
-                            S.srank.n * sizeof(int) + S.anc.n * sizeof(AncBox) +
-                            S.anc_off.n * sizeof(int));
+                            S.srank.n * sizeof(int));
   CK(cudaStreamSynchronize(st));
 }
 
@@ -694,17 +677,6 @@ static int trace_fit() {
   static const int per_sm = blocks_per_sm(k_trace, 128);
   return per_sm;
 }
-// k_trace_pool keeps its rays in dynamic shared memory (one PoolSlots per warp).
-constexpr size_t kPoolSmem = sizeof(PoolSlots) * kPoolWarps;
-static int pool_fit() {
-  static const int per_sm = [] {
-    cudaFuncSetAttribute(k_trace_pool, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPoolSmem));
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_trace_pool, 32 * kPoolWarps, kPoolSmem);
-    return std::max(1, n);
-  }();
-  return per_sm;
-}
 static int capture_fit() {
   static const int per_sm = blocks_per_sm(k_capture_fast, 32 * kCapWarps);
   return per_sm;
@@ -719,8 +691,6 @@ static int trace_grid(const Tuning& t) { return persistent_grid(trace_fit(), t.t
 // Capture: the work counter balances the blocks.
 static int capture_grid(const Tuning& t) { return persistent_grid(capture_fit(), t.capture_bps); }
 
-// The FP64 resolution kernel solves use unless tuned otherwise.
-constexpr int kDefaultTraceKernel = 1;
 constexpr int kFindTris = 2;  // leaf triangles per FP32 search step
 // Rays per search/resolution launch pair: 2^25 holds a level-9 launch's
 // widest depth at six reflections and one transmission (7 rays per launch)
@@ -737,7 +707,7 @@ static Tuning resolved(Tuning t) {
   t.capture_bps = t.capture_bps > 0 ? std::min(t.capture_bps, capture_fit()) : capture_fit();
   if (t.chunk_log2 <= 0) t.chunk_log2 = kTraceChunkLog2;
   t.chunk_log2 = std::min(std::max(t.chunk_log2, 16), 26);
-  if (t.trace_kernel <= 0 || t.trace_kernel > 2) t.trace_kernel = kDefaultTraceKernel;
+  if (t.trace_kernel <= 0 || t.trace_kernel > 2) t.trace_kernel = 1;
   t.graph = t.graph < 0 ? -1 : 1;
   if (t.find_tris <= 0 || t.find_tris > 2) t.find_tris = kFindTris;
   return t;
@@ -1598,7 +1568,6 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       }
     }
     (void)resolved(tu);  // the occupancy queries run before any recording
-    (void)pool_fit();
     // ---- the device pipeline: a fixed sequence of stream operations
     const long long nl_before = nl;
     size_t n_tr = 0;  // k_trace launches (timed one by one)
@@ -1717,15 +1686,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
         CK(cudaMemsetAsync(W.find_work.p, 0, 2 * sizeof(unsigned long long), st));
         ++nl, k_find<<<find_grid(tu), 128, 0, st>>>(fnd);
         mark(W.tr_ev[2 * n_tr]);
-        if (resolved(tu).trace_kernel == 2) {
-          // one block per 128 rays at most, as k_trace: a small launch still
-          // spreads over many warps (each then fills only part of its slots)
-          const long long need = (ta.hi - lo + 127) / 128;
-          const int grid = int(std::min<long long>(device_sms() * pool_fit(), std::max(1LL, need)));
-          ++nl, k_trace_pool<<<grid, 32 * kPoolWarps, kPoolSmem, st>>>(ta);
-        } else {
-          ++nl, k_trace<<<std::min<long long>(trace_grid(tu), (ta.hi - lo + 127) / 128), 128, 0, st>>>(ta);
-        }
+        ++nl, k_trace<<<std::min<long long>(trace_grid(tu), (ta.hi - lo + 127) / 128), 128, 0, st>>>(ta);
         mark(W.tr_ev[2 * n_tr + 1]);
         ++n_tr;
       }
@@ -2692,23 +2653,21 @@ sbr_status sbr_autotune(sbr_scene* scene, const sbr_request* requests, int n_req
     return v;
   };
   const std::vector<int> steps{8, 16, 32, 64, 128}, refill{4, 8, 16, 24, 32},
-      chunk{20, 22, 24, 25, 26},
-      kernels{1, 2}, tris{1, 2};
+      chunk{20, 22, 24, 25, 26}, tris{1, 2};
   for (int round = 0; round < rounds; ++round) {
     bool moved = false;
-    for (int p = 0; p < 8; ++p) {
-      const std::vector<int> cand = p == 0   ? kernels
-                                    : p == 1 ? steps
-                                    : p == 2 ? refill
-                                    : p == 3 ? span(ff)
-                                    : p == 4 ? span(tf)
-                                    : p == 5 ? span(cf)
-                                    : p == 6 ? chunk
+    for (int p = 0; p < 7; ++p) {
+      const std::vector<int> cand = p == 0   ? steps
+                                    : p == 1 ? refill
+                                    : p == 2 ? span(ff)
+                                    : p == 3 ? span(tf)
+                                    : p == 4 ? span(cf)
+                                    : p == 5 ? chunk
                                              : tris;
       for (int v : cand) {
         Tuning t = cur;
-        int* f[8] = {&t.trace_kernel, &t.find_steps, &t.find_refill, &t.find_bps, &t.trace_bps,
-                     &t.capture_bps, &t.chunk_log2, &t.find_tris};
+        int* f[7] = {&t.find_steps,  &t.find_refill, &t.find_bps, &t.trace_bps,
+                     &t.capture_bps, &t.chunk_log2,  &t.find_tris};
         if (*f[p] == v) continue;
         *f[p] = v;
         if ((st = time_of(t, ms)) != SBR_OK) return st;

@@ -8,12 +8,27 @@
 #include <cuda_runtime.h>
 
 #include "sbr_device.h"
+#include "sbr_soft64.cuh"
 
 namespace sbr {
 
 constexpr double kEps64 = 1.1920928955078125e-07;  // FLT_EPSILON as double, Constants.h:13
 constexpr float kEps32 = 1.1920928955078125e-07f;
-constexpr float kFiltK = 6.103515625e-05f;         // 2^-14: FP32 filter margin factor
+// FP32 filter margin factor of the triangle tests, 2^-18: with unit roundoff
+// e = 2^-24, the rounded inputs (2e per product) and the rounding of each
+// operation give |dh| <= 7e |d||e2| for h = d x e2, |ds| <= 2e (|o| + |v1|) for
+// s = o - v1, hence errors under 11e |e1||e2||d| of a = e1 . h, 12e of
+// U = s . h, and with |dq| <= 9e for q = s x e1, 13e of V = d . q and
+// W = e2 . q, each relative to the magnitudes the margins are formed from.
+// 64e leaves a factor of four and more.  The factor was 2^-14 before: the
+// level-10 terrain solve then left 14 % of its contenders to FP64 for their
+// edges (now 2 %) and sent 8,738 rays with more than eight contenders to the
+// one-pass search (now 15).
+constexpr float kFiltK = 3.814697265625e-06f;
+// The image correction's filters keep 2^-14: their direction is the
+// difference of two rounded points, with an error relative to the points.
+constexpr float kCorrK = 6.103515625e-05f;
+constexpr float kBoxK = 6.103515625e-05f;  // 2^-14 |origin|: FP32 box expansion
 // Margin factor of the FP32 reception test: |dist - radius| and the
 // projection are decided in FP32 only when they clear this times the
 // magnitudes involved (|segment start| + |receiver| + 1 + unfolded length).
@@ -40,35 +55,82 @@ struct Hit {
   int leaf;
 };
 
-// Triangle::RayIntersects (Triangle.cpp:80-124), FP64, reference operation order.
-__device__ __forceinline__ bool mt64(const Tri64& T, const double* o, const double* d, double& t,
-                                     double* P, double& dist) {
-  using namespace x64;
-  double h[3];
-  cross(d, T.e2, h);
-  const double a = dot(T.e1, h);
-  if (a > -kEps64 && a < kEps64) return false;
+// Products, quotients and roots of the FP64 tests: on the FP64 pipe, or in
+// integer arithmetic (sbr_soft64.cuh; the same bits for operands in its range).
+struct Pipe64 {
+  static __device__ __forceinline__ double mul(double a, double b) { return x64::mul(a, b); }
   // 1.0 / a (Triangle.cpp): the correctly rounded reciprocal is the same
   // double as the correctly rounded quotient 1.0 / a
-  const double f = __drcp_rn(a);
-  double s[3];
-  sub3(o, T.v1, s);
-  const double u = mul(f, dot(s, h));
-  if (u < 0.0 || u > 1.0) return false;
-  double q[3];
-  cross(s, T.e1, q);
-  const double v = mul(f, dot(d, q));
-  if (v < 0.0 || add(u, v) > 1.0) return false;
-  const double tt = mul(f, dot(T.e2, q));
-  if (!(tt > kEps64)) return false;
-  P[0] = add(o[0], mul(d[0], tt));
-  P[1] = add(o[1], mul(d[1], tt));
-  P[2] = add(o[2], mul(d[2], tt));
+  static __device__ __forceinline__ double rcp(double a) { return __drcp_rn(a); }
+  static __device__ __forceinline__ double sqrt(double a) { return x64::sqrt_(a); }
+};
+struct Soft64 {
+  static __device__ __forceinline__ double mul(double a, double b) { return soft64::mul(a, b); }
+  static __device__ __forceinline__ double rcp(double a) { return soft64::rcp(a); }
+  static __device__ __forceinline__ double sqrt(double a) { return soft64::sqrt(a); }
+};
+template <class A>
+__device__ __forceinline__ double dot64(const double* a, const double* b) {
+  return x64::add(x64::add(A::mul(a[0], b[0]), A::mul(a[1], b[1])), A::mul(a[2], b[2]));
+}
+template <class A>
+__device__ __forceinline__ void cross64(const double* a, const double* b, double* r) {
+  r[0] = x64::sub(A::mul(a[1], b[2]), A::mul(a[2], b[1]));
+  r[1] = x64::sub(A::mul(a[2], b[0]), A::mul(a[0], b[2]));
+  r[2] = x64::sub(A::mul(a[0], b[1]), A::mul(a[1], b[0]));
+}
+
+// Triangle::RayIntersects (Triangle.cpp:80-124), FP64, reference operation
+// order.  uv_sure: the FP32 filter has shown that the reference's tests of u
+// and v accept (tri_classify), so they are not formed.  No early exit: a lane
+// that fails costs its warp nothing more, and the warp stays together.
+// Comparisons are integer ones, which decide alike without the FP64 pipe.
+template <class A>
+__device__ __forceinline__ bool mt64_t(const Tri64& T, const double* o, const double* d,
+                                       bool uv_sure, double& t, double* P, double& dist) {
+  using x64::add;
+  double h[3], s[3], q[3];
+  cross64<A>(d, T.e2, h);
+  const double a = dot64<A>(T.e1, h);
+  if (soft64::magnitude_below(a, kEps64)) return false;
+  const double f = A::rcp(a);
+  x64::sub3(o, T.v1, s);
+  cross64<A>(s, T.e1, q);
+  if (!uv_sure) {
+    const double u = A::mul(f, dot64<A>(s, h));
+    const double v = A::mul(f, dot64<A>(d, q));
+    if (soft64::negative(u) || soft64::above(u, 1.0) || soft64::negative(v) ||
+        soft64::above(add(u, v), 1.0))
+      return false;
+  }
+  const double tt = A::mul(f, dot64<A>(T.e2, q));
+  if (!soft64::above(tt, kEps64)) return false;
+  P[0] = add(o[0], A::mul(d[0], tt));
+  P[1] = add(o[1], A::mul(d[1], tt));
+  P[2] = add(o[2], A::mul(d[2], tt));
   double w[3];
-  sub3(P, o, w);
-  dist = norm(w);
+  x64::sub3(P, o, w);
+  dist = A::sqrt(dot64<A>(w, w));
   t = tt;
   return true;
+}
+__device__ __forceinline__ bool mt64(const Tri64& T, const double* o, const double* d, double& t,
+                                     double* P, double& dist) {
+  return mt64_t<Pipe64>(T, o, d, false, t, P, dist);
+}
+
+// mt64 out of line, for the rare ray outside soft64's range: the arguments go
+// by value, so the caller's ray stays in registers.
+struct Mt64Result {
+  bool ok;
+  double t, dist, p[3];
+};
+__device__ __noinline__ Mt64Result mt64_call(const Tri64* T, double ox, double oy, double oz,
+                                             double dx, double dy, double dz) {
+  const double o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+  Mt64Result r;
+  r.ok = mt64(*T, o, d, r.t, r.p, r.dist);
+  return r;
 }
 
 // Same test on a CorrTri (image correction looks triangles up by mesh position).
@@ -158,10 +220,10 @@ __device__ __forceinline__ bool tri_filter(const Tri32& T, const float3& o, cons
   float V = d.x * qx + d.y * qy + d.z * qz;
   float W = T.e2[0] * qx + T.e2[1] * qy + T.e2[2] * qz;
   const float ns = no + T.nv1;
-  const float ea = kFiltK * T.ne1 * T.ne2 * nd;
-  const float eU = kFiltK * ns * nd * T.ne2;
-  const float eV = kFiltK * ns * T.ne1 * nd;
-  const float eW = kFiltK * ns * T.ne1 * T.ne2;
+  const float ea = kCorrK * T.ne1 * T.ne2 * nd;
+  const float eU = kCorrK * ns * nd * T.ne2;
+  const float eV = kCorrK * ns * T.ne1 * nd;
+  const float eW = kCorrK * ns * T.ne1 * T.ne2;
   const float A = fabsf(a);
   if (A <= kEps32 + ea) {  // near-parallel: the FP64 test decides
     tlo = 0.0f;
@@ -213,10 +275,10 @@ __device__ __forceinline__ bool tri_filter_from(const Tri32& T, const TriFrom& F
   float U = F.sx * hx + F.sy * hy + F.sz * hz;
   float V = d.x * F.qx + d.y * F.qy + d.z * F.qz;
   float W = F.W;
-  const float ea = kFiltK * T.ne1 * T.ne2 * nd;
-  const float eU = kFiltK * F.ns * nd * T.ne2;
-  const float eV = kFiltK * F.ns * T.ne1 * nd;
-  const float eW = kFiltK * F.ns * T.ne1 * T.ne2;
+  const float ea = kCorrK * T.ne1 * T.ne2 * nd;
+  const float eU = kCorrK * F.ns * nd * T.ne2;
+  const float eV = kCorrK * F.ns * T.ne1 * nd;
+  const float eW = kCorrK * F.ns * T.ne1 * T.ne2;
   const float A = fabsf(a);
   if (A <= kEps32 + ea) return true;  // near-parallel: the FP64 test decides
   if (a < 0.0f) {
@@ -231,8 +293,10 @@ __device__ __forceinline__ bool tri_filter_from(const Tri32& T, const TriFrom& F
   return W + eW > (kEps32 * 0.5f) * (A - ea);
 }
 
-// As tri_filter, also telling whether the FP64 test certainly hits (2) or
-// may go either way (1); 0 = certainly misses.  [tlo, thi] bounds t.
+// As tri_filter, also telling what the FP64 test certainly decides: 0 = it
+// misses, else kMayHit, with kSureUV when its tests of u and v accept and
+// kSureHit when it hits.  [tlo, thi] bounds t.
+constexpr int kMayHit = 1, kSureHit = 2, kSureUV = 4;
 __device__ __forceinline__ int tri_classify(const Tri32& T, const float3& o, const float3& d,
                                             float no, float nd, float& tlo, float& thi) {
   const float hx = d.y * T.e2[2] - d.z * T.e2[1];
@@ -255,7 +319,7 @@ __device__ __forceinline__ int tri_classify(const Tri32& T, const float3& o, con
   if (A <= kEps32 + ea) {
     tlo = 0.0f;
     thi = INFINITY;
-    return 1;
+    return kMayHit;
   }
   if (a < 0.0f) {
     U = -U;
@@ -268,8 +332,8 @@ __device__ __forceinline__ int tri_classify(const Tri32& T, const float3& o, con
   thi = (W + eW) / (A - ea);
   if (thi <= kEps32 * 0.5f) return 0;
   tlo = (W - eW) / (A + ea);
-  const bool sure = U > eU && V > eV && U + V < A - ea - eU - eV && tlo > 2.0f * kEps32;
-  return sure ? 2 : 1;
+  const bool uv = U > eU && V > eV && U + V < A - ea - eU - eV;
+  return kMayHit | (uv ? (tlo > 2.0f * kEps32 ? kSureUV | kSureHit : kSureUV) : 0);
 }
 
 __device__ __forceinline__ void load_node(const Node32* nodes, int i, float4& f0, float4& f1,
@@ -306,8 +370,10 @@ struct TraceStats {
 // planes, so the FP64 test accepts iff the other axes' intervals contain it.
 // inv = 1/d in FP32: a product with it differs from the quotient by a few
 // ulps, far inside e.
+// zeros: axes whose direction component is exactly 0 and whose planes lie on
+// either side of the origin; their FP64 interval is everything.
 __device__ __forceinline__ int slab_certain(const float* bb, int flatmask, const float3& o,
-                                            const float3& d, const float3& inv) {
+                                            const float3& d, const float3& inv, int zeros) {
   const float K = 9.5367431640625e-07f;  // 2^-20
   float A_lo = -INFINITY, A_hi = -INFINITY, B_lo = INFINITY, B_hi = INFINITY;
   float v = 0.0f, ev = 0.0f;
@@ -318,6 +384,7 @@ __device__ __forceinline__ int slab_certain(const float* bb, int flatmask, const
     const float da = a == 0 ? d.x : (a == 1 ? d.y : d.z);
     const float oa = a == 0 ? o.x : (a == 1 ? o.y : o.z);
     const float ia = a == 0 ? inv.x : (a == 1 ? inv.y : inv.z);
+    if (zeros >> a & 1) continue;
     if (da == 0.0f) return -1;
     const float lo = bb[a], hi = bb[3 + a];
     const float t1 = (lo - oa) * ia, t2 = (hi - oa) * ia;
@@ -345,13 +412,71 @@ __device__ __forceinline__ int slab_certain(const float* bb, int flatmask, const
   return -1;
 }
 
+// Whether every box from `leaf` up to the root of the reference BVH passes the
+// reference's slab test, i.e. whether the reference's traversal reaches the
+// leaf.  An ancestor's box contains the leaf's, and FP64 subtraction and
+// division by one direction component are monotone, so each of the ancestor's
+// slab intervals contains the leaf's exactly as computed, and the leaf's own
+// test decides for the whole chain.  A zero component gives an infinite
+// interval for every box whose planes lie on either side of the origin, the
+// ancestors' with the leaf's; only where a plane of the leaf goes through the
+// origin or past it (0 / 0, which the reference's min/max ignore) is the chain
+// walked.  The leaf's test is FP32 with error bounds (slab_certain), FP64
+// inside them.  Walking the chain for every hit (about 10 boxes in the urban
+// canyon, 16 on the terrain) cost the level-9 canyon solve 0.35 ms, and the
+// FP64 walk for the 0.3 % of its rays with a zero component, which held their
+// whole warp through 600 FP64 instructions, another 2.3 ms (level-7 plan: 0.37
+// of 0.60 ms).
+__device__ __forceinline__ bool zero64(double x) {
+  return (__double_as_longlong(x) << 1) == 0;
+}
+// slab64 out of line (see mt64_call).
+__device__ __noinline__ bool slab_call(const double* bb, double ox, double oy, double oz, double dx,
+                                       double dy, double dz) {
+  const double o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+  return slab64(bb, o, d);
+}
+__device__ __forceinline__ bool leaf_reachable(const DevScene& sc, int leaf, const double* o,
+                                               const double* d, const float3& o32,
+                                               const float3& d32, const float3& inv) {
+  const RefNode& L = sc.ref[leaf];
+  int zeros = 0;
+  bool beside = false;  // a zero component, and the origin not strictly between the planes
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    if (zero64(d[a])) {
+      // fb holds the planes exactly and rounding is monotone, so a rounded
+      // origin strictly between them comes from one that is
+      const float oa = a == 0 ? o32.x : (a == 1 ? o32.y : o32.z);
+      zeros |= 1 << a;
+      beside |= (L.flat & 8) || !(oa > L.fb[a] && oa < L.fb[3 + a]);
+    }
+  if (beside) {
+    for (int n = leaf; n >= 0; n = sc.ref[n].parent)
+      if (!slab_call(sc.ref[n].bb, o[0], o[1], o[2], d[0], d[1], d[2])) return false;
+    return true;
+  }
+  const int v = slab_certain(L.fb, L.flat, o32, d32, inv, zeros);
+  return v < 0 ? slab_call(L.bb, o[0], o[1], o[2], d[0], d[1], d[2]) : v != 0;
+}
+
+// exact_closest for k_trace, out of line: the ray and the hit go by value (see
+// mt64_call).
+__device__ __noinline__ Hit exact_call(const DevScene& sc, double ox, double oy, double oz,
+                                       double dx, double dy, double dz, unsigned* overflow) {
+  const double o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+  Hit best;
+  if (!exact_closest(sc, o, d, best, overflow)) best.rank = INT_MAX;
+  return best;
+}
+
 // Closest hit with the reference's result.  FP32 ordered traversal over the
 // reference BVH (boxes widened by box_margin so no box the FP64 test accepts
 // is missed), FP32 triangle filter, FP64 test for every triangle the filter
 // cannot rule out, lexicographic (distance, depth-first rank) minimum - the
-// reference's strict '<' in visit order.  The winner is accepted only if every
-// ancestor box of its leaf passes the reference's FP64 slab test; otherwise
-// the ray is re-run with the reference-order traversal.
+// reference's strict '<' in visit order.  The winner is accepted only if the
+// reference's slab tests reach its leaf; otherwise the ray is re-run with the
+// reference-order traversal.
 __device__ __noinline__ bool closest_hit(const DevScene& sc, const double* o, const double* d,
                                          Hit& best, TraceStats& st, unsigned* overflow) {
   const float3 o32 = make_float3(float(o[0]), float(o[1]), float(o[2]));
@@ -359,7 +484,7 @@ __device__ __noinline__ bool closest_hit(const DevScene& sc, const double* o, co
   const float3 inv = make_float3(1.0f / d32.x, 1.0f / d32.y, 1.0f / d32.z);
   const float no = sqrtf(o32.x * o32.x + o32.y * o32.y + o32.z * o32.z);
   const float nd = sqrtf(d32.x * d32.x + d32.y * d32.y + d32.z * d32.z);
-  const float m = sc.box_margin + kFiltK * no;
+  const float m = sc.box_margin + kBoxK * no;
   best.rank = INT_MAX;
   best.dist = __longlong_as_double(0x7ff0000000000000ll);
   best.t = best.dist;
@@ -388,7 +513,7 @@ __device__ __noinline__ bool closest_hit(const DevScene& sc, const double* o, co
           cand_leaf[ncand] = pending_leaf;
           cand_t[ncand] = tlo;
           ++ncand;
-          if (k == 2) tcut = fminf(tcut, thi * (1.0f + kTieSlack) + 1e-30f);
+          if (k & kSureHit) tcut = fminf(tcut, thi * (1.0f + kTieSlack) + 1e-30f);
         } else {
           // too many contenders: resolve this one now
           ++st.fp64_tri;
@@ -492,23 +617,24 @@ __device__ __noinline__ bool closest_hit(const DevScene& sc, const double* o, co
       best.leaf = cand_leaf[i];
     }
   }
-  bool ok = !stack_overflow;
-  if (ok && best.rank != INT_MAX) {
-    // every ancestor of the winner's leaf must pass the FP64 slab test
-    for (int n = best.leaf; n >= 0; n = sc.ref[n].parent) {
-      int v = slab_certain(sc.ref[n].fb, sc.ref[n].flat, o32, d32, inv);
-      if (v < 0) v = slab64(sc.ref[n].bb, o, d) ? 1 : 0;
-      if (!v) {
-        ok = false;
-        break;
-      }
-    }
-  }
-  if (!ok) {
+  if (stack_overflow ||
+      (best.rank != INT_MAX && !leaf_reachable(sc, best.leaf, o, d, o32, d32, inv))) {
     ++st.fallback;
     return exact_closest(sc, o, d, best, overflow);
   }
   return best.rank != INT_MAX;
+}
+
+// closest_hit for k_trace, likewise.
+__device__ __noinline__ Hit closest_call(const DevScene& sc, double ox, double oy, double oz,
+                                         double dx, double dy, double dz, Counters* ctr) {
+  const double o[3] = {ox, oy, oz}, d[3] = {dx, dy, dz};
+  Hit best;
+  TraceStats st{0, 0};
+  if (!closest_hit(sc, o, d, best, st, &ctr->overflow)) best.rank = INT_MAX;
+  if (st.fp64_tri) atomicAdd(&ctr->fp64_tri, (unsigned long long)st.fp64_tri);
+  if (st.fallback) atomicAdd(&ctr->fallback, (unsigned long long)st.fallback);
+  return best;
 }
 
 // ---- split closest hit: FP32 candidate search, then FP64 resolution -------
@@ -521,6 +647,10 @@ __device__ __noinline__ bool closest_hit(const DevScene& sc, const double* o, co
 // reference-order FP64 traversal.
 constexpr int kCand = 8;
 constexpr unsigned char kFindFallback = 0xFF;
+// ncand of a ray: its contenders (0..kCand), with kCandUnsafe if its origin or
+// direction is outside soft64's range; kFindFallback as a whole.
+constexpr int kCandCount = 0x0F, kCandUnsafe = 0x40;
+constexpr unsigned kContUV = 0x80000000u;  // contender's rank: u and v are sure (kSureUV)
 
 // Whether the reference's test of the triangle a ray starts on certainly
 // fails (so its FP64 test can be skipped).  The ray's origin is the hit

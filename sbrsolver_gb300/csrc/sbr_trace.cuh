@@ -145,10 +145,43 @@ __device__ __forceinline__ void write_class(ClassInfo& ci, const double* img, ui
   ci.pad2 = 0;
 }
 
+// Records of the freshly interned class `cls`: reached from class `parent` by
+// an interaction of `kind` on the triangle of depth-first rank `rank`.  A
+// reflection's image source is ImagePoint (RTSolver.cpp:910-924) of the
+// parent's (the transmitter for a launch) across the triangle the reference
+// finds at this id's position of its mesh vector; a transmission keeps it.
+__device__ __noinline__ void intern_class(const TraceArgs& A, uint32_t cls, uint32_t parent,
+                                          const double* tx, int rank, uint32_t cop, int kind) {
+  const double* pimg = is_root_class(parent) ? tx : A.cls_info[parent].img;
+  const int mpos = A.sc.rank_to_id[rank];
+  double img[3] = {pimg[0], pimg[1], pimg[2]};
+  if (kind == 1) {
+    const CorrTri& M = A.sc.corr[mpos];
+    double w[3];
+    x64::sub3(pimg, M.v1, w);
+    const double dist = x64::dot(M.n, w);
+    for (int a = 0; a < 3; ++a)
+      img[a] = x64::sub(pimg[a], x64::mul(x64::mul(2.0, dist), M.n[a]));
+  }
+  write_class(A.cls_info[cls], img, parent, rank, cop, kind, A.depth + 1);
+  write_class_cap(A.sc, img, mpos, A.cls_cap[cls]);
+  list_class(A, cls);
+}
+
 // Number of rays entering bounce depth `depth` (known on the device only).
 __device__ __forceinline__ long long rays_at_depth(const Counters* ctr, int depth, long long n_root,
                                                    unsigned long long cap) {
   return depth == 0 ? n_root : (long long)min(ctr->queue[depth], cap);
+}
+
+// Index of the first node of bounce depth `depth`: every ray makes one tree
+// node, and ray i of a depth makes node node_base + i, so no counter hands
+// the nodes out and the records are written in ray order.
+__device__ __forceinline__ unsigned long long node_base(const Counters* ctr, int depth,
+                                                        long long n_root, unsigned long long cap) {
+  unsigned long long b = 0;
+  for (int d = 0; d < depth; ++d) b += (unsigned long long)rays_at_depth(ctr, d, n_root, cap);
+  return b;
 }
 
 // Launch ray g of the batch: origin and direction (FP64).
@@ -161,6 +194,22 @@ __device__ __forceinline__ void root_ray(const TxParams* txp, int n_tx, const do
   for (int a = 0; a < 3; ++a) {
     o[a] = P.tx[a];
     d[a] = dd[a];
+  }
+}
+
+// Origin and direction of ray i of bounce depth `depth`.
+__device__ __forceinline__ void load_ray_line(const TxParams* txp, int n_tx,
+                                              const double* const* dirs, const RayRec* in,
+                                              int depth, long long i, double* o, double* d) {
+  if (depth == 0) {
+    int q;
+    long long li;
+    root_ray(txp, n_tx, dirs, i, o, d, q, li);
+  } else {
+    for (int a = 0; a < 3; ++a) {
+      o[a] = in[i].o[a];
+      d[a] = in[i].d[a];
+    }
   }
 }
 
@@ -186,40 +235,31 @@ __device__ __forceinline__ void load_ray(const TxParams* txp, int n_tx, const do
   }
 }
 
-// The tree node of a resolved ray (RTSolver.cpp:142-257): its record (hot
-// FP32 part and cold FP64 part), the segment counted for its request.  A
-// ray that hits nothing ends at src + 1e10 d (a launch) or src + 100 d
-// (RTSolver.cpp:231,249).  Returns the node index.
-__device__ __forceinline__ unsigned long long emit_node(NodeHot* nodes, NodeCold* cold,
-                                                        unsigned long long cap, Counters* ctr,
-                                                        unsigned long long* seg_per_tx,
-                                                        const RayRec& r, bool root,
-                                                        const float3& o32, const float3& d32,
-                                                        bool hit, const Hit& h) {
-  const unsigned long long ni = warp_reserve(&ctr->nodes, 1);
-  {  // per-request segment count, one atomic per request present in the warp
-    const unsigned peers = __match_any_sync(__activemask(), r.tx);
-    if (int(lane_id()) == __ffs(peers) - 1)
-      atomicAdd(&seg_per_tx[r.tx], (unsigned long long)__popc(peers));
-  }
+// The tree node ni of a resolved ray (RTSolver.cpp:142-257): its record (hot
+// FP32 part and cold FP64 part).  A ray that hits nothing ends at
+// src + 1e10 d (a launch) or src + 100 d (RTSolver.cpp:231,249).
+__device__ __forceinline__ void emit_node(NodeHot* nodes, NodeCold* cold,
+                                          unsigned long long cap, Counters* ctr,
+                                          unsigned long long ni, const RayRec& r, bool root,
+                                          const float3& o32, const float3& d32, bool soft,
+                                          bool hit, const Hit& h) {
   if (ni < cap) {
     NodeCold n;
     NodeHot m;
     n.s[0] = r.o[0]; n.s[1] = r.o[1]; n.s[2] = r.o[2];
     if (hit) {
       n.t[0] = h.p[0]; n.t[1] = h.p[1]; n.t[2] = h.p[2];
-      m.len = float(h.dist);
+      m.len = soft64::to_f32(h.dist);
     } else {
       const double sc = root ? 1E10 : 1E2;  // RTSolver.cpp:231,249
-      n.t[0] = x64::add(r.o[0], x64::mul(r.d[0], sc));
-      n.t[1] = x64::add(r.o[1], x64::mul(r.d[1], sc));
-      n.t[2] = x64::add(r.o[2], x64::mul(r.d[2], sc));
+      for (int a = 0; a < 3; ++a)
+        n.t[a] = x64::add(r.o[a], soft ? soft64::mul(r.d[a], sc) : x64::mul(r.d[a], sc));
       m.len = float(sc);
     }
     n.S = r.S;
     n.pad = 0.0;
     m.s[0] = o32.x; m.s[1] = o32.y; m.s[2] = o32.z;
-    m.S = float(r.S);
+    m.S = soft64::to_f32(r.S);
     m.u[0] = d32.x; m.u[1] = d32.y; m.u[2] = d32.z;
     m.parent = r.parent;
     m.cls = r.cls;
@@ -232,20 +272,64 @@ __device__ __forceinline__ unsigned long long emit_node(NodeHot* nodes, NodeCold
   } else {
     atomicOr(&ctr->overflow, kOvNodes);
   }
-  return ni;
 }
 
-// The position of the j-th (0-based) set bit of m (j < popc(m)).
-__device__ __forceinline__ int nth_set_bit(unsigned m, int j) {
-  int p = 0;
-  for (int w = 16; w >= 1; w >>= 1) {
-    const int c = __popc(m & (((1u << w) - 1u) << p));  // set bits in [p, p + w)
-    if (c <= j) {
-      j -= c;
-      p += w;
-    }
+// Executed segments per request, counted by each lane and added when the
+// request changes (a lane's rays are mostly one request's).
+struct SegmentCount {
+  uint32_t tx;
+  unsigned n;
+  __device__ __forceinline__ void flush(unsigned long long* per_tx) {
+    if (n) atomicAdd(&per_tx[tx], (unsigned long long)n);
+    n = 0;
   }
-  return p;
+  // The whole warp: one atomic per request present.
+  __device__ __forceinline__ void warp_flush(unsigned long long* per_tx) {
+    unsigned left = __ballot_sync(0xffffffffu, n != 0);
+    while (left) {
+      const int lead = __ffs(left) - 1;
+      const uint32_t t = __shfl_sync(0xffffffffu, tx, lead);
+      const bool mine = n != 0 && tx == t;
+      const unsigned sum = __reduce_add_sync(0xffffffffu, mine ? n : 0);
+      if (int(lane_id()) == lead) atomicAdd(&per_tx[tx], (unsigned long long)sum);
+      left &= ~__ballot_sync(0xffffffffu, mine);
+    }
+    n = 0;
+  }
+  __device__ __forceinline__ void add(unsigned long long* per_tx, uint32_t t) {
+    if (t != tx) flush(per_tx);
+    tx = t;
+    ++n;
+  }
+};
+
+// The next rays of the chunk for the idle lanes `im`: the j-th idle lane gets
+// the j-th of them (>= n: none left; exhausted, the same on every lane, when
+// the counter has passed the end).  Exactly as many as there are idle lanes
+// are taken, so that the warps together move through the chunk in order and
+// the children are queued near their neighbours': handing each warp a window
+// of 32 to 256 rays cost the level-9 canyon solve 1.4 ms in the next depths'
+// scattered rays, far more than the atomics it saved.
+__device__ __forceinline__ long long next_rays(unsigned long long* counter, unsigned im,
+                                               unsigned lane, long long n, bool& exhausted) {
+  const int want = __popc(im), leader = __ffs(im) - 1;
+  unsigned long long base = 0;
+  if (int(lane) == leader) base = atomicAdd(counter, (unsigned long long)want);
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if ((long long)base + want >= n) exhausted = true;
+  return (long long)base + __popc(im & ((1u << lane) - 1u));
+}
+
+// x64::normalize for components in soft64's range.
+__device__ __forceinline__ void normalize_soft(const double* a, double* r) {
+  const double z = dot64<Soft64>(a, a);
+  if (soft64::bits(z) != 0) {  // a sum of squares: never -0
+    const double s = soft64::sqrt(z);
+    const uint64_t x = soft64::rcp_of(s);
+    for (int i = 0; i < 3; ++i) r[i] = soft64::div_by(a[i], s, x);
+  } else {
+    for (int i = 0; i < 3; ++i) r[i] = a[i];
+  }
 }
 
 // ---- FP32 candidate search (persistent, rays refilled per warp) ----------
@@ -288,76 +372,69 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
   const long long n = min(n_all, A.hi) - A.lo;
   if (n <= 0) return;
   const unsigned lane = lane_id();
-  long long ray = -1;
   bool exhausted = false;
+  long long ray = -1;
   float3 o32 = make_float3(0, 0, 0), d32 = o32, inv = o32;
   float no = 0.0f, nd = 0.0f, m = 0.0f, tcut = INFINITY;
   int stack[kStack];
   int sp = 0, pending = -1, nc = 0, orank = -1;
-  bool fail = false;
+  bool fail = false, safe = false;
   uint2* out = nullptr;
   while (true) {
-    const bool idle = ray < 0 && !exhausted;
-    const unsigned im = __ballot_sync(0xffffffffu, idle);
-    const unsigned busy = __ballot_sync(0xffffffffu, ray >= 0);
-    if (im && (__popc(im) >= A.refill || busy == 0)) {
-      const int leader = __ffs(im) - 1;
-      unsigned long long base = 0;
-      if (int(lane) == leader) base = atomicAdd(A.work, (unsigned long long)__popc(im));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (idle) {
-        const long long k = (long long)base + __popc(im & ((1u << lane) - 1u));
-        if (k < n) {
-          ray = k;
-          double o[3], d[3];
-          orank = -1;
-          if (A.depth == 0) {
-            int q;
-            long long li;
-            root_ray(A.txp, A.n_tx, A.dirs, A.lo + k, o, d, q, li);
-          } else {
-            RayRec& r = A.in[A.lo + k];
-            for (int a = 0; a < 3; ++a) {
-              o[a] = r.o[a];
-              d[a] = r.d[a];
-            }
-            if (r.heap & 1) {
-              // a reflected ray (heap 2h+1) arrives with Reflect(d, n) not yet
-              // normalised: normalise it here, where a refill runs on at least
-              // half the warp's lanes, and store it for k_trace
-              double v[3] = {d[0], d[1], d[2]};
-              x64::normalize(v, d);
-              for (int a = 0; a < 3; ++a) r.d[a] = d[a];
-            }
-            orank = r.orank;
-          }
-          o32 = make_float3(float(o[0]), float(o[1]), float(o[2]));
-          d32 = make_float3(float(d[0]), float(d[1]), float(d[2]));
-          {
-            float4* f = reinterpret_cast<float4*>(A.ray32 + k);
-            f[0] = make_float4(o32.x, o32.y, o32.z, 0.0f);
-            f[1] = make_float4(d32.x, d32.y, d32.z, 0.0f);
-          }
-          inv = make_float3(1.0f / d32.x, 1.0f / d32.y, 1.0f / d32.z);
-          no = sqrtf(o32.x * o32.x + o32.y * o32.y + o32.z * o32.z);
-          nd = sqrtf(d32.x * d32.x + d32.y * d32.y + d32.z * d32.z);
-          m = A.sc.box_margin + kFiltK * no;
-          tcut = INFINITY;
-          sp = 0;
-          pending = -1;
-          nc = 0;
-          fail = false;
-          stack[sp++] = 0;  // the search root is always a node
-          out = A.cand + size_t(k) * kCand;
+    const unsigned im = __ballot_sync(0xffffffffu, ray < 0);
+    if ((__popc(im) >= A.refill || im == 0xffffffffu) && !exhausted) {
+      const long long k = next_rays(A.work, im, lane, n, exhausted);
+      if (ray < 0 && k < n) {
+        ray = k;
+        double o[3], d[3];
+        orank = -1;
+        if (A.depth == 0) {
+          int q;
+          long long li;
+          root_ray(A.txp, A.n_tx, A.dirs, A.lo + k, o, d, q, li);
         } else {
-          exhausted = true;
+          RayRec& r = A.in[A.lo + k];
+          for (int a = 0; a < 3; ++a) {
+            o[a] = r.o[a];
+            d[a] = r.d[a];
+          }
+          if (r.heap & 1) {
+            // a reflected ray (heap 2h+1) arrives with Reflect(d, n) not yet
+            // normalised: normalise it here, where a refill runs on at least
+            // half the warp's lanes, and store it for k_trace
+            double v[3] = {d[0], d[1], d[2]};
+            if (soft64::safe(v[0]) && soft64::safe(v[1]) && soft64::safe(v[2]))
+              normalize_soft(v, d);
+            else
+              x64::normalize(v, d);
+            for (int a = 0; a < 3; ++a) r.d[a] = d[a];
+          }
+          orank = r.orank;
         }
+        o32 = make_float3(soft64::to_f32(o[0]), soft64::to_f32(o[1]), soft64::to_f32(o[2]));
+        d32 = make_float3(soft64::to_f32(d[0]), soft64::to_f32(d[1]), soft64::to_f32(d[2]));
+        safe = soft64::safe(o[0]) && soft64::safe(o[1]) && soft64::safe(o[2]) &&
+               soft64::safe(d[0]) && soft64::safe(d[1]) && soft64::safe(d[2]);
+        {
+          float4* f = reinterpret_cast<float4*>(A.ray32 + k);
+          f[0] = make_float4(o32.x, o32.y, o32.z, 0.0f);
+          f[1] = make_float4(d32.x, d32.y, d32.z, 0.0f);
+        }
+        inv = make_float3(1.0f / d32.x, 1.0f / d32.y, 1.0f / d32.z);
+        no = sqrtf(o32.x * o32.x + o32.y * o32.y + o32.z * o32.z);
+        nd = sqrtf(d32.x * d32.x + d32.y * d32.y + d32.z * d32.z);
+        m = A.sc.box_margin + kBoxK * no;
+        tcut = INFINITY;
+        sp = 0;
+        pending = -1;
+        nc = 0;
+        fail = false;
+        stack[sp++] = 0;  // the search root is always a node
+        out = A.cand + size_t(k) * kCand;
       }
+      __syncwarp();
     }
-    if (__ballot_sync(0xffffffffu, ray >= 0) == 0) {
-      if (__all_sync(0xffffffffu, exhausted)) break;
-      continue;
-    }
+    if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;  // every lane is out of rays
     if (ray < 0) continue;
     bool done = false;
     for (int it = 0; it < A.steps && !done; ++it) {
@@ -375,14 +452,15 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
           const int rk = __ldg(A.sc.srank + j);
           // the triangle the ray starts on, left at a clear angle: the
           // reference's test of it certainly fails (origin_rejected); such a
-          // contender is never certain (k == 2), so dropping it changes no cut
+          // contender is never a sure hit, so dropping it changes no cut
           if (rk == orank && origin_rejected(T, o32, d32)) continue;
           if (nc == kCand) {
             fail = done = true;
             break;
           }
-          out[nc++] = make_uint2(unsigned(rk), __float_as_uint(tlo));
-          if (k == 2) tcut = fminf(tcut, thi * (1.0f + kTieSlack) + 1e-30f);
+          out[nc++] = make_uint2(unsigned(rk) | (k & kSureUV ? kContUV : 0u),
+                                 __float_as_uint(tlo));
+          if (k & kSureHit) tcut = fminf(tcut, thi * (1.0f + kTieSlack) + 1e-30f);
         }
         continue;
       }
@@ -445,7 +523,7 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
       }
     }
     if (done) {
-      A.ncand[ray] = fail ? kFindFallback : (unsigned char)nc;
+      A.ncand[ray] = fail ? kFindFallback : (unsigned char)(safe ? nc : nc | kCandUnsafe);
       ray = -1;
     }
   }
@@ -453,27 +531,48 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
 
 // Resident blocks of k_trace per SM (register budget 65536 / (128 x this)).
 #ifndef SBR_TRACE_BLOCKS
-#define SBR_TRACE_BLOCKS 4
+#define SBR_TRACE_BLOCKS 5
 #endif
 
+// Queue slots of the active lanes' children, one atomic: the transmitted rays
+// first, then the reflected ones, so that a warp of the next depth finds rays
+// that go the same way.
+__device__ __forceinline__ void reserve_children(unsigned long long* queue, bool do_t, bool do_r,
+                                                 unsigned long long& slot_t,
+                                                 unsigned long long& slot_r) {
+  const unsigned mask = __activemask();
+  const unsigned bt = __ballot_sync(mask, do_t), br = __ballot_sync(mask, do_r);
+  const unsigned lt = (1u << lane_id()) - 1u;
+  const int leader = __ffs(mask) - 1;
+  unsigned long long base = 0;
+  if (lane_id() == unsigned(leader) && (bt | br))
+    base = atomicAdd(queue, (unsigned long long)(__popc(bt) + __popc(br)));
+  base = __shfl_sync(mask, base, leader);
+  slot_t = base + __popc(bt & lt);
+  slot_r = base + __popc(bt) + __popc(br & lt);
+}
+
 // The tree node of a resolved ray and its children (RTSolver.cpp:142-257):
-// node record, reflected and transmitted rays, path-class interning.
-__device__ __forceinline__ void finish_ray(const TraceArgs& A, const RayRec& r, const float3& o32,
-                                           const float3& d32, bool hit, const Hit& h) {
+// node record (node ni), reflected and transmitted rays, path-class interning.
+// The three table probes are begun together: one memory latency, not three.
+__device__ __forceinline__ void finish_ray(const TraceArgs& A, unsigned long long ni,
+                                           const RayRec& r, const float3& o32, const float3& d32,
+                                           bool soft, bool hit, const Hit& h) {
   const TxParams& P = A.txp[r.tx];
-  const unsigned long long ni = emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, A.seg_per_tx,
-                                          r, A.depth == 0, o32, d32, hit, h);
   // children (RTSolver.cpp:186-221)
-  unsigned nch = 0;
-  bool do_r = false, do_t = false;
-  if (hit) {
-    do_r = r.rc < P.R;
-    do_t = r.tc < P.T;
-    nch = unsigned(do_r) + unsigned(do_t);
+  const bool do_r = hit && r.rc < P.R, do_t = hit && r.tc < P.T;
+  HashProbe p_cop, p_t, p_r;
+  if (do_r || do_t) {
+    p_cop = ht_probe(A.cop_tab, (unsigned long long)r.cop << 32 | uint32_t(A.tri_cop[h.rank]));
+    const unsigned long long key = (unsigned long long)r.cls << 32 | uint32_t(h.rank) << 1;
+    if (do_t) p_t = ht_probe(A.cls_tab, key | 1u);
+    if (do_r) p_r = ht_probe(A.cls_tab, key);
   }
-  const unsigned long long base = warp_reserve(&A.ctr->queue[A.depth + 1], nch);
-  if (nch) {
-    const Tri64& T = A.sc.tri64[h.rank];
+  unsigned long long slot_t, slot_r;
+  reserve_children(&A.ctr->queue[A.depth + 1], do_t, do_r, slot_t, slot_r);
+  emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, ni, r, A.depth == 0, o32, d32, soft,
+            hit, h);
+  if (do_r || do_t) {
     const double cum = x64::add(r.total, h.dist);  // node pathLength
     RayRec c;
     c.o[0] = h.p[0]; c.o[1] = h.p[1]; c.o[2] = h.p[2];
@@ -483,415 +582,210 @@ __device__ __forceinline__ void finish_ray(const TraceArgs& A, const RayRec& r, 
     c.launch = r.launch;
     c.tx = r.tx;
     c.orank = h.rank;
-    const int cop = A.tri_cop[h.rank];
-    const unsigned long long ck = (unsigned long long)r.cop << 32 | uint32_t(cop);
-    const uint32_t cop_cls = ht_insert(A.cop_tab, ck, &A.ctr->overflow, kOvCop, &A.ctr->used_cop,
-                                         &A.ctr->lost_cop);
-    // image source of the parent ray's class (the transmitter for a launch)
-    const double* pimg = is_root_class(r.cls) ? P.tx : A.cls_info[r.cls].img;
-    unsigned long long slot = base;
+    const uint32_t cop_cls = ht_insert(A.cop_tab, p_cop, &A.ctr->overflow, kOvCop,
+                                       &A.ctr->used_cop, &A.ctr->lost_cop);
+    c.cop = cop_cls;
     if (do_t) {  // transmitted: same direction, heap 2h, same image source
       c.d[0] = r.d[0]; c.d[1] = r.d[1]; c.d[2] = r.d[2];
       c.heap = r.heap * 2;
       c.rc = r.rc;
       c.tc = r.tc + 1;
-      const unsigned long long key = (unsigned long long)r.cls << 32 | (uint32_t(h.rank) << 1 | 1u);
       bool fresh = false;
-      c.cls = ht_insert(A.cls_tab, key, &A.ctr->overflow, kOvClass, &A.ctr->used_cls,
+      c.cls = ht_insert(A.cls_tab, p_t, &A.ctr->overflow, kOvClass, &A.ctr->used_cls,
                         &A.ctr->lost_cls, &fresh);
-      c.cop = cop_cls;
-      if (fresh) {  // only the thread that interned the class writes its records
-        write_class(A.cls_info[c.cls], pimg, r.cls, h.rank, cop_cls, 2, A.depth + 1);
-        write_class_cap(A.sc, pimg, A.sc.rank_to_id[h.rank], A.cls_cap[c.cls]);
-        list_class(A, c.cls);
-      }
-      if (slot < A.out_cap) A.out[slot] = c;
+      if (fresh)  // only the thread that interned the class writes its records
+        intern_class(A, c.cls, r.cls, P.tx, h.rank, cop_cls, 2);
+      if (slot_t < A.out_cap) A.out[slot_t] = c;
       else atomicOr(&A.ctr->overflow, kOvQueue);
-      ++slot;
     }
     if (do_r) {  // reflected: Reflect(d, n), heap 2h+1; k_find normalises it
-      const double dn = x64::dot(T.n, r.d);
-      for (int a = 0; a < 3; ++a) c.d[a] = x64::sub(r.d[a], x64::mul(x64::mul(2.0, T.n[a]), dn));
+      const double* n = A.sc.tri64[h.rank].n;
+      // (2 n) dn and n (2 dn) are the same number rounded once
+      if (soft) {
+        const double dn2 = 2.0 * dot64<Soft64>(n, r.d);
+        for (int a = 0; a < 3; ++a) c.d[a] = x64::sub(r.d[a], soft64::mul(n[a], dn2));
+      } else {
+        const double dn2 = 2.0 * x64::dot(n, r.d);
+        for (int a = 0; a < 3; ++a) c.d[a] = x64::sub(r.d[a], x64::mul(n[a], dn2));
+      }
       c.heap = r.heap * 2 + 1;
       c.rc = r.rc + 1;
       c.tc = r.tc;
-      const unsigned long long key = (unsigned long long)r.cls << 32 | (uint32_t(h.rank) << 1);
       bool fresh = false;
-      c.cls = ht_insert(A.cls_tab, key, &A.ctr->overflow, kOvClass, &A.ctr->used_cls,
+      c.cls = ht_insert(A.cls_tab, p_r, &A.ctr->overflow, kOvClass, &A.ctr->used_cls,
                         &A.ctr->lost_cls, &fresh);
-      c.cop = cop_cls;
-      if (fresh) {  // only the thread that interned the class writes its records
-        // ImagePoint (RTSolver.cpp:910-924) across the triangle the
-        // reference finds at this id's position of its mesh vector
-        const CorrTri& M = A.sc.corr[A.sc.rank_to_id[h.rank]];
-        double w[3], img[3];
-        x64::sub3(pimg, M.v1, w);
-        const double dist = x64::dot(M.n, w);
-        for (int a = 0; a < 3; ++a) img[a] = x64::sub(pimg[a], x64::mul(x64::mul(2.0, dist), M.n[a]));
-        write_class(A.cls_info[c.cls], img, r.cls, h.rank, cop_cls, 1, A.depth + 1);
-        write_class_cap(A.sc, img, A.sc.rank_to_id[h.rank], A.cls_cap[c.cls]);
-        list_class(A, c.cls);
-      }
-      if (slot < A.out_cap) A.out[slot] = c;
+      if (fresh) intern_class(A, c.cls, r.cls, P.tx, h.rank, cop_cls, 1);
+      if (slot_r < A.out_cap) A.out[slot_r] = c;
       else atomicOr(&A.ctr->overflow, kOvQueue);
     }
   }
 }
 
-// Every ancestor box of the winner's leaf in the reference BVH must pass the
-// reference's slab test, else the ray takes the reference-order traversal.
-__device__ __forceinline__ bool reachable_or_exact(const DevScene& sc, const RayRec& r,
-                                                   const float3& o32, const float3& d32, Hit& best,
-                                                   TraceStats& st, unsigned* overflow) {
-  best.leaf = sc.tri64[best.rank].node;
-  const float3 i32 = make_float3(1.0f / d32.x, 1.0f / d32.y, 1.0f / d32.z);
-  for (const AncBox* a = sc.anc + sc.anc_off[best.leaf];; ++a) {
-    const AncBox b = *a;
-    if (b.node < 0) break;
-    int v = slab_certain(b.fb, b.flat, o32, d32, i32);
-    if (v < 0) v = slab64(sc.ref[b.node].bb, r.o, r.d) ? 1 : 0;
-    if (!v) {
-      ++st.fallback;
-      return exact_closest(sc, r.o, r.d, best, overflow);
+// The untested contender with the lowest bound on t (the first of equal ones,
+// as a stable sort would give): its index, or -1 when none is left.
+__device__ __forceinline__ int next_contender(const uint2* cand, int nc, unsigned tested, float& t,
+                                              int& code) {
+  int k = -1;
+#pragma unroll 1
+  for (int j = 0; j < nc; ++j) {
+    if (tested >> j & 1u) continue;
+    const uint2 e = cand[j];
+    const float tj = __uint_as_float(e.y);
+    if (k < 0 || tj < t) {
+      k = j;
+      t = tj;
+      code = int(e.x);
     }
   }
-  return true;
+  return k;
 }
 
 // FP64 resolution of the contenders k_find left: they are tested in
 // ascending order of their FP32 lower bound on t until none can reach the
 // best exact distance; the answer is the lexicographic minimum (distance,
 // depth-first rank), the reference's strict '<' in visit order, accepted if
-// its leaf is reachable in the reference BVH (reachable_or_exact).  The kernel
+// its leaf is reachable in the reference BVH (leaf_reachable), else the ray
+// takes the reference-order traversal.  The kernel
 // is persistent: each lane holds one ray and runs at most one
-// FP64 triangle test per round, so the warp's FP64 instructions serve every
+// triangle test per round, so the warp's instructions serve every
 // lane that has a test due, whether it is a ray's first contender or a later
 // one.  A lane whose ray is resolved writes the node and children in the
-// same round and takes a new ray (one atomic per warp); a ray needing a
+// same round and takes a new ray; a ray needing a
 // second test no longer holds the whole warp through a second pass of the
-// test with a few lanes.
-__global__ void __launch_bounds__(128, SBR_TRACE_BLOCKS) k_trace(TraceArgs A) {
+// test with a few lanes.  The warp is brought together after each part of a
+// round.  A lane keeps only the ray's origin and direction and the best hit
+// between rounds; the rest of its record is read again when it is resolved.
+__global__ void __launch_bounds__(128, SBR_TRACE_BLOCKS) k_trace(const __grid_constant__ TraceArgs A) {
   if (A.ctr->overflow & kOvTrace) return;  // this solve will be repeated
   const long long n_all = rays_at_depth(A.ctr, A.depth, A.n_root, A.out_cap);
   const long long n = min(n_all, A.hi) - A.lo;
   if (n <= 0) return;
   const unsigned lane = lane_id();
-  TraceStats st{0, 0};
-  long long c = -1;  // the lane's ray (index in the chunk), -1 = none
+  unsigned fp64_tri = 0, fallback = 0;
+  SegmentCount seg{0, 0};
   bool exhausted = false;
-  RayRec r;
-  float3 o32 = make_float3(0.0f, 0.0f, 0.0f), d32 = o32;
-  int cr[kCand];
-  float ct[kCand];
-  int nc = 0, next = 0;
+  const unsigned long long base = node_base(A.ctr, A.depth, A.n_root, A.out_cap) + A.lo;
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&A.ctr->nodes, (unsigned long long)n);
+  long long c = -1;  // the lane's ray (index in the chunk), -1 = none
+  double o[3] = {0, 0, 0}, d[3] = {0, 0, 0};
+  int nc = 0;
+  unsigned tested = 0;      // contenders already tested (bit mask)
+  int next = -1, code = 0;  // the contender due: its index (-1 none), rank | kContUV
+  float tn = 0.0f;          // and lower bound on t
+  float tbest = 0.0f;       // FP32 copy of best.t
   Hit best;
   best.rank = INT_MAX;
+  best.leaf = -1;
+  best.t = 0.0;
   while (true) {
     // Refill: the idle lanes take the next window of rays (the j-th idle
     // lane the window's j-th ray, so the loads stay in order).  A ray k_find
     // left without a contender hits nothing: its lane writes the node at once
     // and stays idle, so such rays never hold a lane through a round of FP64
-    // tests.  Windows repeat until no lane is idle or the chunk is done;
-    // `exhausted` is the same on every lane.
+    // tests.  This repeats until no lane is idle or the chunk is done.
     unsigned im = __ballot_sync(0xffffffffu, c < 0);
     while (im && !exhausted) {
-      const int want = __popc(im);
-      const int leader = __ffs(im) - 1;
-      unsigned long long base = 0;
-      if (int(lane) == leader) base = atomicAdd(A.work, (unsigned long long)want);
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if ((long long)base + want >= n) exhausted = true;
-      const long long k = (long long)base + __popc(im & ((1u << lane) - 1u));
+      const long long k = next_rays(A.work, im, lane, n, exhausted);
       if (c < 0 && k < n) {
-        load_ray(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + k, r);
-        const float4* f = reinterpret_cast<const float4*>(A.ray32 + k);
-        const float4 fo = f[0], fd = f[1];
-        o32 = make_float3(fo.x, fo.y, fo.z);
-        d32 = make_float3(fd.x, fd.y, fd.z);
         nc = A.ncand[k];
-        if (nc == 0) {
-          Hit none;
-          emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, A.seg_per_tx, r, A.depth == 0,
-                    o32, d32, false, none);
-        } else {
-          c = k;
-          if (nc != kFindFallback) {
-            const uint2* cand = A.cand + size_t(k) * kCand;
-            for (int j = 0; j < nc; ++j) {
-              const uint2 e = cand[j];
-              const float t = __uint_as_float(e.y);
-              int m = j - 1;
-              while (m >= 0 && ct[m] > t) {  // insertion by lower bound (stable)
-                ct[m + 1] = ct[m];
-                cr[m + 1] = cr[m];
-                --m;
-              }
-              ct[m + 1] = t;
-              cr[m + 1] = int(e.x);
-            }
-          }
-          next = 0;
-          best.rank = INT_MAX;
-          best.dist = __longlong_as_double(0x7ff0000000000000ll);
-          best.t = best.dist;
-        }
-      }
-      im = __ballot_sync(0xffffffffu, c < 0);
-    }
-    if (__ballot_sync(0xffffffffu, c >= 0) == 0) break;  // every lane is out of rays
-    if (c < 0) continue;
-    bool done, hit;
-    if (nc == kFindFallback) {  // more contenders than kept, or a deep stack: one-pass search
-      hit = closest_hit(A.sc, r.o, r.d, best, st, &A.ctr->overflow);
-      done = true;
-    } else {
-      if (next < nc) {  // the next contender, nearest lower bound first
-        const int rk = cr[next++];
-        ++st.fp64_tri;
-        double t, P[3], dist;
-        if (mt64(A.sc.tri64[rk], r.o, r.d, t, P, dist) &&
-            (dist < best.dist || (dist == best.dist && rk < best.rank))) {
-          best.dist = dist;
-          best.t = t;
-          best.p[0] = P[0];
-          best.p[1] = P[1];
-          best.p[2] = P[2];
-          best.rank = rk;
-        }
-      }
-      // resolved when no further contender can reach the best exact distance
-      done = !(next < nc &&
-               (best.rank == INT_MAX || ct[next] <= float(best.t) * (1.0f + kTieSlack) + 1e-30f));
-      hit = false;
-      if (done && best.rank != INT_MAX)
-        hit = reachable_or_exact(A.sc, r, o32, d32, best, st, &A.ctr->overflow);
-    }
-    if (done) {
-      finish_ray(A, r, o32, d32, hit, best);
-      c = -1;
-    }
-  }
-  if (st.fp64_tri) atomicAdd(&A.ctr->fp64_tri, (unsigned long long)st.fp64_tri);
-  if (st.fallback) atomicAdd(&A.ctr->fallback, (unsigned long long)st.fallback);
-}
-
-}  // namespace sbr
-
-namespace sbr {
-
-// ---- FP64 resolution with the rays in shared memory ----------------------
-//
-// The same resolution as k_trace, scheduled so the FP64 work runs on full
-// warps.  k_trace keeps one ray per lane, so a warp's FP64 instructions
-// serve only the lanes whose ray has a test (or a node to write) due that
-// round: about a third of the lanes, measured.  Here each warp keeps
-// kPoolSlots rays in shared memory, more than its lanes; every round it lists
-// the slots with a test due and hands them out to its lanes in order (the
-// n-th lane takes the n-th listed slot), then lists the resolved slots and
-// hands those out for the node record and children, then refills the empty
-// slots (one atomic per warp).  A ray's tests still run one at a time in
-// ascending order of their lower bounds, so every decision is k_trace's.
-constexpr int kPoolSlots = 48;  // at most 64 (two ballot words)
-constexpr int kPoolWarps = 4;   // warps per block
-
-struct PoolSlots {  // one warp's slots, structure of arrays
-  double o[3][kPoolSlots], d[3][kPoolSlots];
-  double total[kPoolSlots], S[kPoolSlots];
-  double bt[kPoolSlots], bdist[kPoolSlots], bp[3][kPoolSlots];
-  float o32[3][kPoolSlots], d32[3][kPoolSlots];
-  float ct[kCand][kPoolSlots];
-  int cr[kCand][kPoolSlots];
-  int brank[kPoolSlots], orank[kPoolSlots];
-  uint32_t parent[kPoolSlots], cls[kPoolSlots], cop[kPoolSlots], launch[kPoolSlots];
-  uint32_t heap[kPoolSlots], tx[kPoolSlots];
-  uint16_t rc[kPoolSlots], tc[kPoolSlots];
-  uint8_t nc[kPoolSlots], nx[kPoolSlots], active[kPoolSlots], pad[kPoolSlots];
-};
-
-// The position of the j-th (0-based) set bit of the 64-slot mask (m0, m1).
-__device__ __forceinline__ int nth_slot(unsigned m0, unsigned m1, int j) {
-  const int c0 = __popc(m0);
-  return j < c0 ? nth_set_bit(m0, j) : 32 + nth_set_bit(m1, j - c0);
-}
-
-__global__ void __launch_bounds__(32 * kPoolWarps, 4) k_trace_pool(TraceArgs A) {
-  if (A.ctr->overflow & kOvTrace) return;  // this solve will be repeated
-  const long long n_all = rays_at_depth(A.ctr, A.depth, A.n_root, A.out_cap);
-  const long long n = min(n_all, A.hi) - A.lo;
-  if (n <= 0) return;
-  extern __shared__ __align__(16) unsigned char pool_smem[];
-  PoolSlots& P = reinterpret_cast<PoolSlots*>(pool_smem)[threadIdx.x >> 5];
-  const unsigned lane = lane_id();
-  TraceStats st{0, 0};
-  const bool hi_slot = lane + 32 < unsigned(kPoolSlots);  // this lane's second slot exists
-  P.active[lane] = 0;
-  if (hi_slot) P.active[lane + 32] = 0;
-  bool exhausted = false;
-  __syncwarp();
-  while (true) {
-    // ---- refill the empty slots
-    const unsigned e0 = __ballot_sync(0xffffffffu, !P.active[lane]);
-    const unsigned e1 = __ballot_sync(0xffffffffu, hi_slot && !P.active[lane + 32]);
-    const int n_empty = __popc(e0) + __popc(e1);
-    if (!exhausted && n_empty > 0) {
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(A.work, (unsigned long long)n_empty);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if ((long long)base + n_empty >= n) exhausted = true;
-      for (int j = int(lane); j < n_empty; j += 32) {
-        const long long k = (long long)base + j;
-        if (k >= n) break;
-        const int s = nth_slot(e0, e1, j);
-        RayRec r;
-        load_ray(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + k, r);
-        if (A.ncand[k] == 0) {  // no contender: it hits nothing; its slot stays empty
+        if (!(nc & kCandCount)) {
+          RayRec r;
+          load_ray(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + k, r);
           const float4* f = reinterpret_cast<const float4*>(A.ray32 + k);
           const float4 fo = f[0], fd = f[1];
           Hit none;
-          emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, A.seg_per_tx, r, A.depth == 0,
-                    make_float3(fo.x, fo.y, fo.z), make_float3(fd.x, fd.y, fd.z), false, none);
-          continue;
-        }
-        for (int a = 0; a < 3; ++a) {
-          P.o[a][s] = r.o[a];
-          P.d[a][s] = r.d[a];
-        }
-        P.total[s] = r.total;
-        P.S[s] = r.S;
-        P.parent[s] = r.parent;
-        P.cls[s] = r.cls;
-        P.cop[s] = r.cop;
-        P.launch[s] = r.launch;
-        P.heap[s] = r.heap;
-        P.rc[s] = r.rc;
-        P.tc[s] = r.tc;
-        P.tx[s] = r.tx;
-        P.orank[s] = r.orank;
-        const float4* f = reinterpret_cast<const float4*>(A.ray32 + k);
-        const float4 fo = f[0], fd = f[1];
-        P.o32[0][s] = fo.x;
-        P.o32[1][s] = fo.y;
-        P.o32[2][s] = fo.z;
-        P.d32[0][s] = fd.x;
-        P.d32[1][s] = fd.y;
-        P.d32[2][s] = fd.z;
-        const int nc = A.ncand[k];
-        P.nc[s] = uint8_t(nc);
-        if (nc != kFindFallback) {
-          // contenders by ascending lower bound (stable insertion)
-          float ct[kCand];
-          int cr[kCand];
-          const uint2* cand = A.cand + size_t(k) * kCand;
-          for (int c = 0; c < nc; ++c) {
-            const uint2 e = cand[c];
-            const float t = __uint_as_float(e.y);
-            int m = c - 1;
-            while (m >= 0 && ct[m] > t) {
-              ct[m + 1] = ct[m];
-              cr[m + 1] = cr[m];
-              --m;
-            }
-            ct[m + 1] = t;
-            cr[m + 1] = int(e.x);
-          }
-          for (int c = 0; c < nc; ++c) {
-            P.ct[c][s] = ct[c];
-            P.cr[c][s] = cr[c];
-          }
-        }
-        P.nx[s] = 0;
-        P.brank[s] = INT_MAX;
-        P.bdist[s] = __longlong_as_double(0x7ff0000000000000ll);
-        P.bt[s] = P.bdist[s];
-        P.active[s] = 1;
-      }
-    }
-    __syncwarp();
-    const unsigned a0 = __ballot_sync(0xffffffffu, P.active[lane]);
-    const unsigned a1 = __ballot_sync(0xffffffffu, hi_slot && P.active[lane + 32]);
-    if (!(a0 | a1) && exhausted) break;
-    // ---- one FP64 test for every slot with one due, slots handed out in order
-    auto due = [&](int s) {
-      return P.active[s] && P.nc[s] != kFindFallback && P.nx[s] < P.nc[s];
-    };
-    const unsigned t0 = __ballot_sync(0xffffffffu, due(int(lane)));
-    const unsigned t1 = __ballot_sync(0xffffffffu, hi_slot && due(int(lane) + 32));
-    const int n_test = __popc(t0) + __popc(t1);
-    for (int j = int(lane); j < n_test; j += 32) {
-      const int s = nth_slot(t0, t1, j);
-      const int rk = P.cr[P.nx[s]][s];
-      P.nx[s] = uint8_t(P.nx[s] + 1);
-      ++st.fp64_tri;
-      const double o[3] = {P.o[0][s], P.o[1][s], P.o[2][s]};
-      const double d[3] = {P.d[0][s], P.d[1][s], P.d[2][s]};
-      double t, Q[3], dist;
-      if (mt64(A.sc.tri64[rk], o, d, t, Q, dist) &&
-          (dist < P.bdist[s] || (dist == P.bdist[s] && rk < P.brank[s]))) {
-        P.bdist[s] = dist;
-        P.bt[s] = t;
-        P.bp[0][s] = Q[0];
-        P.bp[1][s] = Q[1];
-        P.bp[2][s] = Q[2];
-        P.brank[s] = rk;
-      }
-    }
-    __syncwarp();
-    // ---- resolved slots: no further contender can reach the best distance
-    auto resolved = [&](int s) {
-      if (!P.active[s]) return false;
-      if (P.nc[s] == kFindFallback) return true;
-      const int nx = P.nx[s];
-      return !(nx < P.nc[s] &&
-               (P.brank[s] == INT_MAX || P.ct[nx][s] <= float(P.bt[s]) * (1.0f + kTieSlack) + 1e-30f));
-    };
-    const unsigned r0 = __ballot_sync(0xffffffffu, resolved(int(lane)));
-    const unsigned r1 = __ballot_sync(0xffffffffu, hi_slot && resolved(int(lane) + 32));
-    const int n_res = __popc(r0) + __popc(r1);
-    for (int j0 = 0; j0 < n_res; j0 += 32) {
-      const int j = j0 + int(lane);
-      if (j < n_res) {
-        const int s = nth_slot(r0, r1, j);
-        RayRec r;
-        for (int a = 0; a < 3; ++a) {
-          r.o[a] = P.o[a][s];
-          r.d[a] = P.d[a][s];
-        }
-        r.total = P.total[s];
-        r.S = P.S[s];
-        r.parent = P.parent[s];
-        r.cls = P.cls[s];
-        r.cop = P.cop[s];
-        r.launch = P.launch[s];
-        r.heap = P.heap[s];
-        r.rc = P.rc[s];
-        r.tc = P.tc[s];
-        r.tx = P.tx[s];
-        r.orank = P.orank[s];
-        const float3 o32 = make_float3(P.o32[0][s], P.o32[1][s], P.o32[2][s]);
-        const float3 d32 = make_float3(P.d32[0][s], P.d32[1][s], P.d32[2][s]);
-        Hit best;
-        best.rank = P.brank[s];
-        best.dist = P.bdist[s];
-        best.t = P.bt[s];
-        best.p[0] = P.bp[0][s];
-        best.p[1] = P.bp[1][s];
-        best.p[2] = P.bp[2][s];
-        bool hit;
-        if (P.nc[s] == kFindFallback) {  // more contenders than kept: one-pass search
-          hit = closest_hit(A.sc, r.o, r.d, best, st, &A.ctr->overflow);
+          seg.add(A.seg_per_tx, r.tx);
+          emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, base + k, r, A.depth == 0,
+                    make_float3(fo.x, fo.y, fo.z), make_float3(fd.x, fd.y, fd.z),
+                    !(nc & kCandUnsafe), false, none);
         } else {
-          hit = best.rank != INT_MAX && reachable_or_exact(A.sc, r, o32, d32, best, st,
-                                                            &A.ctr->overflow);
+          load_ray_line(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + k, o, d);
+          c = k;
+          tested = 0;
+          next = nc != kFindFallback
+                     ? next_contender(A.cand + size_t(k) * kCand, nc & kCandCount, 0u, tn, code)
+                     : -1;
+          best.rank = INT_MAX;
+          best.dist = __longlong_as_double(0x7ff0000000000000ll);
         }
-        finish_ray(A, r, o32, d32, hit, best);
-        P.active[s] = 0;
       }
-      // finish_ray's warp-wide reservations need every lane: the loop bound is uniform
+      __syncwarp();
+      im = __ballot_sync(0xffffffffu, c < 0);
+    }
+    if (__ballot_sync(0xffffffffu, c >= 0) == 0) break;  // every lane is out of rays
+    const bool soft = A.sc.soft && !(nc & kCandUnsafe);
+    if (c >= 0 && next >= 0) {  // the contender due
+      const int rk = code & ~int(kContUV);
+      ++fp64_tri;
+      const Tri64& T = A.sc.tri64[rk];
+      double t, P[3], dist;
+      bool ok;
+      if (soft) {
+        ok = mt64_t<Soft64>(T, o, d, code < 0, t, P, dist);
+      } else {
+        const Mt64Result m = mt64_call(&T, o[0], o[1], o[2], d[0], d[1], d[2]);
+        ok = m.ok;
+        t = m.t;
+        dist = m.dist;
+        for (int a = 0; a < 3; ++a) P[a] = m.p[a];
+      }
+      if (ok && (soft64::less(dist, best.dist) ||
+                 (soft64::same(dist, best.dist) && rk < best.rank))) {
+        best.dist = dist;
+        tbest = soft64::to_f32(t);
+        best.p[0] = P[0];
+        best.p[1] = P[1];
+        best.p[2] = P[2];
+        best.rank = rk;
+      }
+    }
+    __syncwarp();
+    bool done = false, hit = false;
+    if (c >= 0) {
+      if (nc == kFindFallback) {  // more contenders than kept, or a deep stack: one-pass search
+        best = closest_call(A.sc, o[0], o[1], o[2], d[0], d[1], d[2], A.ctr);
+        hit = best.rank != INT_MAX;
+        done = true;
+      } else {
+        // resolved when no further contender can reach the best exact distance
+        tested |= 1u << next;
+        next = (nc & kCandCount) > 1
+                   ? next_contender(A.cand + size_t(c) * kCand, nc & kCandCount, tested, tn, code)
+                   : -1;
+        done = next < 0 ||
+               !(best.rank == INT_MAX || tn <= tbest * (1.0f + kTieSlack) + 1e-30f);
+        hit = done && best.rank != INT_MAX;
+      }
+    }
+    __syncwarp();
+    if (done) {
+      RayRec r;
+      load_ray(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + c, r);
+      const float4* f = reinterpret_cast<const float4*>(A.ray32 + c);
+      const float4 fo = f[0], fd = f[1];
+      const float3 o32 = make_float3(fo.x, fo.y, fo.z), d32 = make_float3(fd.x, fd.y, fd.z);
+      for (int a = 0; a < 3; ++a) {
+        r.o[a] = o[a];
+        r.d[a] = d[a];
+      }
+      if (hit && nc != kFindFallback) {
+        const float3 i32 = make_float3(1.0f / d32.x, 1.0f / d32.y, 1.0f / d32.z);
+        if (!leaf_reachable(A.sc, A.sc.tri64[best.rank].node, o, d, o32, d32, i32)) {
+          ++fallback;
+          best = exact_call(A.sc, o[0], o[1], o[2], d[0], d[1], d[2], &A.ctr->overflow);
+          hit = best.rank != INT_MAX;
+        }
+      }
+      seg.add(A.seg_per_tx, r.tx);
+      finish_ray(A, base + c, r, o32, d32, soft, hit, best);
+      c = -1;
     }
     __syncwarp();
   }
-  if (st.fp64_tri) atomicAdd(&A.ctr->fp64_tri, (unsigned long long)st.fp64_tri);
-  if (st.fallback) atomicAdd(&A.ctr->fallback, (unsigned long long)st.fallback);
+  seg.warp_flush(A.seg_per_tx);
+  fp64_tri = __reduce_add_sync(0xffffffffu, fp64_tri);
+  if (lane == 0 && fp64_tri) atomicAdd(&A.ctr->fp64_tri, (unsigned long long)fp64_tri);
+  if (fallback) atomicAdd(&A.ctr->fallback, (unsigned long long)fallback);
 }
 
 }  // namespace sbr
