@@ -173,7 +173,8 @@ struct NodeSpan {
 // rb of its segment (rb bounds the sphere radius (S + |P|) tan(beta), with
 // |P| <= (cmax + S tan b) / (1 - tan b) for any capturing point).  All
 // ranges are widened well beyond their FP32 rounding.
-__device__ __forceinline__ NodeSpan node_span(const NodeHot& nd, const TxParams& P,
+template <class Node>
+__device__ __forceinline__ NodeSpan node_span(const Node& nd, const TxParams& P,
                                               const RxGrid& g, float cmax, int use_cone) {
   NodeSpan sp{0.0f, -1.0f, 0.0f, 0.0f, 0, use_cone};
   if (P.n_rx <= 0) return sp;
@@ -230,7 +231,8 @@ struct ChunkBox {
   int nrows;
 };
 
-__device__ __forceinline__ ChunkBox chunk_box(const NodeHot& nd, const RxGrid& g,
+template <class Node>
+__device__ __forceinline__ ChunkBox chunk_box(const Node& nd, const RxGrid& g,
                                               const NodeSpan& sp, int ch, float cmax, float tanb,
                                               bool use_cone, const float* cone) {
   ChunkBox cb;
@@ -583,6 +585,34 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
   }
 }
 
+// Items of a work counter handed to a warp, a window at a time: every warp of
+// the grid asks the same counter, which serves an atomic in about 0.65 ns, so
+// a warp takes a part of what was left when it last asked (at least
+// `smallest`, a multiple of 32, at most 256 items) and the windows shrink
+// towards the end, where an uneven last one would leave warps waiting.
+struct WorkWindow {
+  unsigned long long* counter;
+  long long next, end, n;  // the window's rest; items in all
+  float share;
+  int smallest;
+  __device__ __forceinline__ WorkWindow(unsigned long long* c, long long items, int least)
+      : counter(c), next(0), end(0), n(items), smallest(least) {
+    share = 0.125f / (32.0f * float(gridDim.x) * float(blockDim.x >> 5));
+  }
+  // Fetches a window if the last one is used up; false when no item is left
+  // (the same on every lane; the whole warp calls).
+  __device__ __forceinline__ bool refill() {
+    if (next < end) return true;
+    if (next >= n && end > 0) return false;
+    const int size = min(256, max(smallest, 32 * int(float(n - next) * share)));
+    unsigned long long base = 0;
+    if (lane_id() == 0) base = atomicAdd(counter, (unsigned long long)size);
+    next = (long long)__shfl_sync(0xffffffffu, base, 0);
+    end = min(next + size, n);
+    return next < n;
+  }
+};
+
 // ---- fast path, flattened over the nodes of a batch ------------------------
 //
 // The same tests as k_capture's fast path with the same chunks, cell boxes
@@ -618,6 +648,28 @@ __device__ __forceinline__ int warp_find(int incl, int k) {
 
 constexpr int kFastB = 32;  // nodes staged per warp and batch (one per lane)
 
+// What the fast path keeps of a node in shared memory.
+struct StagedNode {
+  float s[3], S, u[3], len;
+  uint32_t cls, tx;
+};
+
+// Pairs for k_capture_finish, gathered per warp so that one atomic on the pair
+// counter (which every warp of the grid adds to) serves more than 32 of them.
+constexpr int kPairBuf = 64;
+__device__ __forceinline__ void flush_pairs(const CaptureArgs& A, const uint2* buf, int& n,
+                                            int lane) {
+  __syncwarp();
+  unsigned long long base = 0;
+  if (lane == 0 && n) base = atomicAdd(&A.ctr->pairs, (unsigned long long)n);
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (lane == 0 && base + n > A.pair_cap) atomicOr(&A.ctr->overflow, kOvPairs);
+  for (int j = lane; j < n; j += 32)
+    if (base + j < A.pair_cap) A.pairs[base + j] = buf[j];
+  n = 0;
+  __syncwarp();
+}
+
 __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast(CaptureArgs A) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
@@ -625,21 +677,24 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
   const unsigned long long n_nodes = min(A.ctr->nodes, A.node_cap);
   unsigned long long cand = 0;
   constexpr int B = kFastB;
-  __shared__ NodeHot s_nh[kCapWarps][B];
+  __shared__ StagedNode s_nh[kCapWarps][B];
+  __shared__ uint2 s_pr[kCapWarps][kPairBuf];
+  int n_pr = 0;  // pairs gathered (the same on every lane)
   __shared__ Tri32 s_tl[kCapWarps][B];      // the class's last triangle
   __shared__ float s_fl[kCapWarps][B][12];  // image source + correction filter terms
   __shared__ float s_cn[kCapWarps][B][16];  // loosened correction cone
   __shared__ NodeSpan s_sp[kCapWarps][B];   // clipped span and chunking
   __shared__ ChunkBox s_ck[kCapWarps][32];  // the current 32 (node, chunk) items
   __shared__ int s_ckn[kCapWarps][32];      // their node (batch index) | chunk << 8
-  for (unsigned long long base = next_batch(A.work, lane, B); base < n_nodes;
-       base = next_batch(A.work, lane, B)) {
+  for (WorkWindow work(A.work, (long long)n_nodes, B); work.refill(); work.next += B) {
+    const unsigned long long base = work.next;
     int nck = 0;  // chunks of this lane's node
     {
       const unsigned long long my = base + lane;
       if (lane < B && my < n_nodes) {
         const NodeHot h = A.nodes[my];
-        s_nh[warp][lane] = h;
+        s_nh[warp][lane] = StagedNode{{h.s[0], h.s[1], h.s[2]}, h.S, {h.u[0], h.u[1], h.u[2]},
+                                      h.len, h.cls, h.tx};
         const float cmax = A.gb[h.tx].cmax;
         int cone_ok = 0;
         if (!is_root_class(h.cls)) {
@@ -677,7 +732,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
       int nrows = 0;
       if (k < n_ck) {
         const int ch = k - (j_incl - j_n);
-        const NodeHot& nd = s_nh[warp][j];
+        const StagedNode& nd = s_nh[warp][j];
         const NodeSpan& sp = s_sp[warp][j];
         const ChunkBox cb = chunk_box(nd, A.grids[nd.tx], sp, ch, A.gb[nd.tx].cmax,
                                       A.txp[nd.tx].tan_beta32, sp.use_cone != 0, s_cn[warp][j]);
@@ -699,7 +754,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
           const int ridx = r - (ci_incl - ci_n);
           const ChunkBox& cb = s_ck[warp][ci];
           const int jn = s_ckn[warp][ci] & 0xff;
-          const NodeHot& nd = s_nh[warp][jn];
+          const StagedNode& nd = s_nh[warp][jn];
           const RxGrid& g = A.grids[nd.tx];
           const float3 s = make_float3(nd.s[0], nd.s[1], nd.s[2]);
           const float3 u = make_float3(nd.u[0], nd.u[1], nd.u[2]);
@@ -755,73 +810,78 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
           const int rcnt = __shfl_sync(FULL, cnt, rl);
           const int rbeg = __shfl_sync(FULL, beg, rl);
           const int rci = __shfl_sync(FULL, ci, rl);
-          if (q >= n_c) continue;
-          const int ckn = s_ckn[warp][rci];
-          const int jn = ckn & 0xff, ch = ckn >> 8;
-          const NodeHot& nd = s_nh[warp][jn];
-          const NodeSpan& sp = s_sp[warp][jn];
-          const float a = s_ck[warp][rci].a, b = s_ck[warp][rci].b, mr = s_ck[warp][rci].mr;
-          const RxGrid& g = A.grids[nd.tx];
-          const float3 s = make_float3(nd.s[0], nd.s[1], nd.s[2]);
-          const float3 u = make_float3(nd.u[0], nd.u[1], nd.u[2]);
-          const float4 c4 = g.rx32[rbeg + (q - (rincl - rcnt))];
-          const float3 c = make_float3(c4.x, c4.y, c4.z);
-          const float wx = c.x - s.x, wy = c.y - s.y, wz = c.z - s.z;
-          const float lam = u.x * wx + u.y * wy + u.z * wz;
-          if (ch > 0 && lam < a) continue;                 // owned by an earlier chunk
-          if (ch < sp.nchunk - 1 && lam >= b) continue;    // owned by a later chunk
-          const int gi = __float_as_int(c4.w);
-          ++cand;
-          if (is_root_class(nd.cls)) {
-            if (!A.direct_ok[gi]) continue;
-          } else {
-            // MultiPathCorrection's last step must cross the class's last
-            // triangle: FP32 filter from the image source towards the receiver
-            const float* fl = s_fl[warp][jn];
-            const TriFrom Fl{fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10]};
-            const float3 dd = make_float3(c.x - fl[0], c.y - fl[1], c.z - fl[2]);
-            if (!tri_filter_from(s_tl[warp][jn], Fl, dd,
-                                 sqrt_up(dd.x * dd.x + dd.y * dd.y + dd.z * dd.z)))
-              continue;
-          }
-          const float tanb = A.txp[nd.tx].tan_beta32;
-          const float len = nd.len, S = nd.S;
-          int v;
-          if (lam < a || lam > b) {
-            // outside the chunk's own range: full-margin test
-            v = reception32(s, u, len, S, c, tanb);
-          } else {
-            const float ml = kRecK * (sp.ns + A.gb[nd.tx].cmax + 1.0f);
-            if (lam < -ml) {
-              v = 0;
-            } else if (lam <= ml) {
-              v = -1;
+          uint2 pair = make_uint2(0, 0);
+          auto passes = [&]() -> bool {
+            if (q >= n_c) return false;
+            const int ckn = s_ckn[warp][rci];
+            const int jn = ckn & 0xff, ch = ckn >> 8;
+            const StagedNode& nd = s_nh[warp][jn];
+            const NodeSpan& sp = s_sp[warp][jn];
+            const float a = s_ck[warp][rci].a, b = s_ck[warp][rci].b, mr = s_ck[warp][rci].mr;
+            const RxGrid& g = A.grids[nd.tx];
+            const float3 s = make_float3(nd.s[0], nd.s[1], nd.s[2]);
+            const float3 u = make_float3(nd.u[0], nd.u[1], nd.u[2]);
+            const float4 c4 = g.rx32[rbeg + (q - (rincl - rcnt))];
+            const float3 c = make_float3(c4.x, c4.y, c4.z);
+            const float wx = c.x - s.x, wy = c.y - s.y, wz = c.z - s.z;
+            const float lam = u.x * wx + u.y * wy + u.z * wz;
+            if (ch > 0 && lam < a) return false;                 // owned by an earlier chunk
+            if (ch < sp.nchunk - 1 && lam >= b) return false;    // owned by a later chunk
+            const int gi = __float_as_int(c4.w);
+            ++cand;
+            if (is_root_class(nd.cls)) {
+              if (!A.direct_ok[gi]) return false;
             } else {
-              const float lcl = fminf(lam, len);
-              const float px = s.x + lcl * u.x, py = s.y + lcl * u.y, pz = s.z + lcl * u.z;
-              const float np = sqrt_up(px * px + py * py + pz * pz);
-              const float ex = c.x - px, ey = c.y - py, ez = c.z - pz;
-              const float d2 = ex * ex + ey * ey + ez * ez;
-              const float rad = (S + np) * tanb;
-              const float rh = rad + mr, rl2 = rad - mr;
-              v = d2 > rh * rh ? 0 : ((rl2 > 0.0f && d2 < rl2 * rl2) ? 1 : -1);
+              // MultiPathCorrection's last step must cross the class's last
+              // triangle: FP32 filter from the image source towards the receiver
+              const float* fl = s_fl[warp][jn];
+              const TriFrom Fl{fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10]};
+              const float3 dd = make_float3(c.x - fl[0], c.y - fl[1], c.z - fl[2]);
+              if (!tri_filter_from(s_tl[warp][jn], Fl, dd,
+                                   sqrt_up(dd.x * dd.x + dd.y * dd.y + dd.z * dd.z)))
+                return false;
             }
-          }
+            const float tanb = A.txp[nd.tx].tan_beta32;
+            const float len = nd.len, S = nd.S;
+            int v;
+            if (lam < a || lam > b) {
+              // outside the chunk's own range: full-margin test
+              v = reception32(s, u, len, S, c, tanb);
+            } else {
+              const float ml = kRecK * (sp.ns + A.gb[nd.tx].cmax + 1.0f);
+              if (lam < -ml) {
+                v = 0;
+              } else if (lam <= ml) {
+                v = -1;
+              } else {
+                const float lcl = fminf(lam, len);
+                const float px = s.x + lcl * u.x, py = s.y + lcl * u.y, pz = s.z + lcl * u.z;
+                const float np = sqrt_up(px * px + py * py + pz * pz);
+                const float ex = c.x - px, ey = c.y - py, ez = c.z - pz;
+                const float d2 = ex * ex + ey * ey + ez * ez;
+                const float rad = (S + np) * tanb;
+                const float rh = rad + mr, rl2 = rad - mr;
+                v = d2 > rh * rh ? 0 : ((rl2 > 0.0f && d2 < rl2 * rl2) ? 1 : -1);
+              }
+            }
+            if (v == 0) return false;
+            pair = make_uint2(uint32_t(base + jn), uint32_t(gi) | (v < 0 ? 0x80000000u : 0u));
+            return true;
+          };
           // the exact reception test, image correction and ancestor
           // suppression run densely in k_capture_finish
-          if (v == 0) continue;
-          const unsigned long long slot = warp_reserve(&A.ctr->pairs, 1);
-          if (slot < A.pair_cap)
-            A.pairs[slot] =
-                make_uint2(uint32_t(base + jn), uint32_t(gi) | (v < 0 ? 0x80000000u : 0u));
-          else
-            atomicOr(&A.ctr->overflow, kOvPairs);
+          const bool pass = passes();
+          const unsigned pm = __ballot_sync(FULL, pass);
+          if (pass) s_pr[warp][n_pr + __popc(pm & ((1u << lane) - 1u))] = pair;
+          n_pr += __popc(pm);
+          if (n_pr > kPairBuf - 32) flush_pairs(A, s_pr[warp], n_pr, lane);
         }
       }
       __syncwarp();  // the next group of items overwrites s_ck
     }
     __syncwarp();  // the next batch overwrites the staged records
   }
+  flush_pairs(A, s_pr[warp], n_pr, lane);
   for (int o = 16; o; o >>= 1) cand += __shfl_xor_sync(FULL, cand, o);
   if (lane == 0 && cand) atomicAdd(&A.ctr->cand, cand);
 }
