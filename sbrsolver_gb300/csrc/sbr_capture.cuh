@@ -134,23 +134,26 @@ __device__ __forceinline__ bool cone_meets_box(const float* cone, const float* l
   return true;
 }
 
-// Narrows the cell range [x0, x1] of grid row (iy, iz) to the cells whose
-// box can hold a point inside the cone; an empty row gets x0 > x1.
+// Narrows the cell range [x0, x1] of the grid row at (i1, i2) along the other
+// two axes to the cells whose box can hold a point inside the cone; an empty
+// row gets x0 > x1.  cone[12 + k]: 1 / the row component of plane k's normal.
 __device__ __forceinline__ void cone_cells(const float* cone, const RxGrid& g, float inv_cell,
-                                           int iy, int iz, int& x0, int& x1) {
-  const float y0 = g.org[1] + iy * g.cell, y1 = y0 + g.cell;
-  const float z0 = g.org[2] + iz * g.cell, z1 = z0 + g.cell;
+                                           int i1, int i2, int& x0, int& x1) {
+  const int ar = g.ax[0], am = g.ax[1], al = g.ax[2];
+  const float y0 = g.org[am] + i1 * g.cell, y1 = y0 + g.cell;
+  const float z0 = g.org[al] + i2 * g.cell, z1 = z0 + g.cell;
   for (int k = 0; k < 3; ++k) {
-    const float nx = cone[4 * k], ny = cone[4 * k + 1], nz = cone[4 * k + 2], off = cone[4 * k + 3];
-    // need nx*x >= off - max over the row's y/z band of (ny*y + nz*z)
+    const float nx = cone[4 * k + ar], ny = cone[4 * k + am], nz = cone[4 * k + al],
+                off = cone[4 * k + 3];
+    // need nx*x >= off - max over the row's band of (ny*y + nz*z)
     const float r = off - fmaxf(ny * y0, ny * y1) - fmaxf(nz * z0, nz * z1);
     const float slack = 1e-3f * g.cell;
     if (nx > 0.0f) {
       const float xl = r * cone[12 + k];  // x >= xl
-      if (isfinite(xl)) x0 = max(x0, int(floorf((xl - g.org[0] - slack) * inv_cell)));
+      if (isfinite(xl)) x0 = max(x0, int(floorf((xl - g.org[ar] - slack) * inv_cell)));
     } else if (nx < 0.0f) {
       const float xh = r * cone[12 + k];  // x <= xh
-      if (isfinite(xh)) x1 = min(x1, int(floorf((xh - g.org[0] + slack) * inv_cell)));
+      if (isfinite(xh)) x1 = min(x1, int(floorf((xh - g.org[ar] + slack) * inv_cell)));
     } else if (r > 0.0f) {
       x1 = x0 - 1;
     }
@@ -210,8 +213,13 @@ __device__ __forceinline__ NodeSpan node_span(const Node& nd, const TxParams& P,
     }
   }
   if (!(lo <= hi)) return sp;
+  // chunks about as long as the sphere's radius at the middle of the span: a
+  // chunk's receivers come from a radius around it, and shorter ones would
+  // read the same receivers again and again (level 2, 3 km of receivers on a
+  // line: 12 m chunks under 900 m spheres, 1.8 ms of capture)
   const float r0 = (S + sqrt_up(ss + 2.0f * lo * su + lo * lo)) * tanb;
-  const float lc = fmaxf(g.chunk_len, r0);
+  const float r1 = (S + sqrt_up(ss + 2.0f * hi * su + hi * hi)) * tanb;
+  const float lc = fmaxf(g.chunk_len, 0.5f * (r0 + r1));
   int nchunk = int(ceilf(__fdividef(hi - lo, lc)));
   nchunk = max(1, min(nchunk, 4096));
   sp.lo = lo;
@@ -252,8 +260,11 @@ __device__ __forceinline__ ChunkBox chunk_box(const Node& nd, const RxGrid& g,
     cb.c0[k] = max(0, int(floorf((fminf(pa[k], pb[k]) - cb.rb - g.org[k]) * g.inv_cell)));
     cb.c1[k] = min(g.dim[k] - 1, int(floorf((fmaxf(pa[k], pb[k]) + cb.rb - g.org[k]) * g.inv_cell)));
   }
-  const int ny = cb.c1[1] - cb.c0[1] + 1, nz = cb.c1[2] - cb.c0[2] + 1;
-  cb.nrows = (cb.c0[0] <= cb.c1[0] && ny > 0 && nz > 0) ? ny * nz : 0;
+  int e[3];  // cells along each axis
+  for (int k = 0; k < 3; ++k) e[k] = cb.c1[k] - cb.c0[k] + 1;
+  cb.nrows = 0;
+  if (e[0] > 0 && e[1] > 0 && e[2] > 0)
+    cb.nrows = g.ax[0] == 0 ? e[1] * e[2] : (g.ax[0] == 1 ? e[0] * e[2] : e[0] * e[1]);
   if (use_cone && cb.nrows) {  // the chunk's cells all outside the cone: skip it
     float blo[3], bhi[3];
     for (int k = 0; k < 3; ++k) {
@@ -309,6 +320,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
         const NodeHot h = A.nodes[my];
         s_nh[warp][lane] = h;
         const float cmax = A.gb[h.tx].cmax;
+        const int ar = A.grids[h.tx].ax[0];
         int cone_ok = 0;
         if (!is_root_class(h.cls)) {
           const ClassCap c = A.cls_cap[h.cls];
@@ -326,7 +338,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
             cn[4 * k + 1] = c.n[k][1];
             cn[4 * k + 2] = c.n[k][2];
             cn[4 * k + 3] = c.n[k][3] - 2.0f * m;
-            cn[12 + k] = c.inv_nx[k];
+            cn[12 + k] = 1.0f / (ar == 0 ? c.n[k][0] : (ar == 1 ? c.n[k][1] : c.n[k][2]));
           }
         }
         const NodeSpan sp = node_span(h, A.txp[h.tx], A.grids[h.tx], cmax, cone_ok);
@@ -349,7 +361,11 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
       // Reciprocals for the cell-range arithmetic below.  Every range there is
       // widened by at least 2e-3 m + cell/100, far more than the few ulps a
       // product with a reciprocal differs from the quotient.
-      const float inv_uy = __frcp_rn(u.y), inv_uz = __frcp_rn(u.z);
+      const int ar = g.ax[0], am = g.ax[1], al = g.ax[2];
+      const NodeHot& sn = s_nh[warp][jj];  // in shared memory: indexed by axis
+      const float sr = sn.s[ar], sm = sn.s[am], sl = sn.s[al];
+      const float ur = sn.u[ar], um = sn.u[am], ul = sn.u[al];
+      const float inv_um = __frcp_rn(um), inv_ul = __frcp_rn(ul);
       const float inv_cell = g.inv_cell;
       // Stage the ancestor chain when every capture is checked against it
       // (stage counts); otherwise only corrected captures (~0.1% of captures)
@@ -394,48 +410,51 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
         const float ml = kRecK * (ns + cmax + 1.0f);
         {
           for (int ch = 0; ch < nchunk; ++ch) {
-            const ChunkBox cb = ch == 0 ? s_ck[warp][jj]
-                                        : chunk_box(nd, g, sp, ch, cmax, tanb, use_cone, cone_w);
+            if (ch > 0) {  // every lane forms the same box
+              const ChunkBox next = chunk_box(nd, g, sp, ch, cmax, tanb, use_cone, cone_w);
+              __syncwarp();
+              if (lane == 0) s_ck[warp][jj] = next;
+              __syncwarp();
+            }
+            const ChunkBox& cb = s_ck[warp][jj];
             const float a = cb.a, b = cb.b, rb = cb.rb, mr = cb.mr;
-            const int c0[3] = {cb.c0[0], cb.c0[1], cb.c0[2]};
-            const int c1[3] = {cb.c1[0], cb.c1[1], cb.c1[2]};
-            const int ny = c1[1] - c0[1] + 1;
+            const int ny = cb.c1[am] - cb.c0[am] + 1;
             const int nrows = cb.nrows;
             for (int rbase = 0; rbase < nrows; rbase += 32) {
-              // this lane's row: the part of the chunk within rb of its y/z band
+              // this lane's row: the part of the chunk within rb of its band
               int beg = 0, cnt = 0;
               const int ridx = rbase + lane;
               if (ridx < nrows) {
                 // one layer of cells (receivers on a plane) needs no division
-                const bool flat = c1[2] == c0[2];
-                const int iy = c0[1] + (flat ? ridx : ridx % ny);
-                const int iz = c0[2] + (flat ? 0 : ridx / ny);
-                const float y0 = g.org[1] + iy * g.cell - rb, y1 = g.org[1] + (iy + 1) * g.cell + rb;
-                const float z0 = g.org[2] + iz * g.cell - rb, z1 = g.org[2] + (iz + 1) * g.cell + rb;
+                const bool flat = cb.c1[al] == cb.c0[al];
+                const int im = cb.c0[am] + (flat ? ridx : ridx % ny);
+                const int il = cb.c0[al] + (flat ? 0 : ridx / ny);
+                const float y0 = g.org[am] + im * g.cell - rb, y1 = g.org[am] + (im + 1) * g.cell + rb;
+                const float z0 = g.org[al] + il * g.cell - rb, z1 = g.org[al] + (il + 1) * g.cell + rb;
                 float la = a, lb = b;
                 bool ok = true;
-                if (fabsf(u.y) > 1e-20f) {
-                  const float t1 = (y0 - s.y) * inv_uy, t2 = (y1 - s.y) * inv_uy;
+                if (fabsf(um) > 1e-20f) {
+                  const float t1 = (y0 - sm) * inv_um, t2 = (y1 - sm) * inv_um;
                   la = fmaxf(la, fminf(t1, t2));
                   lb = fminf(lb, fmaxf(t1, t2));
-                } else if (s.y < y0 || s.y > y1) {
+                } else if (sm < y0 || sm > y1) {
                   ok = false;
                 }
-                if (fabsf(u.z) > 1e-20f) {
-                  const float t1 = (z0 - s.z) * inv_uz, t2 = (z1 - s.z) * inv_uz;
+                if (fabsf(ul) > 1e-20f) {
+                  const float t1 = (z0 - sl) * inv_ul, t2 = (z1 - sl) * inv_ul;
                   la = fmaxf(la, fminf(t1, t2));
                   lb = fminf(lb, fmaxf(t1, t2));
-                } else if (s.z < z0 || s.z > z1) {
+                } else if (sl < z0 || sl > z1) {
                   ok = false;
                 }
                 if (ok && la <= lb) {
-                  const float xa = s.x + la * u.x, xb = s.x + lb * u.x;
-                  int x0 = max(c0[0], int(floorf((fminf(xa, xb) - rb - g.org[0]) * inv_cell)));
-                  int x1 = min(c1[0], int(floorf((fmaxf(xa, xb) + rb - g.org[0]) * inv_cell)));
+                  const float xa = sr + la * ur, xb = sr + lb * ur;
+                  int x0 = max(cb.c0[ar], int(floorf((fminf(xa, xb) - rb - g.org[ar]) * inv_cell)));
+                  int x1 = min(cb.c1[ar], int(floorf((fmaxf(xa, xb) + rb - g.org[ar]) * inv_cell)));
                   if (use_cone && x0 <= x1)
-                    cone_cells(cone_w, g, inv_cell, iy, iz, x0, x1);
+                    cone_cells(cone_w, g, inv_cell, im, il, x0, x1);
                   if (x0 <= x1) {
-                    const int row = (iz * g.dim[1] + iy) * g.dim[0];
+                    const int row = (il * g.dim[am] + im) * g.dim[ar];
                     beg = g.cell_start[row + x0];
                     cnt = g.cell_start[row + x1 + 1] - beg;
                   }
@@ -686,16 +705,24 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
   __shared__ NodeSpan s_sp[kCapWarps][B];   // clipped span and chunking
   __shared__ ChunkBox s_ck[kCapWarps][32];  // the current 32 (node, chunk) items
   __shared__ int s_ckn[kCapWarps][32];      // their node (batch index) | chunk << 8
-  for (WorkWindow work(A.work, (long long)n_nodes, B); work.refill(); work.next += B) {
+  // fewer nodes than the grid's lanes: fewer nodes per warp, so that each
+  // node's chunks still find a warp of their own (184 nodes of up to 250
+  // chunks on 6 warps took 1.9 ms)
+  const long long warps = (long long)gridDim.x * kCapWarps;
+  const int batch = int(min((long long)B, max(1ll, ((long long)n_nodes + warps - 1) / warps)));
+  for (WorkWindow work(A.work, (long long)n_nodes, batch); work.refill();) {
     const unsigned long long base = work.next;
+    const int n_here = int(min((long long)batch, work.end - work.next));
+    work.next += n_here;
     int nck = 0;  // chunks of this lane's node
     {
       const unsigned long long my = base + lane;
-      if (lane < B && my < n_nodes) {
+      if (lane < n_here) {
         const NodeHot h = A.nodes[my];
         s_nh[warp][lane] = StagedNode{{h.s[0], h.s[1], h.s[2]}, h.S, {h.u[0], h.u[1], h.u[2]},
                                       h.len, h.cls, h.tx};
         const float cmax = A.gb[h.tx].cmax;
+        const int ar = A.grids[h.tx].ax[0];
         int cone_ok = 0;
         if (!is_root_class(h.cls)) {
           const ClassCap c = A.cls_cap[h.cls];
@@ -713,7 +740,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
             cn[4 * k + 1] = c.n[k][1];
             cn[4 * k + 2] = c.n[k][2];
             cn[4 * k + 3] = c.n[k][3] - 2.0f * m;
-            cn[12 + k] = c.inv_nx[k];
+            cn[12 + k] = 1.0f / (ar == 0 ? c.n[k][0] : (ar == 1 ? c.n[k][1] : c.n[k][2]));
           }
         }
         const NodeSpan sp = node_span(h, A.txp[h.tx], A.grids[h.tx], cmax, cone_ok);
@@ -756,45 +783,46 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
           const int jn = s_ckn[warp][ci] & 0xff;
           const StagedNode& nd = s_nh[warp][jn];
           const RxGrid& g = A.grids[nd.tx];
-          const float3 s = make_float3(nd.s[0], nd.s[1], nd.s[2]);
-          const float3 u = make_float3(nd.u[0], nd.u[1], nd.u[2]);
+          const int ar = g.ax[0], am = g.ax[1], al = g.ax[2];
+          const float sr = nd.s[ar], sm = nd.s[am], sl = nd.s[al];
+          const float ur = nd.u[ar], um = nd.u[am], ul = nd.u[al];
           // Reciprocals for the cell-range arithmetic: every range is widened
           // by at least 2e-3 m + cell/100, far more than the few ulps a product
           // with a reciprocal differs from the quotient.
-          const float inv_uy = __frcp_rn(u.y), inv_uz = __frcp_rn(u.z);
+          const float inv_um = __frcp_rn(um), inv_ul = __frcp_rn(ul);
           const float rb = cb.rb;
-          const int ny = cb.c1[1] - cb.c0[1] + 1;
+          const int ny = cb.c1[am] - cb.c0[am] + 1;
           // one layer of cells (receivers on a plane) needs no division
-          const bool flat = cb.c1[2] == cb.c0[2];
-          const int iy = cb.c0[1] + (flat ? ridx : ridx % ny);
-          const int iz = cb.c0[2] + (flat ? 0 : ridx / ny);
-          const float y0 = g.org[1] + iy * g.cell - rb, y1 = g.org[1] + (iy + 1) * g.cell + rb;
-          const float z0 = g.org[2] + iz * g.cell - rb, z1 = g.org[2] + (iz + 1) * g.cell + rb;
+          const bool flat = cb.c1[al] == cb.c0[al];
+          const int im = cb.c0[am] + (flat ? ridx : ridx % ny);
+          const int il = cb.c0[al] + (flat ? 0 : ridx / ny);
+          const float y0 = g.org[am] + im * g.cell - rb, y1 = g.org[am] + (im + 1) * g.cell + rb;
+          const float z0 = g.org[al] + il * g.cell - rb, z1 = g.org[al] + (il + 1) * g.cell + rb;
           float la = cb.a, lb = cb.b;
           bool ok = true;
-          if (fabsf(u.y) > 1e-20f) {
-            const float t1 = (y0 - s.y) * inv_uy, t2 = (y1 - s.y) * inv_uy;
+          if (fabsf(um) > 1e-20f) {
+            const float t1 = (y0 - sm) * inv_um, t2 = (y1 - sm) * inv_um;
             la = fmaxf(la, fminf(t1, t2));
             lb = fminf(lb, fmaxf(t1, t2));
-          } else if (s.y < y0 || s.y > y1) {
+          } else if (sm < y0 || sm > y1) {
             ok = false;
           }
-          if (fabsf(u.z) > 1e-20f) {
-            const float t1 = (z0 - s.z) * inv_uz, t2 = (z1 - s.z) * inv_uz;
+          if (fabsf(ul) > 1e-20f) {
+            const float t1 = (z0 - sl) * inv_ul, t2 = (z1 - sl) * inv_ul;
             la = fmaxf(la, fminf(t1, t2));
             lb = fminf(lb, fmaxf(t1, t2));
-          } else if (s.z < z0 || s.z > z1) {
+          } else if (sl < z0 || sl > z1) {
             ok = false;
           }
           if (ok && la <= lb) {
             const float inv_cell = g.inv_cell;
-            const float xa = s.x + la * u.x, xb = s.x + lb * u.x;
-            int x0 = max(cb.c0[0], int(floorf((fminf(xa, xb) - rb - g.org[0]) * inv_cell)));
-            int x1 = min(cb.c1[0], int(floorf((fmaxf(xa, xb) + rb - g.org[0]) * inv_cell)));
+            const float xa = sr + la * ur, xb = sr + lb * ur;
+            int x0 = max(cb.c0[ar], int(floorf((fminf(xa, xb) - rb - g.org[ar]) * inv_cell)));
+            int x1 = min(cb.c1[ar], int(floorf((fmaxf(xa, xb) + rb - g.org[ar]) * inv_cell)));
             if (s_sp[warp][jn].use_cone && x0 <= x1)
-              cone_cells(s_cn[warp][jn], g, inv_cell, iy, iz, x0, x1);
+              cone_cells(s_cn[warp][jn], g, inv_cell, im, il, x0, x1);
             if (x0 <= x1) {
-              const int row = (iz * g.dim[1] + iy) * g.dim[0];
+              const int row = (il * g.dim[am] + im) * g.dim[ar];
               beg = g.cell_start[row + x0];
               cnt = g.cell_start[row + x1 + 1] - beg;
             }

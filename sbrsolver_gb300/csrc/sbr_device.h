@@ -164,6 +164,8 @@ struct TxParams {
 struct RxGrid {
   float org[3], cell;
   int dim[3];
+  int ax[3];       // row axis (the one with most cells), then the other two: cells of a
+                   // row are consecutive, rows along ax[1], layers along ax[2]
   float inv_cell;  // 1 / cell
   float chunk_len; // minimum chunk length along a node's segment in capture (m)
   const int* cell_start;  // ncell + 1
@@ -203,7 +205,6 @@ struct __align__(16) ClassCap {
   float nn[3];     // |n_k|
   float w[3];      // |n_k| (|img| + |T| + 1)
   float gc[3];     // |n_k . (centroid - img)|
-  float inv_nx[3]; // 1 / n_k.x
 };
 
 // A capture whose image correction succeeded (one reference path before

@@ -138,6 +138,12 @@ __global__ void k_grid_shape(GridBuild* gb, RxGrid* grids, const TxParams* txp, 
       g.bmin[a] = lo[a];
       g.bmax[a] = hi[a];
     }
+    // rows run along the axis with most cells: a capture test takes a row of
+    // cells per lane, and receivers on a line along y would otherwise lie in
+    // thousands of rows of one cell (3,000 on a line: 11.3 ms of capture)
+    g.ax[0] = dim[1] > dim[0] ? (dim[2] > dim[1] ? 2 : 1) : (dim[2] > dim[0] ? 2 : 0);
+    g.ax[1] = g.ax[0] == 1 ? 0 : 1;
+    g.ax[2] = g.ax[0] == 2 ? 0 : 2;
     g.cell = cell;
     g.inv_cell = 1.0f / cell;
     g.chunk_len = float(k < 3 ? SBR_CAP_CHUNK_CELLS_FLAT : SBR_CAP_CHUNK_CELLS) * cell;
@@ -150,10 +156,10 @@ __global__ void k_grid_shape(GridBuild* gb, RxGrid* grids, const TxParams* txp, 
 }
 
 __device__ __forceinline__ int cell_of(const RxGrid& g, float x, float y, float z) {
-  int ix = min(g.dim[0] - 1, max(0, int((x - g.org[0]) / g.cell)));
-  int iy = min(g.dim[1] - 1, max(0, int((y - g.org[1]) / g.cell)));
-  int iz = min(g.dim[2] - 1, max(0, int((z - g.org[2]) / g.cell)));
-  return (iz * g.dim[1] + iy) * g.dim[0] + ix;
+  const int i[3] = {min(g.dim[0] - 1, max(0, int((x - g.org[0]) / g.cell))),
+                    min(g.dim[1] - 1, max(0, int((y - g.org[1]) / g.cell))),
+                    min(g.dim[2] - 1, max(0, int((z - g.org[2]) / g.cell)))};
+  return (i[g.ax[2]] * g.dim[g.ax[1]] + i[g.ax[1]]) * g.dim[g.ax[0]] + i[g.ax[0]];
 }
 
 __global__ void k_rx_count(const double* rx, const TxParams* txp, int n_tx, const RxGrid* grids,

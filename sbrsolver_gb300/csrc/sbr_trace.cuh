@@ -114,7 +114,6 @@ __global__ void k_class_cones(const uint32_t* list, const Counters* ctr, uint32_
       cc.nn[k] = float(nn * (1.0 + 1e-6));
       cc.w[k] = cc.nn[k] * tmag;
       cc.gc[k] = float(fabs(gc));
-      cc.inv_nx[k] = 1.0f / cc.n[k][0];
     }
   }
 }
