@@ -1629,7 +1629,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     CK(cudaEventRecord(W.fork, st));
     CK(cudaStreamWaitEvent(W.side, W.fork, 0));
     if (rx_total)
-      ++nl, k_direct<<<grid_for(rx_total, 64), 64, 0, W.side>>>(S.dev, W.txp.p, W.rx.p, W.rx_req.p,
+      ++nl, k_direct<<<grid_for(rx_total, 32), 32, 0, W.side>>>(S.dev, W.txp.p, W.rx.p, W.rx_req.p,
                                                              rx_total, W.direct_ok.p, W.ctr.p);
     CK(cudaEventRecord(W.join, W.side));
     // ---- trace

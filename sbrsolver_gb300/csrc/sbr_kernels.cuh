@@ -310,28 +310,26 @@ __device__ __forceinline__ int tri_classify(const Tri32& T, const float3& o, con
   const float qz = sx * T.e1[1] - sy * T.e1[0];
   float V = d.x * qx + d.y * qy + d.z * qz;
   float W = T.e2[0] * qx + T.e2[1] * qy + T.e2[2] * qz;
-  const float ns = no + T.nv1;
-  const float ea = kFiltK * T.ne1 * T.ne2 * nd;
-  const float eU = kFiltK * ns * nd * T.ne2;
-  const float eV = kFiltK * ns * T.ne1 * nd;
-  const float eW = kFiltK * ns * T.ne1 * T.ne2;
+  const float k = kFiltK * (no + T.nv1), kd = k * nd;
+  const float eU = kd * T.ne2, eV = kd * T.ne1, eW = k * T.ne2 * T.ne1;
+  const float ea = kFiltK * nd * T.ne1 * T.ne2;
   const float A = fabsf(a);
-  if (A <= kEps32 + ea) {
+  U = copysignf(1.0f, a) * U;
+  V = copysignf(1.0f, a) * V;
+  W = copysignf(1.0f, a) * W;
+  // one decision at the end: the lanes of a warp reject for different reasons
+  const bool miss = U < -eU || V < -eV || U + V > A + ea + eU + eV ||
+                    W + eW <= (kEps32 * 0.5f) * (A - ea);
+  if (A <= kEps32 + ea) {  // near-parallel: the FP64 test decides
     tlo = 0.0f;
     thi = INFINITY;
     return kMayHit;
   }
-  if (a < 0.0f) {
-    U = -U;
-    V = -V;
-    W = -W;
-  }
-  if (U < -eU || V < -eV) return 0;
-  if (U > A + ea + eU) return 0;
-  if (U + V > A + ea + eU + eV) return 0;
-  thi = (W + eW) / (A - ea);
-  if (thi <= kEps32 * 0.5f) return 0;
-  tlo = (W - eW) / (A + ea);
+  if (miss) return 0;
+  // (approximate quotients: the margins exceed W's and a's errors by more than
+  // 2^-19 of W and A, the quotient's error is 2^-22)
+  thi = __fdividef(W + eW, A - ea);
+  tlo = __fdividef(W - eW, A + ea);
   const bool uv = U > eU && V > eV && U + V < A - ea - eU - eV;
   return kMayHit | (uv ? (tlo > 2.0f * kEps32 ? kSureUV | kSureHit : kSureUV) : 0);
 }
@@ -651,6 +649,79 @@ constexpr unsigned char kFindFallback = 0xFF;
 // direction is outside soft64's range; kFindFallback as a whole.
 constexpr int kCandCount = 0x0F, kCandUnsafe = 0x40;
 constexpr unsigned kContUV = 0x80000000u;  // contender's rank: u and v are sure (kSureUV)
+
+// A ray prepared for the search BVH's slab tests: along axis a a plane at b is
+// crossed at b * inv[a] + off, with off_near / off_far holding -(o +- m) / d,
+// the box expansion m folded in.  One fused operation per plane, no near/far
+// exchange: the near plane of a box is its low one where d > 0, else its high
+// one, picked by address.  Rounding (off to 2 units, the product with inv's
+// error common to both terms) moves a plane by under 5 * 2^-24 (|b| + |o| + m),
+// far inside m = 2^-14 (extent + 1 + |o|).  A component below 1e-18 counts as
+// 1e-18: products stay finite and a box is kept iff the origin is within m of
+// its slab, as with an infinite reciprocal.
+struct SlabRay {
+  float inv[3], off_near[3], off_far[3];
+  int near;  // bit a: the near plane along axis a is the high one
+};
+__device__ __forceinline__ SlabRay slab_ray(const float3& o, const float3& d, float m) {
+  SlabRay r;
+  r.near = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float oa = a == 0 ? o.x : (a == 1 ? o.y : o.z);
+    const float da = a == 0 ? d.x : (a == 1 ? d.y : d.z);
+    const float inv = 1.0f / (fabsf(da) < 1e-18f ? copysignf(1e-18f, da) : da);
+    const float sm = copysignf(m, da);
+    r.inv[a] = inv;
+    r.off_near[a] = -(oa + sm) * inv;
+    r.off_far[a] = -(oa - sm) * inv;
+    r.near |= signbit(da) ? 1 << a : 0;
+  }
+  return r;
+}
+
+// The children of a four-wide node that the ray's slab test keeps within
+// [0, tcut], nearest first; returns how many (c[0..n)).
+__device__ __forceinline__ int visit_node4(const Node4* node, const SlabRay& r, float tcut,
+                                           int c[4]) {
+  const float4* p = reinterpret_cast<const float4*>(node);
+  const int sx = r.near & 1 ? 3 : 0, sy = r.near & 2 ? 3 : 0, sz = r.near & 4 ? 3 : 0;
+  const float4 nx = __ldg(p + sx), ny = __ldg(p + 1 + sy), nz = __ldg(p + 2 + sz);
+  const float4 fx = __ldg(p + 3 - sx), fy = __ldg(p + 4 - sy), fz = __ldg(p + 5 - sz);
+  const int4 cr = __ldg(reinterpret_cast<const int4*>(p + 6));
+  auto visit = [&](float ax, float ay, float az, float bx, float by, float bz, int child,
+                   float& t) -> int {
+    const float tn = fmaxf(fmaxf(fmaf(ax, r.inv[0], r.off_near[0]), fmaf(ay, r.inv[1], r.off_near[1])),
+                           fmaxf(fmaf(az, r.inv[2], r.off_near[2]), 0.0f));
+    const float tf = fminf(fminf(fmaf(bx, r.inv[0], r.off_far[0]), fmaf(by, r.inv[1], r.off_far[1])),
+                           fminf(fmaf(bz, r.inv[2], r.off_far[2]), tcut));
+    const bool h = tn <= tf;  // an absent child's planes are at infinity the wrong way round
+    t = h ? tn : INFINITY;
+    return h ? child : kEmptyChild;
+  };
+  float t0, t1, t2, t3;
+  c[0] = visit(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, cr.x, t0);
+  c[1] = visit(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, cr.y, t1);
+  c[2] = visit(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, cr.z, t2);
+  c[3] = visit(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, cr.w, t3);
+  auto order = [](float& ta, int& ca, float& tb, int& cb) {
+    if (tb < ta) {
+      const float t = ta;
+      ta = tb;
+      tb = t;
+      const int x = ca;
+      ca = cb;
+      cb = x;
+    }
+  };
+  order(t0, c[0], t1, c[1]);  // sorting network for four
+  order(t2, c[2], t3, c[3]);
+  order(t0, c[0], t2, c[2]);
+  order(t1, c[1], t3, c[3]);
+  order(t1, c[1], t2, c[2]);
+  return int(c[0] != kEmptyChild) + int(c[1] != kEmptyChild) + int(c[2] != kEmptyChild) +
+         int(c[3] != kEmptyChild);
+}
 
 // Whether the reference's test of the triangle a ray starts on certainly
 // fails (so its FP64 test can be skipped).  The ray's origin is the hit
