@@ -113,13 +113,20 @@ __device__ __forceinline__ float sqrt_up(float x) {
 // (MultiPathCorrection's first test for a capture at c; RTSolver.cpp:356).
 // Three planes through img and T's edges, n_k . p >= n_k . img, formed once
 // per class in FP64 and rounded to FP32 (k_class_cones); k_capture loosens
-// each by 2 m_k, m_k = 2^-19 |n_k| (cmax + |img| + |T| + 1).  The FP32 test
+// each by 2 m_k, m_k = 2^-21 |n_k| (cmax + |img| + |T| + 1).  The FP32 test
 // of a point p (|p| <= cmax) or of a cell corner errs by under
 // 10 * 2^-24 |n_k| (cmax + |img| + |T|): the plane's rounding, the rounding
-// of p, and the dot product.  No cone is used when a plane is
-// ill-conditioned (the centroid within 4 m_k of it).  The reference's FP64 test accepts
+// of p, and the dot product.  A plane counts as long as FP64 settles its
+// orientation (k_class_cones); under the loosening a thin cone is merely
+// thicker than it could be.  (Dropping every cone with the centroid within
+// four 2^-19 margins of a plane left 71 % of the level-10 terrain's receiver
+// candidates, behind small triangles seen at a grazing angle, without one:
+// k_capture_fast 13.0 ms, with them 12.1.)
+// The reference's FP64 test accepts
 // only points inside the exact cone, so receivers outside the loosened one
 // are skipped without changing a result.
+
+constexpr float kConeK = 4.76837158203125e-07f;  // 2^-21
 
 // Whether the box [lo, hi] may hold a point of the cone.
 __device__ __forceinline__ bool cone_meets_box(const float* cone, const float* lo, const float* hi) {
@@ -328,12 +335,12 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
           float* fl = s_fl[warp][lane];
           for (int q = 0; q < 3; ++q) fl[q] = c.img[q];
           for (int q = 0; q < 8; ++q) fl[3 + q] = c.F[q];
-          // the cone's planes loosened by 2 m, m = 2^-19 |n| (cmax + |img| + |T| + 1)
+          // the cone's planes loosened by 2 m, m = 2^-21 |n| (cmax + |img| + |T| + 1)
           float* cn = s_cn[warp][lane];
           cone_ok = !kStage;
           for (int k = 0; k < 3; ++k) {
-            const float m = 1.9073486328125e-06f * (c.nn[k] * cmax + c.w[k]);
-            cone_ok &= (c.gc[k] > 4.0f * m && isfinite(m)) ? 1 : 0;
+            const float m = kConeK * (c.nn[k] * cmax + c.w[k]);
+            cone_ok &= (c.gc[k] > 0.0f && isfinite(m)) ? 1 : 0;
             cn[4 * k + 0] = c.n[k][0];
             cn[4 * k + 1] = c.n[k][1];
             cn[4 * k + 2] = c.n[k][2];
@@ -607,8 +614,11 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
 // Items of a work counter handed to a warp, a window at a time: every warp of
 // the grid asks the same counter, which serves an atomic in about 0.65 ns, so
 // a warp takes a part of what was left when it last asked (at least
-// `smallest`, a multiple of 32, at most 256 items) and the windows shrink
-// towards the end, where an uneven last one would leave warps waiting.
+// `smallest`, a multiple of 32) and the windows shrink
+// towards the end, where an uneven last one would leave warps waiting.  At
+// most 64 items: costly nodes lie next to each other, and a warp that drew
+// 256 of them held up the level-10 terrain's capture (12.2 ms; 128: 8.0,
+// 64 and 32: 7.1).
 struct WorkWindow {
   unsigned long long* counter;
   long long next, end, n;  // the window's rest; items in all
@@ -623,7 +633,7 @@ struct WorkWindow {
   __device__ __forceinline__ bool refill() {
     if (next < end) return true;
     if (next >= n && end > 0) return false;
-    const int size = min(256, max(smallest, 32 * int(float(n - next) * share)));
+    const int size = min(64, max(smallest, 32 * int(float(n - next) * share)));
     unsigned long long base = 0;
     if (lane_id() == 0) base = atomicAdd(counter, (unsigned long long)size);
     next = (long long)__shfl_sync(0xffffffffu, base, 0);
@@ -730,12 +740,12 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
           float* fl = s_fl[warp][lane];
           for (int q = 0; q < 3; ++q) fl[q] = c.img[q];
           for (int q = 0; q < 8; ++q) fl[3 + q] = c.F[q];
-          // the cone's planes loosened by 2 m, m = 2^-19 |n| (cmax + |img| + |T| + 1)
+          // the cone's planes loosened by 2 m, m = 2^-21 |n| (cmax + |img| + |T| + 1)
           float* cn = s_cn[warp][lane];
           cone_ok = 1;
           for (int k = 0; k < 3; ++k) {
-            const float m = 1.9073486328125e-06f * (c.nn[k] * cmax + c.w[k]);
-            cone_ok &= (c.gc[k] > 4.0f * m && isfinite(m)) ? 1 : 0;
+            const float m = kConeK * (c.nn[k] * cmax + c.w[k]);
+            cone_ok &= (c.gc[k] > 0.0f && isfinite(m)) ? 1 : 0;
             cn[4 * k + 0] = c.n[k][0];
             cn[4 * k + 1] = c.n[k][1];
             cn[4 * k + 2] = c.n[k][2];

@@ -204,7 +204,7 @@ struct __align__(16) ClassCap {
   float n[3][4];   // cone plane k: oriented normal, n . img
   float nn[3];     // |n_k|
   float w[3];      // |n_k| (|img| + |T| + 1)
-  float gc[3];     // |n_k . (centroid - img)|
+  float gc[3];     // |n_k . (centroid - img)|, 0 where plane k cannot be used
 };
 
 // A capture whose image correction succeeded (one reference path before

@@ -95,6 +95,7 @@ __global__ void k_class_cones(const uint32_t* list, const Counters* ctr, uint32_
     const double* im = ci.img;
     const double g[3] = {(v[0][0] + v[1][0] + v[2][0]) / 3.0, (v[0][1] + v[1][1] + v[2][1]) / 3.0,
                          (v[0][2] + v[1][2] + v[2][2]) / 3.0};
+    auto ab2 = [](const double* x) { return x[0] * x[0] + x[1] * x[1] + x[2] * x[2]; };
     auto norm3 = [](const double* x) { return sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]); };
     const float tmag =
         float((norm3(im) + norm3(T.v1) + norm3(T.e1) + norm3(T.e2)) * (1.0 + 1e-6)) + 1.0f;
@@ -113,7 +114,11 @@ __global__ void k_class_cones(const uint32_t* list, const Counters* ctr, uint32_
       cc.n[k][3] = float(sg * (n[0] * im[0] + n[1] * im[1] + n[2] * im[2]));
       cc.nn[k] = float(nn * (1.0 + 1e-6));
       cc.w[k] = cc.nn[k] * tmag;
-      cc.gc[k] = float(fabs(gc));
+      // FP64 forms n to within 2^-50 |a||b| and gc to within that times the
+      // distance: the plane is used where both are far below what they are
+      // compared with (n's FP32 rounding, gc's sign)
+      const double ab = sqrt(ab2(a) * ab2(b));
+      cc.gc[k] = nn > 1e-6 * ab && fabs(gc) > 4e-9 * nn * double(tmag) ? float(fabs(gc)) : 0.0f;
     }
   }
 }
