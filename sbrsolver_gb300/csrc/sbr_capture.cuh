@@ -25,7 +25,9 @@ struct CaptureArgs {
   const NodeHot* nodes;
   const NodeCold* nodes_cold;
   const TxParams* txp;
-  const RxGrid* grids;
+  const RxGrid* grids;  // per request, all receivers; then per request, those with a direct
+                        // path, for the launch rays' own segments
+  int n_tx;
   const GridBuild* gb;
   const double* rx;
   const ClassInfo* cls_info;
@@ -184,14 +186,13 @@ struct NodeSpan {
 // |P| <= (cmax + S tan b) / (1 - tan b) for any capturing point).  All
 // ranges are widened well beyond their FP32 rounding.
 template <class Node>
-__device__ __forceinline__ NodeSpan node_span(const Node& nd, const TxParams& P,
-                                              const RxGrid& g, float cmax, int use_cone) {
+__device__ __forceinline__ NodeSpan node_span(const Node& nd, const RxGrid& g, int use_cone) {
   NodeSpan sp{0.0f, -1.0f, 0.0f, 0.0f, 0, use_cone};
-  if (P.n_rx <= 0) return sp;
+  if (g.n <= 0) return sp;
   const float3 s = make_float3(nd.s[0], nd.s[1], nd.s[2]);
   const float3 u = make_float3(nd.u[0], nd.u[1], nd.u[2]);
   const float len = nd.len, S = nd.S;
-  const float tanb = P.tan_beta32;
+  const float tanb = g.tanb, cmax = g.cmax;
   const float pmax = __fdividef(cmax + S * tanb, fmaxf(1e-6f, 1.0f - tanb)) * 1.0001f + 1.0f;
   const float su = s.x * u.x + s.y * u.y + s.z * u.z;
   const float ss = s.x * s.x + s.y * s.y + s.z * s.z;
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
             cn[12 + k] = 1.0f / (ar == 0 ? c.n[k][0] : (ar == 1 ? c.n[k][1] : c.n[k][2]));
           }
         }
-        const NodeSpan sp = node_span(h, A.txp[h.tx], A.grids[h.tx], cmax, cone_ok);
+        const NodeSpan sp = node_span(h, A.grids[h.tx], cone_ok);
         s_sp[warp][lane] = sp;
         if (sp.nchunk > 0)
           s_ck[warp][lane] = chunk_box(h, A.grids[h.tx], sp, 0, cmax, A.txp[h.tx].tan_beta32,
@@ -680,7 +681,7 @@ constexpr int kFastB = 32;  // nodes staged per warp and batch (one per lane)
 // What the fast path keeps of a node in shared memory.
 struct StagedNode {
   float s[3], S, u[3], len;
-  uint32_t cls, tx;
+  uint32_t cls, grid;  // grid: its receivers' grid (CaptureArgs::grids)
 };
 
 // Pairs for k_capture_finish, gathered per warp so that one atomic on the pair
@@ -729,10 +730,12 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
       const unsigned long long my = base + lane;
       if (lane < n_here) {
         const NodeHot h = A.nodes[my];
+        const uint32_t gi = h.tx + (is_root_class(h.cls) ? A.n_tx : 0);
         s_nh[warp][lane] = StagedNode{{h.s[0], h.s[1], h.s[2]}, h.S, {h.u[0], h.u[1], h.u[2]},
-                                      h.len, h.cls, h.tx};
-        const float cmax = A.gb[h.tx].cmax;
-        const int ar = A.grids[h.tx].ax[0];
+                                      h.len, h.cls, gi};
+        const RxGrid& g = A.grids[gi];
+        const float cmax = g.cmax;
+        const int ar = g.ax[0];
         int cone_ok = 0;
         if (!is_root_class(h.cls)) {
           const ClassCap c = A.cls_cap[h.cls];
@@ -753,7 +756,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
             cn[12 + k] = 1.0f / (ar == 0 ? c.n[k][0] : (ar == 1 ? c.n[k][1] : c.n[k][2]));
           }
         }
-        const NodeSpan sp = node_span(h, A.txp[h.tx], A.grids[h.tx], cmax, cone_ok);
+        const NodeSpan sp = node_span(h, g, cone_ok);
         s_sp[warp][lane] = sp;
         nck = sp.nchunk;
       }
@@ -771,8 +774,9 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
         const int ch = k - (j_incl - j_n);
         const StagedNode& nd = s_nh[warp][j];
         const NodeSpan& sp = s_sp[warp][j];
-        const ChunkBox cb = chunk_box(nd, A.grids[nd.tx], sp, ch, A.gb[nd.tx].cmax,
-                                      A.txp[nd.tx].tan_beta32, sp.use_cone != 0, s_cn[warp][j]);
+        const RxGrid& g = A.grids[nd.grid];
+        const ChunkBox cb = chunk_box(nd, g, sp, ch, g.cmax, g.tanb, sp.use_cone != 0,
+                                      s_cn[warp][j]);
         s_ck[warp][lane] = cb;
         s_ckn[warp][lane] = j | ch << 8;
         nrows = cb.nrows;
@@ -792,7 +796,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
           const ChunkBox& cb = s_ck[warp][ci];
           const int jn = s_ckn[warp][ci] & 0xff;
           const StagedNode& nd = s_nh[warp][jn];
-          const RxGrid& g = A.grids[nd.tx];
+          const RxGrid& g = A.grids[nd.grid];
           const int ar = g.ax[0], am = g.ax[1], al = g.ax[2];
           const float sr = nd.s[ar], sm = nd.s[am], sl = nd.s[al];
           const float ur = nd.u[ar], um = nd.u[am], ul = nd.u[al];
@@ -856,7 +860,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
             const StagedNode& nd = s_nh[warp][jn];
             const NodeSpan& sp = s_sp[warp][jn];
             const float a = s_ck[warp][rci].a, b = s_ck[warp][rci].b, mr = s_ck[warp][rci].mr;
-            const RxGrid& g = A.grids[nd.tx];
+            const RxGrid& g = A.grids[nd.grid];
             const float3 s = make_float3(nd.s[0], nd.s[1], nd.s[2]);
             const float3 u = make_float3(nd.u[0], nd.u[1], nd.u[2]);
             const float4 c4 = g.rx32[rbeg + (q - (rincl - rcnt))];
@@ -867,9 +871,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
             if (ch < sp.nchunk - 1 && lam >= b) return false;    // owned by a later chunk
             const int gi = __float_as_int(c4.w);
             ++cand;
-            if (is_root_class(nd.cls)) {
-              if (!A.direct_ok[gi]) return false;
-            } else {
+            if (!is_root_class(nd.cls)) {
               // MultiPathCorrection's last step must cross the class's last
               // triangle: FP32 filter from the image source towards the receiver
               const float* fl = s_fl[warp][jn];
@@ -879,14 +881,14 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
                                    sqrt_up(dd.x * dd.x + dd.y * dd.y + dd.z * dd.z)))
                 return false;
             }
-            const float tanb = A.txp[nd.tx].tan_beta32;
+            const float tanb = g.tanb;
             const float len = nd.len, S = nd.S;
             int v;
             if (lam < a || lam > b) {
               // outside the chunk's own range: full-margin test
               v = reception32(s, u, len, S, c, tanb);
             } else {
-              const float ml = kRecK * (sp.ns + A.gb[nd.tx].cmax + 1.0f);
+              const float ml = kRecK * (sp.ns + g.cmax + 1.0f);
               if (lam < -ml) {
                 v = 0;
               } else if (lam <= ml) {

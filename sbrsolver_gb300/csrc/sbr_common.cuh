@@ -117,10 +117,30 @@ __device__ __forceinline__ uint32_t ht_find(HashTable t, unsigned long long key)
   return 0xFFFFFFFFu;
 }
 
-__global__ void k_fill_u64(unsigned long long* p, size_t n, unsigned long long v) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * blockDim.x)
-    p[i] = v;
+// Sets every range of the list to its byte value, all in one launch: a solve
+// clears some twenty tables and counters, and as separate fills and memsets
+// they cost a small solve more than its capture.
+struct FillRange {
+  unsigned char* p;
+  unsigned long long bytes;
+  unsigned value;  // the byte, four times
+};
+constexpr int kFillRanges = 24;
+struct FillList {
+  FillRange r[kFillRanges];
+  int n;
+};
+__global__ void __launch_bounds__(256) k_fill(const __grid_constant__ FillList L) {
+  const unsigned long long t0 = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+  for (int k = 0; k < L.n; ++k) {
+    const FillRange R = L.r[k];
+    const unsigned long long words = R.bytes >> 4;
+    uint4* w = reinterpret_cast<uint4*>(R.p);  // allocations are 256-byte aligned
+    for (unsigned long long i = t0; i < words; i += step)
+      w[i] = make_uint4(R.value, R.value, R.value, R.value);
+    if (t0 < (R.bytes & 15)) R.p[(words << 4) + t0] = (unsigned char)R.value;
+  }
 }
 
 }  // namespace sbr

@@ -171,6 +171,9 @@ struct RxGrid {
   const int* cell_start;  // ncell + 1
   const float4* rx32;     // sorted by cell: xyz, w = receiver index (int bits)
   float bmin[3], bmax[3];
+  int n;           // receivers in the grid
+  float tanb;      // TxParams::tan_beta32 of the request
+  float cmax;      // max |receiver| of the request (all of its receivers)
 };
 
 struct HashTable {

@@ -156,17 +156,18 @@ struct Workspace {
   cudaEvent_t fork = nullptr, join = nullptr;
   cudaEvent_t cap_ev[2] = {};  // around the capture kernel
   std::vector<cudaEvent_t> tr_ev;  // before and after each k_trace launch
-  DBuf<TxParams> txp;
-  DBuf<double> rx;
-  DBuf<int> rx_req;
+  DBuf<unsigned char> up;  // a solve's uploads, one copy: txp | gb | direct gb | rx_req | rx
   DBuf<int> rx_bad;  // set when a device-resident receiver has a non-finite coordinate
   DBuf<double> path_bound, field_bound;  // FP32 field mode: error bounds per path / receiver
   DBuf<int> rx_flag;                     // FP32 field mode: receivers recomputed in FP64
   DBuf<unsigned long long> fstat;
-  DBuf<GridBuild> gb;
-  DBuf<RxGrid> grids;
-  DBuf<int> cell_base, cell_counts, cell_starts, cell_cursor;
-  DBuf<float4> rx32;
+  // a receiver grid (all receivers, or those with a direct path)
+  struct Grid {
+    DBuf<int> base, counts, starts, sums;  // counts: the cells' counts, then their cursors
+    DBuf<float4> rx32;
+  };
+  Grid all, direct;
+  DBuf<RxGrid> grids;  // per request, all; then per request, direct
   DBuf<RayRec> q0, q1;
   DBuf<RayF32> ray32;                  // FP32 copies of a chunk's rays (k_find -> k_trace)
   DBuf<NodeHot> nodes;
@@ -191,12 +192,9 @@ struct Workspace {
   DBuf<unsigned long long> seg_tx;
   DBuf<uint2> cand;                    // FP32 search contenders, kCand per ray of a chunk
   DBuf<unsigned char> ncand;
-  DBuf<unsigned long long> find_work;  // work counter of the running search launch
-  // pinned staging of a solve's uploads
-  HBuf<TxParams> h_txp;
-  HBuf<int> h_rxreq;
-  HBuf<double> h_rx;
-  HBuf<GridBuild> h_gb;
+  DBuf<unsigned long long> find_work;  // work counters: two per search/resolution launch
+                                       // pair, one for the capture
+  HBuf<unsigned char> h_up;   // pinned staging of a solve's uploads (up)
   HBuf<unsigned char> h_res;  // a solve's results on their way to the host
   // the device pipeline as a CUDA graph: captured the second time the same
   // pipeline (pipeline_key) runs, replayed whenever it comes again.  A few
@@ -750,6 +748,21 @@ static void swap_buf(DBuf<T>& a, DBuf<T>& b) {
 
 // Exclusive scan of in[0, n) into out[0, n], out[n] = total, over many
 // blocks; sums: scratch of at least n / kScanTile + 1 ints.
+// Exclusive scan of a solve's counts: one block up to kScanOne items, else three
+// launches over many blocks (sums: a tile total each); returns the launches.
+// (One block over the level-10 terrain's 400,000 cells took 361 us, the three
+// launches 14; at 4,096 items one block takes 4 us and the three 9.)
+static int scan_ints(const int* in, int* out, int n, int* sums, cudaStream_t st) {
+  if (n <= kScanOne) {
+    k_scan_exclusive<<<1, 1024, 0, st>>>(in, out, n);
+    return 1;
+  }
+  const int nb = (n + kScanTile - 1) / kScanTile;
+  k_tile_sums<<<nb, kScanThreads, 0, st>>>(in, n, sums);
+  k_sums_scan<<<1, 1024, 0, st>>>(sums, nb, out + n);
+  k_tile_scan<<<nb, kScanThreads, 0, st>>>(in, n, sums, out);
+  return 3;
+}
 static void scan_exclusive(const int* in, int* out, int n, int* sums, cudaStream_t st) {
   const int nb = std::max(1, (n + kScanTile - 1) / kScanTile);
   k_tile_sums<<<nb, kScanThreads, 0, st>>>(in, n, sums);
@@ -1259,9 +1272,11 @@ static std::string pipeline_key(const SceneImpl& S, const Workspace& W, const sb
   const unsigned long long caps[9] = {W.cap_nodes, W.cap_queue, W.cap_cls, W.cap_cop, W.cap_dd,
                                       W.cap_cc,    W.cap_corr,  W.cap_surv, W.cap_pairs};
   put(caps, sizeof caps);
-  const void* ptrs[] = {W.txp.p, W.rx.p, W.rx_req.p, W.rx_bad.p, W.path_bound.p, W.field_bound.p,
-                        W.rx_flag.p, W.fstat.p, W.gb.p, W.grids.p, W.cell_base.p, W.cell_counts.p,
-                        W.cell_starts.p, W.cell_cursor.p, W.rx32.p, W.q0.p, W.q1.p, W.ray32.p,
+  const void* ptrs[] = {W.up.p, W.rx_bad.p, W.path_bound.p, W.field_bound.p, W.rx_flag.p,
+                        W.fstat.p, W.grids.p, W.all.base.p, W.all.counts.p, W.all.starts.p,
+                        W.all.sums.p, W.all.rx32.p, W.direct.base.p,
+                        W.direct.counts.p, W.direct.starts.p, W.direct.sums.p, W.direct.rx32.p,
+                        W.q0.p, W.q1.p, W.ray32.p,
                         W.nodes.p, W.nodes_cold.p, W.cls_keys.p, W.cop_keys.p, W.dd_keys.p,
                         W.dd_rank.p, W.cc_keys.p, W.cls_list.p, W.cc_val.p, W.cls_info.p,
                         W.cls_cap.p, W.corr_list.p, W.pairs.p, W.direct_ok.p, W.surv.p,
@@ -1269,7 +1284,7 @@ static std::string pipeline_key(const SceneImpl& S, const Workspace& W, const sb
                         W.path_pts.p, W.field.p, W.seg.p, W.path_mat.p, W.path_field64.p,
                         W.field64.p, W.path_nray.p, W.path_tri.p, W.path_cop.p, W.path_kind.p,
                         W.path_near.p, W.ctr.p, W.seg_tx.p, W.cand.p, W.ncand.p, W.find_work.p,
-                        W.h_txp.p, W.h_rxreq.p, W.h_rx.p, W.h_gb.p, S.dir_table.p,
+                        W.h_up.p, S.dir_table.p,
                         S.tri_cop.p, S.rank_to_id.p};
   put(ptrs, sizeof ptrs);
   put_v(W.tr_ev.size());
@@ -1431,27 +1446,41 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
   int max_rx = 1;
   for (auto& p : tp) max_rx = std::max(max_rx, p.n_rx);
   const dim3 rg(std::min(1024, (max_rx + 255) / 256), n_req);
-  W.h_txp.ensure(size_t(n_req));
-  std::memcpy(W.h_txp.p, tp.data(), sizeof(TxParams) * n_req);
-  W.h_rxreq.ensure(size_t(std::max(1, rx_total)));
-  W.h_rx.ensure(3 * size_t(std::max(1, rx_total)));
+  // one staging area and one device area of the same layout
+  size_t up_bytes = 0;
+  auto up_at = [&up_bytes](size_t bytes) {
+    const size_t o = up_bytes;
+    up_bytes += (bytes + 255) & ~size_t(255);
+    return o;
+  };
+  const size_t up_txp = up_at(sizeof(TxParams) * n_req), up_gb = up_at(sizeof(GridBuild) * n_req),
+               up_gbd = up_at(sizeof(GridBuild) * n_req),
+               up_req = up_at(sizeof(int) * std::max(1, rx_total)),
+               up_rx = up_at(sizeof(double) * 3 * std::max(1, rx_total));
+  bool host_rx = false;  // receivers from the host are staged too
+  for (int r = 0; r < n_req; ++r) host_rx |= reqs[r].n_rx > 0 && !reqs[r].rx_on_device;
+  W.h_up.ensure(up_bytes);
+  std::memcpy(W.h_up.p + up_txp, tp.data(), sizeof(TxParams) * n_req);
+  int* const h_req = reinterpret_cast<int*>(W.h_up.p + up_req);
+  double* const h_rx = reinterpret_cast<double*>(W.h_up.p + up_rx);
   for (int r = 0; r < n_req; ++r) {
     const sbr_request& q = reqs[r];
-    for (int i = 0; i < q.n_rx; ++i) W.h_rxreq.p[tp[r].rx_first + i] = r;
+    for (int i = 0; i < q.n_rx; ++i) h_req[tp[r].rx_first + i] = r;
     if (q.n_rx && !q.rx_on_device)
-      std::memcpy(W.h_rx.p + 3 * size_t(tp[r].rx_first), q.rx, 3 * sizeof(double) * q.n_rx);
+      std::memcpy(h_rx + 3 * size_t(tp[r].rx_first), q.rx, 3 * sizeof(double) * q.n_rx);
   }
-  W.h_gb.ensure(size_t(n_req));
-  for (int r = 0; r < n_req; ++r) {
-    GridBuild& g = W.h_gb.p[r];
-    for (int a = 0; a < 3; ++a) {
-      g.bmin[a] = INT_MAX;
-      g.bmax[a] = INT_MIN;
+  for (size_t at : {up_gb, up_gbd})
+    for (int r = 0; r < n_req; ++r) {
+      GridBuild& g = reinterpret_cast<GridBuild*>(W.h_up.p + at)[r];
+      for (int a = 0; a < 3; ++a) {
+        g.bmin[a] = INT_MAX;
+        g.bmax[a] = INT_MIN;
+      }
+      g.cmax_o = INT_MIN;
+      g.cmax = 0;
+      g.ncell = 0;
+      g.n = 0;
     }
-    g.cmax_o = INT_MIN;
-    g.cmax = 0;
-    g.ncell = 0;
-  }
   const FieldConsts K = field_consts();
   {
     // Size node pool and queues at the ray-tree bounds so a pass needs no
@@ -1508,17 +1537,19 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     W.surv.ensure(W.cap_surv);
     W.seg_tx.ensure(n_req);
     // receivers and their grid
-    W.txp.ensure(size_t(n_req));
-    W.rx.ensure(std::max(1, 3 * rx_total));
+    W.up.ensure(up_bytes);
     W.direct_ok.ensure(std::max(1, rx_total));
-    W.rx_req.ensure(size_t(std::max(1, rx_total)));
-    W.gb.ensure(n_req);
-    W.grids.ensure(n_req);
-    W.cell_base.ensure(n_req + 1);
-    W.cell_counts.ensure(cell_cap);
-    W.cell_starts.ensure(cell_cap + 1);
-    W.cell_cursor.ensure(cell_cap);
-    W.rx32.ensure(std::max(1, rx_total));
+    const TxParams* const d_txp = reinterpret_cast<TxParams*>(W.up.p + up_txp);
+    const int* const d_req = reinterpret_cast<int*>(W.up.p + up_req);
+    double* const d_rx = reinterpret_cast<double*>(W.up.p + up_rx);
+    W.grids.ensure(2 * size_t(n_req));
+    for (Workspace::Grid* g : {&W.all, &W.direct}) {
+      g->base.ensure(n_req + 1);
+      g->counts.ensure(2 * cell_cap);
+      g->starts.ensure(cell_cap + 1);
+      g->sums.ensure(std::max(cell_cap, size_t(rx_total)) / kScanTile + 1);
+      g->rx32.ensure(std::max(1, rx_total));
+    }
     W.rx_bad.ensure(1);
     // trace chunks: each depth runs in chunks of at most kTraceChunk rays
     const long long kTraceChunk =
@@ -1528,13 +1559,13 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     W.cand.ensure(size_t(chunk) * kCand);
     W.ncand.ensure(size_t(chunk));
     W.ray32.ensure(size_t(chunk));
-    W.find_work.ensure(2);  // [0] k_find's work counter, [1] k_trace's
     size_t n_launch_pairs = 0;  // k_find / k_trace launch pairs of the trace
     {
       for (int d = 0; d <= max_depth; ++d) {
         const long long bound = d == 0 ? launches : (long long)W.cap_queue;
         n_launch_pairs += size_t((bound + chunk - 1) / chunk);
       }
+      W.find_work.ensure(2 * n_launch_pairs + 1);
       if (2 * n_launch_pairs > W.tr_ev.size()) {
         W.tr_ev.resize(2 * n_launch_pairs, nullptr);
         for (auto& e : W.tr_ev)
@@ -1584,58 +1615,72 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     };
     auto record = [&]() {
   mark(W.ev[0]);
-  CK(cudaMemcpyAsync(W.txp.p, W.h_txp.p, sizeof(TxParams) * n_req, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(W.up.p, W.h_up.p, host_rx ? up_bytes : up_rx, cudaMemcpyHostToDevice, st));
   for (int r = 0; r < n_req; ++r) {
     const sbr_request& q = reqs[r];
-    if (!q.n_rx) continue;
-    const size_t o = 3 * size_t(tp[r].rx_first);
-    if (q.rx_on_device)
-      CK(cudaMemcpyAsync(W.rx.p + o, q.rx, 3 * sizeof(double) * q.n_rx, cudaMemcpyDeviceToDevice, st));
-    else
-      CK(cudaMemcpyAsync(W.rx.p + o, W.h_rx.p + o, 3 * sizeof(double) * q.n_rx,
-                         cudaMemcpyHostToDevice, st));
+    if (q.n_rx && q.rx_on_device)
+      CK(cudaMemcpyAsync(d_rx + 3 * size_t(tp[r].rx_first), q.rx, 3 * sizeof(double) * q.n_rx,
+                         cudaMemcpyDeviceToDevice, st));
   }
-  CK(cudaMemcpyAsync(W.rx_req.p, W.h_rxreq.p, sizeof(int) * std::max(1, rx_total),
-                     cudaMemcpyHostToDevice, st));
   mark(W.ev[1]);
-  // ---- receiver grid
-  CK(cudaMemcpyAsync(W.gb.p, W.h_gb.p, sizeof(GridBuild) * n_req, cudaMemcpyHostToDevice, st));
-  CK(cudaMemsetAsync(W.cell_counts.p, 0, sizeof(int) * cell_cap, st));
-  CK(cudaMemsetAsync(W.cell_cursor.p, 0, sizeof(int) * cell_cap, st));
-  CK(cudaMemsetAsync(W.rx_bad.p, 0, sizeof(int), st));
-  ++nl, k_rx_bounds<<<rg, 256, 0, st>>>(W.rx.p, W.txp.p, n_req, W.gb.p, W.rx_bad.p);
-  ++nl, k_grid_shape<<<1, 1, 0, st>>>(W.gb.p, W.grids.p, W.txp.p, n_req, max_cells, W.cell_base.p);
-  ++nl, k_rx_count<<<rg, 256, 0, st>>>(W.rx.p, W.txp.p, n_req, W.grids.p, W.cell_base.p, W.cell_counts.p);
-  ++nl, k_scan_exclusive<<<1, 1024, 0, st>>>(W.cell_counts.p, W.cell_starts.p, int(cell_cap));
-  ++nl, k_rx_scatter<<<rg, 256, 0, st>>>(W.rx.p, W.txp.p, n_req, W.grids.p, W.cell_base.p,
-                                   W.cell_starts.p, W.cell_cursor.p, W.rx32.p);
-  ++nl, k_grid_finish<<<(n_req + 127) / 128, 128, 0, st>>>(W.grids.p, W.cell_starts.p, W.cell_base.p,
-                                                    W.rx32.p, n_req);
-  CK(cudaGetLastError());
-
-    CK(cudaMemsetAsync(W.ctr.p, 0, sizeof(Counters), st));
-    CK(cudaMemsetAsync(W.seg_tx.p, 0, sizeof(unsigned long long) * n_req, st));
-    const int fb = 256;
-    ++nl, k_fill_u64<<<grid_for(W.cap_cls, fb), fb, 0, st>>>(W.cls_keys.p, W.cap_cls, kEmptyKey);
-    ++nl, k_fill_u64<<<grid_for(W.cap_cop, fb), fb, 0, st>>>(W.cop_keys.p, W.cap_cop, kEmptyKey);
-    ++nl, k_fill_u64<<<grid_for(W.cap_dd, fb), fb, 0, st>>>(W.dd_keys.p, W.cap_dd, kEmptyKey);
-    ++nl, k_fill_u64<<<grid_for(W.cap_dd, fb), fb, 0, st>>>(W.dd_rank.p, W.cap_dd, kEmptyKey);
-    ++nl, k_fill_u64<<<grid_for(W.cap_cc, fb), fb, 0, st>>>(W.cc_keys.p, W.cap_cc, kEmptyKey);
-    CK(cudaMemsetAsync(W.cc_val.p, 0, W.cap_cc, st));
+    // ---- every table and counter of the solve, cleared by one launch
+    FillList fl;
+    fl.n = 0;
+    auto fill = [&fl](void* p, size_t bytes, unsigned char v) {
+      fl.r[fl.n++] = FillRange{static_cast<unsigned char*>(p), bytes, v * 0x01010101u};
+    };
+    for (Workspace::Grid* g : {&W.all, &W.direct}) fill(g->counts.p, sizeof(int) * 2 * cell_cap, 0);
+    fill(W.rx_bad.p, sizeof(int), 0);
+    fill(W.ctr.p, sizeof(Counters), 0);
+    fill(W.seg_tx.p, sizeof(unsigned long long) * n_req, 0);
+    fill(W.find_work.p, sizeof(unsigned long long) * (2 * n_launch_pairs + 1), 0);
+    static_assert(kEmptyKey == ~0ull, "tables are cleared byte by byte");
+    fill(W.cls_keys.p, sizeof(unsigned long long) * W.cap_cls, 0xFF);
+    fill(W.cop_keys.p, sizeof(unsigned long long) * W.cap_cop, 0xFF);
+    fill(W.dd_keys.p, sizeof(unsigned long long) * W.cap_dd, 0xFF);
+    fill(W.dd_rank.p, sizeof(unsigned long long) * W.cap_dd, 0xFF);
+    fill(W.cc_keys.p, sizeof(unsigned long long) * W.cap_cc, 0xFF);
+    fill(W.cc_val.p, W.cap_cc, 0);
+    fill(W.rx_flag.p, sizeof(int) * std::max(1, rx_total), 0);
+    fill(W.fstat.p, 2 * sizeof(unsigned long long), 0);
+    fill(W.s_counts.p, sizeof(int) * (rx_total + 1), 0);
+    fill(W.s_cursor.p, sizeof(int) * (rx_total + 1), 0);
+    size_t fill_bytes = 0;
+    for (int k = 0; k < fl.n; ++k) fill_bytes = std::max<size_t>(fill_bytes, fl.r[k].bytes);
+    ++nl, k_fill<<<grid_for((long long)(fill_bytes / 16), 256), 256, 0, st>>>(fl);
+    CK(cudaGetLastError());
     mark(W.ev[2]);
-    // The direct-path test of every receiver (DirectPathCorrection) needs
-    // only the scene and the receivers: it runs on the side stream while the
-    // trace runs, and the capture stage waits for it.
+    // The receiver grids and the direct-path test of every receiver
+    // (DirectPathCorrection) need only the scene and the receivers: they run
+    // on the side stream while the trace runs, and the capture stage waits for
+    // them (level-7 plan 1.38 -> 1.22 ms, level-10 terrain 24.2 -> 21.8 ms with
+    // the direct receivers' own grid and one launch for all clearing).
     CK(cudaEventRecord(W.fork, st));
     CK(cudaStreamWaitEvent(W.side, W.fork, 0));
+    auto build_grid = [&](Workspace::Grid& g, RxGrid* grids, size_t gb_at,
+                          const unsigned char* only) {
+      GridBuild* const gb = reinterpret_cast<GridBuild*>(W.up.p + gb_at);
+      int *const counts = g.counts.p, *const cursor = g.counts.p + cell_cap;
+      ++nl, k_rx_bounds<<<rg, 256, 0, W.side>>>(d_rx, d_txp, n_req, gb, W.rx_bad.p, only);
+      ++nl, k_grid_shape<<<1, 256, 0, W.side>>>(gb, grids, d_txp, n_req, max_cells, g.base.p,
+                                                g.starts.p, g.rx32.p, only ? W.grids.p : nullptr);
+      ++nl, k_rx_count<<<rg, 256, 0, W.side>>>(d_rx, d_txp, n_req, grids, g.base.p, counts,
+                                               only);
+      nl += scan_ints(counts, g.starts.p, int(cell_cap), g.sums.p, W.side);
+      ++nl, k_rx_scatter<<<rg, 256, 0, W.side>>>(d_rx, d_txp, n_req, grids, g.base.p,
+                                                 g.starts.p, cursor, g.rx32.p, only);
+    };
+    build_grid(W.all, W.grids.p, up_gb, nullptr);
     if (rx_total)
-      ++nl, k_direct<<<grid_for(rx_total, 32), 32, 0, W.side>>>(S.dev, W.txp.p, W.rx.p, W.rx_req.p,
-                                                             rx_total, W.direct_ok.p, W.ctr.p);
+      ++nl, k_direct<<<grid_for(rx_total, 32), 32, 0, W.side>>>(S.dev, d_txp, d_rx, d_req, rx_total,
+                                                                W.direct_ok.p, W.ctr.p);
+    if (!stage_counts) build_grid(W.direct, W.grids.p + n_req, up_gbd, W.direct_ok.p);
+    CK(cudaGetLastError());
     CK(cudaEventRecord(W.join, W.side));
     // ---- trace
     TraceArgs ta;
     ta.sc = S.dev;
-    ta.txp = W.txp.p;
+    ta.txp = d_txp;
     ta.n_tx = n_req;
     ta.dirs = S.dir_table.p;
     ta.nodes = W.nodes.p;
@@ -1657,13 +1702,12 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     // return at once.
     FindArgs fnd;
     fnd.sc = S.dev;
-    fnd.txp = W.txp.p;
+    fnd.txp = d_txp;
     fnd.n_tx = n_req;
     fnd.dirs = S.dir_table.p;
     fnd.ctr = W.ctr.p;
     fnd.in_cap = W.cap_queue;
     fnd.n_root = launches;
-    fnd.work = W.find_work.p;
     fnd.cand = W.cand.p;
     fnd.ncand = W.ncand.p;
     fnd.ray32 = W.ray32.p;
@@ -1673,7 +1717,6 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ta.cand = W.cand.p;
     ta.ncand = W.ncand.p;
     ta.ray32 = W.ray32.p;
-    ta.work = W.find_work.p + 1;
     n_tr = 0;
     for (int d = 0; d <= max_depth; ++d) {
       ta.depth = fnd.depth = d;
@@ -1683,7 +1726,8 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       for (long long lo = 0; lo < bound; lo += chunk) {
         ta.lo = fnd.lo = lo;
         ta.hi = fnd.hi = std::min(bound, lo + chunk);
-        CK(cudaMemsetAsync(W.find_work.p, 0, 2 * sizeof(unsigned long long), st));
+        fnd.work = W.find_work.p + 2 * n_tr;
+        ta.work = fnd.work + 1;
         ++nl, k_find<<<find_grid(tu), 128, 0, st>>>(fnd);
         mark(W.tr_ev[2 * n_tr]);
         ++nl, k_trace<<<std::min<long long>(trace_grid(tu), (ta.hi - lo + 127) / 128), 128, 0, st>>>(ta);
@@ -1701,10 +1745,11 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ca.sc = S.dev;
     ca.nodes = W.nodes.p;
     ca.nodes_cold = W.nodes_cold.p;
-    ca.txp = W.txp.p;
+    ca.txp = d_txp;
     ca.grids = W.grids.p;
-    ca.gb = W.gb.p;
-    ca.rx = W.rx.p;
+    ca.n_tx = n_req;
+    ca.gb = reinterpret_cast<GridBuild*>(W.up.p + up_gb);
+    ca.rx = d_rx;
     ca.cls_info = W.cls_info.p;
     ca.cls_cap = W.cls_cap.p;
     ca.direct_ok = W.direct_ok.p;
@@ -1717,8 +1762,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ca.pair_cap = W.cap_pairs;
     ca.corr_cache = HashTable{W.cc_keys.p, W.cap_cc - 1};
     ca.corr_val = W.cc_val.p;
-    ca.work = W.find_work.p;  // the trace is done with it
-    CK(cudaMemsetAsync(W.find_work.p, 0, sizeof(unsigned long long), st));
+    ca.work = W.find_work.p + 2 * n_launch_pairs;
     CK(cudaStreamWaitEvent(st, W.join, 0));
     mark(W.cap_ev[0]);
     if (stage_counts) {
@@ -1746,9 +1790,9 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     const unsigned long long ns_cap = W.cap_surv;
     FieldArgs fa;
     fa.sc = S.dev;
-    fa.txp = W.txp.p;
-    fa.rx = W.rx.p;
-    fa.rx_req = W.rx_req.p;
+    fa.txp = d_txp;
+    fa.rx = d_rx;
+    fa.rx_req = d_req;
     fa.cls_info = W.cls_info.p;
     fa.rank_to_id = S.rank_to_id.p;
     fa.surv = W.surv.p;
@@ -1767,28 +1811,24 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     fa.path_mat = W.path_mat.p;
     bool any_fp32 = false;  // a request in the FP32 field mode (error bounds, escalation)
     for (int r = 0; r < n_req; ++r) any_fp32 |= tp[r].precision == 1;
-    CK(cudaMemsetAsync(W.rx_flag.p, 0, sizeof(int) * std::max(1, rx_total), st));
-    CK(cudaMemsetAsync(W.fstat.p, 0, 2 * sizeof(unsigned long long), st));
     fa.path_bound = W.path_bound.p;
     fa.rx_flag = W.rx_flag.p;
     fa.fstat = W.fstat.p;
     ++nl, k_path<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
     ++nl, k_seg<<<grid_for(ns_cap * (kMaxDepth + 1), 64), 64, 0, st>>>(fa);
     ++nl, k_combine<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
-    CK(cudaMemsetAsync(W.s_counts.p, 0, sizeof(int) * (rx_total + 1), st));
-    CK(cudaMemsetAsync(W.s_cursor.p, 0, sizeof(int) * (rx_total + 1), st));
     ++nl, k_surv_hist<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv, W.s_counts.p);
-    ++nl, k_scan_exclusive<<<1, 1024, 0, st>>>(W.s_counts.p, W.s_starts.p, rx_total);
+    nl += scan_ints(W.s_counts.p, W.s_starts.p, rx_total, W.all.sums.p, st);
     ++nl, k_surv_scatter<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv,
                                                           W.s_starts.p, W.s_cursor.p, W.s_order.p);
     if (rx_total)
       ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(
-          W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, -1, W.rx_req.p, W.txp.p,
+          W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, -1, d_req, d_txp,
           W.field.p, W.path_bound.p, W.field_bound.p, W.rx_flag.p, W.fstat.p);
     if (any_fp32 && rx_total) {  // receivers the FP32 bound could not certify, in FP64
       ++nl, k_escalate<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
       ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(
-          W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, 0, W.rx_req.p, W.txp.p,
+          W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, 0, d_req, d_txp,
           W.field.p, nullptr, W.field_bound.p, nullptr, nullptr, W.rx_flag.p);
     }
     CK(cudaGetLastError());
@@ -1803,7 +1843,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       if (rx_total)
         ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(W.surv.p, W.s_starts.p, W.s_order.p,
                                                           rx_total, W.path_field64.p, 0,
-                                                          W.rx_req.p, W.txp.p, W.field64.p);
+                                                          d_req, d_txp, W.field64.p);
       CK(cudaGetLastError());
     }
     };  // record
