@@ -50,15 +50,17 @@ __device__ __forceinline__ HashProbe ht_probe(HashTable t, unsigned long long ke
   return p;
 }
 
-__device__ __forceinline__ uint32_t ht_insert(HashTable t, const HashProbe& p, unsigned* ov,
+// The insert past the home slot (out of line: most probes end there).
+__device__ __noinline__ uint32_t ht_insert_on(unsigned long long* keys, uint32_t mask,
+                                              unsigned long long key, uint32_t h,
+                                              unsigned long long first, unsigned* ov,
                                               unsigned bit, unsigned long long* used,
-                                              unsigned long long* lost, bool* fresh = nullptr) {
-  uint32_t h = p.slot;
-  const unsigned long long key = p.key;
+                                              unsigned long long* lost, bool* fresh) {
+  const HashTable t{keys, mask};
   const uint32_t lim = min(kMaxProbe, t.mask + 1);
   for (uint32_t i = 0; i < lim; ++i) {
     const unsigned long long k =
-        i == 0 ? p.first : *reinterpret_cast<volatile unsigned long long*>(&t.keys[h]);
+        i == 0 ? first : *reinterpret_cast<volatile unsigned long long*>(&t.keys[h]);
     if (k == key) return h;
     if (k == kEmptyKey) {
       unsigned long long old = atomicCAS(&t.keys[h], kEmptyKey, key);
@@ -74,6 +76,12 @@ __device__ __forceinline__ uint32_t ht_insert(HashTable t, const HashProbe& p, u
   atomicOr(ov, bit);
   atomicAdd(lost, 1ull);
   return 0xFFFFFFFFu;
+}
+__device__ __forceinline__ uint32_t ht_insert(HashTable t, const HashProbe& p, unsigned* ov,
+                                              unsigned bit, unsigned long long* used,
+                                              unsigned long long* lost, bool* fresh = nullptr) {
+  if (p.first == p.key) return p.slot;
+  return ht_insert_on(t.keys, t.mask, p.key, p.slot, p.first, ov, bit, used, lost, fresh);
 }
 __device__ __forceinline__ uint32_t ht_insert(HashTable t, unsigned long long key, unsigned* ov,
                                               unsigned bit, unsigned long long* used,

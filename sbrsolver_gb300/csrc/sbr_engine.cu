@@ -672,7 +672,7 @@ static int find_fit() {
   return per_sm;
 }
 static int trace_fit() {
-  static const int per_sm = blocks_per_sm(k_trace, 128);
+  static const int per_sm = blocks_per_sm(k_trace<false>, 128);
   return per_sm;
 }
 static int capture_fit() {
@@ -1730,7 +1730,9 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
         ta.work = fnd.work + 1;
         ++nl, k_find<<<find_grid(tu), 128, 0, st>>>(fnd);
         mark(W.tr_ev[2 * n_tr]);
-        ++nl, k_trace<<<std::min<long long>(trace_grid(tu), (ta.hi - lo + 127) / 128), 128, 0, st>>>(ta);
+        const int tg = int(std::min<long long>(trace_grid(tu), (ta.hi - lo + 127) / 128));
+        if (d == 0) ++nl, k_trace<true><<<tg, 128, 0, st>>>(ta);
+        else ++nl, k_trace<false><<<tg, 128, 0, st>>>(ta);
         mark(W.tr_ev[2 * n_tr + 1]);
         ++n_tr;
       }

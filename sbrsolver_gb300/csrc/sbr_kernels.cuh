@@ -58,6 +58,7 @@ struct Hit {
 // Products, quotients and roots of the FP64 tests: on the FP64 pipe, or in
 // integer arithmetic (sbr_soft64.cuh; the same bits for operands in its range).
 struct Pipe64 {
+  static constexpr bool kSoft = false;
   static __device__ __forceinline__ double mul(double a, double b) { return x64::mul(a, b); }
   // 1.0 / a (Triangle.cpp): the correctly rounded reciprocal is the same
   // double as the correctly rounded quotient 1.0 / a
@@ -65,19 +66,42 @@ struct Pipe64 {
   static __device__ __forceinline__ double sqrt(double a) { return x64::sqrt_(a); }
 };
 struct Soft64 {
+  static constexpr bool kSoft = true;
   static __device__ __forceinline__ double mul(double a, double b) { return soft64::mul(a, b); }
   static __device__ __forceinline__ double rcp(double a) { return soft64::rcp(a); }
   static __device__ __forceinline__ double sqrt(double a) { return soft64::sqrt(a); }
 };
+// The dot and cross products of the integer form are functions: they are used
+// nine times, and inline their products alone are 20 KB of code, in a kernel
+// (k_trace) whose warps wait for instructions a third of the time.
+struct D3 {
+  double x, y, z;
+};
+__device__ __noinline__ double dot_soft(double a0, double a1, double a2, double b0, double b1,
+                                        double b2) {
+  return x64::add(x64::add(soft64::mul(a0, b0), soft64::mul(a1, b1)), soft64::mul(a2, b2));
+}
+__device__ __noinline__ D3 cross_soft(double a0, double a1, double a2, double b0, double b1,
+                                      double b2) {
+  return D3{x64::sub(soft64::mul(a1, b2), soft64::mul(a2, b1)),
+            x64::sub(soft64::mul(a2, b0), soft64::mul(a0, b2)),
+            x64::sub(soft64::mul(a0, b1), soft64::mul(a1, b0))};
+}
 template <class A>
 __device__ __forceinline__ double dot64(const double* a, const double* b) {
-  return x64::add(x64::add(A::mul(a[0], b[0]), A::mul(a[1], b[1])), A::mul(a[2], b[2]));
+  if (A::kSoft) return dot_soft(a[0], a[1], a[2], b[0], b[1], b[2]);
+  return x64::dot(a, b);
 }
 template <class A>
 __device__ __forceinline__ void cross64(const double* a, const double* b, double* r) {
-  r[0] = x64::sub(A::mul(a[1], b[2]), A::mul(a[2], b[1]));
-  r[1] = x64::sub(A::mul(a[2], b[0]), A::mul(a[0], b[2]));
-  r[2] = x64::sub(A::mul(a[0], b[1]), A::mul(a[1], b[0]));
+  if (A::kSoft) {
+    const D3 v = cross_soft(a[0], a[1], a[2], b[0], b[1], b[2]);
+    r[0] = v.x;
+    r[1] = v.y;
+    r[2] = v.z;
+  } else {
+    x64::cross(a, b, r);
+  }
 }
 
 // Triangle::RayIntersects (Triangle.cpp:80-124), FP64, reference operation

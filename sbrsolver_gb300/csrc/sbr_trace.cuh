@@ -75,7 +75,9 @@ __device__ void write_class_cap(const DevScene& sc, const double* img, int tpos,
 // Correction cones of the interned classes (one thread per class-table
 // slot, after the trace): three planes through the image source and the
 // last triangle's edges, formed in FP64 and rounded to FP32, so a plane's
-// error is its FP32 rounding alone.
+// error is its FP32 rounding alone.  Bound by the FP64 pipe: some 60
+// instructions per class (its lengths' FP64 roots and quotients made them 330;
+// the level-10 terrain's 1.36M classes 0.71 ms, now 0.55).
 __global__ void k_class_cones(const uint32_t* list, const Counters* ctr, uint32_t cap,
                               const ClassInfo* info, DevScene sc, ClassCap* caps) {
   if (ctr->overflow & kOvTrace) return;  // this solve will be repeated
@@ -86,39 +88,41 @@ __global__ void k_class_cones(const uint32_t* list, const Counters* ctr, uint32_
     const ClassInfo& ci = info[s];
     const CorrTri& T = sc.corr[sc.rank_to_id[ci.tri]];
     ClassCap& cc = caps[s];
-    double v[3][3];
-    for (int a = 0; a < 3; ++a) {
-      v[0][a] = T.v1[a];
-      v[1][a] = T.v1[a] + T.e1[a];
-      v[2][a] = T.v1[a] + T.e2[a];
-    }
     const double* im = ci.img;
-    const double g[3] = {(v[0][0] + v[1][0] + v[2][0]) / 3.0, (v[0][1] + v[1][1] + v[2][1]) / 3.0,
-                         (v[0][2] + v[1][2] + v[2][2]) / 3.0};
-    auto ab2 = [](const double* x) { return x[0] * x[0] + x[1] * x[1] + x[2] * x[2]; };
-    auto norm3 = [](const double* x) { return sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]); };
-    const float tmag =
-        float((norm3(im) + norm3(T.v1) + norm3(T.e1) + norm3(T.e2)) * (1.0 + 1e-6)) + 1.0f;
+    // the vertices and the centroid from the image source
+    double v[3][3], g[3];
+    for (int a = 0; a < 3; ++a) {
+      v[0][a] = T.v1[a] - im[a];
+      v[1][a] = v[0][a] + T.e1[a];
+      v[2][a] = v[0][a] + T.e2[a];
+      g[a] = (v[0][a] + v[1][a] + v[2][a]) * (1.0 / 3.0);
+    }
+    // lengths enter margins and thresholds only: FP32, rounded up
+    auto norm32 = [](const double* x) {
+      const float a = soft64::to_f32(x[0]), b = soft64::to_f32(x[1]), c = soft64::to_f32(x[2]);
+      return sqrtf(a * a + b * b + c * c) * (1.0f + 1e-6f);
+    };
+    const float tmag = norm32(im) + norm32(T.v1) + norm32(T.e1) + norm32(T.e2) + 1.0f;
+    const float len[3] = {norm32(v[0]), norm32(v[1]), norm32(v[2])};
     for (int k = 0; k < 3; ++k) {
-      const double* p = v[k];
-      const double* q = v[k == 2 ? 0 : k + 1];
-      const double a[3] = {p[0] - im[0], p[1] - im[1], p[2] - im[2]};
-      const double b[3] = {q[0] - im[0], q[1] - im[1], q[2] - im[2]};
+      const double* a = v[k];
+      const double* b = v[k == 2 ? 0 : k + 1];
       const double n[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2],
                            a[0] * b[1] - a[1] * b[0]};
-      const double nn = norm3(n);
+      const float nn = norm32(n);
       // orient towards the triangle's centroid, which lies inside the cone
-      const double gc = n[0] * (g[0] - im[0]) + n[1] * (g[1] - im[1]) + n[2] * (g[2] - im[2]);
-      const double sg = gc > 0.0 ? 1.0 : -1.0;
-      for (int c = 0; c < 3; ++c) cc.n[k][c] = float(sg * n[c]);
-      cc.n[k][3] = float(sg * (n[0] * im[0] + n[1] * im[1] + n[2] * im[2]));
-      cc.nn[k] = float(nn * (1.0 + 1e-6));
-      cc.w[k] = cc.nn[k] * tmag;
+      const double gc = n[0] * g[0] + n[1] * g[1] + n[2] * g[2];
+      const float sg = soft64::negative(gc) ? -1.0f : 1.0f;
+      const double off = n[0] * im[0] + n[1] * im[1] + n[2] * im[2];
+      for (int c = 0; c < 3; ++c) cc.n[k][c] = sg * soft64::to_f32(n[c]);
+      cc.n[k][3] = sg * soft64::to_f32(off);
+      cc.nn[k] = nn;
+      cc.w[k] = nn * tmag;
       // FP64 forms n to within 2^-50 |a||b| and gc to within that times the
       // distance: the plane is used where both are far below what they are
       // compared with (n's FP32 rounding, gc's sign)
-      const double ab = sqrt(ab2(a) * ab2(b));
-      cc.gc[k] = nn > 1e-6 * ab && fabs(gc) > 4e-9 * nn * double(tmag) ? float(fabs(gc)) : 0.0f;
+      const float ga = fabsf(soft64::to_f32(gc));
+      cc.gc[k] = nn > 1e-6f * (len[k] * len[k == 2 ? 0 : k + 1]) && ga > 4e-9f * cc.w[k] ? ga : 0.0f;
     }
   }
 }
@@ -510,9 +514,19 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
 }
 
 // Resident blocks of k_trace per SM (register budget 65536 / (128 x this)).
+// Level-9 canyon, k_trace in all: 4 blocks 5.28 ms, 5 5.38 (spills), 6 5.97, 3
+// 5.80; its warps wait for memory and for instructions alike.
 #ifndef SBR_TRACE_BLOCKS
-#define SBR_TRACE_BLOCKS 5
+#define SBR_TRACE_BLOCKS 4
 #endif
+
+// Reflect(d, n) with the FP64 pipe's products (see mt64_call).
+__device__ __noinline__ D3 reflect_call(const double* n, double dx, double dy, double dz) {
+  const double d[3] = {dx, dy, dz};
+  const double dn2 = 2.0 * x64::dot(n, d);
+  return D3{x64::sub(dx, x64::mul(n[0], dn2)), x64::sub(dy, x64::mul(n[1], dn2)),
+            x64::sub(dz, x64::mul(n[2], dn2))};
+}
 
 // Queue slots of the active lanes' children, one atomic: the transmitted rays
 // first, then the reflected ones, so that a warp of the next depth finds rays
@@ -585,8 +599,10 @@ __device__ __forceinline__ void finish_ray(const TraceArgs& A, unsigned long lon
         const double dn2 = 2.0 * dot64<Soft64>(n, r.d);
         for (int a = 0; a < 3; ++a) c.d[a] = x64::sub(r.d[a], soft64::mul(n[a], dn2));
       } else {
-        const double dn2 = 2.0 * x64::dot(n, r.d);
-        for (int a = 0; a < 3; ++a) c.d[a] = x64::sub(r.d[a], x64::mul(n[a], dn2));
+        const D3 v = reflect_call(n, r.d[0], r.d[1], r.d[2]);
+        c.d[0] = v.x;
+        c.d[1] = v.y;
+        c.d[2] = v.z;
       }
       c.heap = r.heap * 2 + 1;
       c.rc = r.rc + 1;
@@ -633,9 +649,12 @@ __device__ __forceinline__ int next_contender(const uint2* cand, int nc, unsigne
 // same round and takes a new ray; a ray needing a
 // second test no longer holds the whole warp through a second pass of the
 // test with a few lanes.  The warp is brought together after each part of a
-// round.  A lane keeps only the ray's origin and direction and the best hit
-// between rounds; the rest of its record is read again when it is resolved.
-__global__ void __launch_bounds__(128, SBR_TRACE_BLOCKS) k_trace(const __grid_constant__ TraceArgs A) {
+// round.  kRoot: the launch rays (depth 0).  A lane keeps only the ray's
+// origin and direction and the best hit between rounds; the rest of its
+// record is read again when it is resolved.
+template <bool kRoot>
+__global__ void __launch_bounds__(128, SBR_TRACE_BLOCKS)
+    k_trace(const __grid_constant__ TraceArgs A) {
   if (A.ctr->overflow & kOvTrace) return;  // this solve will be repeated
   const long long n_all = rays_at_depth(A.ctr, A.depth, A.n_root, A.out_cap);
   const long long n = min(n_all, A.hi) - A.lo;
@@ -670,16 +689,16 @@ __global__ void __launch_bounds__(128, SBR_TRACE_BLOCKS) k_trace(const __grid_co
         nc = A.ncand[k];
         if (!(nc & kCandCount)) {
           RayRec r;
-          load_ray(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + k, r);
+          load_ray(A.txp, A.n_tx, A.dirs, A.in, kRoot ? 0 : 1, A.lo + k, r);
           const float4* f = reinterpret_cast<const float4*>(A.ray32 + k);
           const float4 fo = f[0], fd = f[1];
           Hit none;
           seg.add(A.seg_per_tx, r.tx);
-          emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, base + k, r, A.depth == 0,
+          emit_node(A.nodes, A.nodes_cold, A.node_cap, A.ctr, base + k, r, kRoot,
                     make_float3(fo.x, fo.y, fo.z), make_float3(fd.x, fd.y, fd.z),
                     !(nc & kCandUnsafe), false, none);
         } else {
-          load_ray_line(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + k, o, d);
+          load_ray_line(A.txp, A.n_tx, A.dirs, A.in, kRoot ? 0 : 1, A.lo + k, o, d);
           c = k;
           tested = 0;
           next = nc != kFindFallback
@@ -740,7 +759,7 @@ __global__ void __launch_bounds__(128, SBR_TRACE_BLOCKS) k_trace(const __grid_co
     __syncwarp();
     if (done) {
       RayRec r;
-      load_ray(A.txp, A.n_tx, A.dirs, A.in, A.depth, A.lo + c, r);
+      load_ray(A.txp, A.n_tx, A.dirs, A.in, kRoot ? 0 : 1, A.lo + c, r);
       const float4* f = reinterpret_cast<const float4*>(A.ray32 + c);
       const float4 fo = f[0], fd = f[1];
       const float3 o32 = make_float3(fo.x, fo.y, fo.z), d32 = make_float3(fd.x, fd.y, fd.z);
