@@ -233,6 +233,7 @@ struct Counters {
   unsigned long long anc;        // ancestor re-tests for suppression
   unsigned long long used_cc;    // (class, receiver) corrections cached
   unsigned long long cls_listed; // classes listed for their correction cones
+  unsigned long long seg_tasks, int_tasks;  // field-stage tasks (k_path lists, k_seg runs them)
   unsigned int overflow;         // bit mask of capacity overflows
   unsigned int pad;
 };

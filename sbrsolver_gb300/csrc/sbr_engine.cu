@@ -185,6 +185,7 @@ struct Workspace {
   DBuf<int> s_counts, s_starts, s_cursor, s_order;
   DBuf<double> path_field, path_pts, field;
   DBuf<SegTerms> seg;                  // field terms per path segment
+  DBuf<uint32_t> seg_list, int_list;   // k_seg's tasks
   DBuf<int> path_mat;                  // material of each ray's start per path
   DBuf<double> path_field64, field64;  // FP64 shadow of an FP32 field (field_check)
   DBuf<int> path_nray, path_tri, path_cop, path_kind, path_near;
@@ -1281,7 +1282,7 @@ static std::string pipeline_key(const SceneImpl& S, const Workspace& W, const sb
                         W.dd_rank.p, W.cc_keys.p, W.cls_list.p, W.cc_val.p, W.cls_info.p,
                         W.cls_cap.p, W.corr_list.p, W.pairs.p, W.direct_ok.p, W.surv.p,
                         W.s_counts.p, W.s_starts.p, W.s_cursor.p, W.s_order.p, W.path_field.p,
-                        W.path_pts.p, W.field.p, W.seg.p, W.path_mat.p, W.path_field64.p,
+                        W.path_pts.p, W.field.p, W.seg.p, W.seg_list.p, W.int_list.p, W.path_mat.p, W.path_field64.p,
                         W.field64.p, W.path_nray.p, W.path_tri.p, W.path_cop.p, W.path_kind.p,
                         W.path_near.p, W.ctr.p, W.seg_tx.p, W.cand.p, W.ncand.p, W.find_work.p,
                         W.h_up.p, S.dir_table.p,
@@ -1583,6 +1584,8 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       W.path_near.ensure(nsa);
       W.path_pts.ensure(nsa * (kMaxDepth + 2) * 3);
       W.seg.ensure(nsa * (kMaxDepth + 1));
+      W.seg_list.ensure(nsa * (kMaxDepth + 1));
+      W.int_list.ensure(nsa * kMaxDepth);
       W.path_mat.ensure(nsa * (kMaxDepth + 1));
       W.field.ensure(std::max(1, 6 * rx_total));
       W.s_counts.ensure(rx_total + 1);
@@ -1811,6 +1814,8 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     fa.path_pts = W.path_pts.p;
     fa.seg = W.seg.p;
     fa.path_mat = W.path_mat.p;
+    fa.seg_list = W.seg_list.p;
+    fa.int_list = W.int_list.p;
     bool any_fp32 = false;  // a request in the FP32 field mode (error bounds, escalation)
     for (int r = 0; r < n_req; ++r) any_fp32 |= tp[r].precision == 1;
     fa.path_bound = W.path_bound.p;
@@ -1819,6 +1824,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ++nl, k_path<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
     ++nl, k_seg<<<grid_for(ns_cap * (kMaxDepth + 1), 64), 64, 0, st>>>(fa);
     ++nl, k_combine<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
+    if (any_fp32) ++nl, k_escalate<<<grid_for(ns_cap * 32, 64), 64, 0, st>>>(fa, false);
     ++nl, k_surv_hist<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv, W.s_counts.p);
     nl += scan_ints(W.s_counts.p, W.s_starts.p, rx_total, W.all.sums.p, st);
     ++nl, k_surv_scatter<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv,
@@ -1828,7 +1834,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
           W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, -1, d_req, d_txp,
           W.field.p, W.path_bound.p, W.field_bound.p, W.rx_flag.p, W.fstat.p);
     if (any_fp32 && rx_total) {  // receivers the FP32 bound could not certify, in FP64
-      ++nl, k_escalate<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
+      ++nl, k_escalate<<<grid_for(ns_cap * 32, 64), 64, 0, st>>>(fa, true);
       ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(
           W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, 0, d_req, d_txp,
           W.field.p, nullptr, W.field_bound.p, nullptr, nullptr, W.rx_flag.p);

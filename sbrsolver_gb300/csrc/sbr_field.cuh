@@ -234,6 +234,11 @@ __device__ void fresnel_pair(bool reflect, R theta_i, Cx<R> eps_t, Cx<R> ph, boo
 // this fraction of their terms take the FP64 coefficients (fresnel_pair).
 constexpr float kFresnelCond32 = 0.125f;
 
+// The terms come in two independent parts, which k_seg gives to different
+// threads: the direction (length, angles, launch pattern) and the interaction
+// at the segment's start (angle of incidence and coefficients).
+enum SegPart { kSegDirection = 1, kSegInteraction = 2, kSegBoth = 3 };
+
 struct SegTerms {
   double r;               // segment length (FP64)
   double st, ct, sp, cp;  // sin / cos of the direction's theta and phi
@@ -265,106 +270,110 @@ template <class R>
 __device__ void seg_terms(int i, const double (*pts)[3], const double* const* frames,
                           const int* kind, const int* mat, const Material* mats,
                           const double* txcs, double freq, double pt, int antenna, bool fresnel,
-                          const FieldConsts& K, SegTerms& out, const PatternTab* pat = nullptr) {
-  const double lam64 = 2.99792458e8 / freq;
-  const M3<R> cur = start_frame<R>(i, frames, txcs);
+                          const FieldConsts& K, SegTerms& out, const PatternTab* pat = nullptr,
+                          int part = kSegBoth) {
   double vg64[3] = {pts[i + 1][0] - pts[i][0], pts[i + 1][1] - pts[i][1], pts[i + 1][2] - pts[i][2]};
-  R vg[3] = {R(vg64[0]), R(vg64[1]), R(vg64[2])};
-  R vl[3];
-  mv(cur, vg, vl);
-  // CartesianToSpherical (VecMatDef.h:132-155); r is kept in FP64, the length
-  // of the vector rotated by the FP64 frame, as in the reference (the FP32
-  // mode forms it the same way below).
-  if constexpr (sizeof(R) == sizeof(double)) {
-    double vl64[3];
-    for (int j = 0; j < 3; ++j)
-      vl64[j] = (cur.m[3 * j] * vg64[0] + cur.m[3 * j + 1] * vg64[1]) + cur.m[3 * j + 2] * vg64[2];
-    out.r = sqrt((vl64[0] * vl64[0] + vl64[1] * vl64[1]) + vl64[2] * vl64[2]);
-  }
-  R th, ph;
-  if (vl[0] == R(0) && vl[1] == R(0) && vl[2] == R(0)) th = R(K.pi_hi * 0.5);
-  else th = atan2(sqrt(vl[0] * vl[0] + vl[1] * vl[1]), vl[2]);
-  ph = atan2(vl[1], vl[0]);
-  if (ph < R(0)) ph = R((double(ph) + 2.0 * K.pi_hi) + 2.0 * K.pi_lo);
-  if constexpr (sizeof(R) == sizeof(double)) {
-    out.st = sin(th);
-    out.ct = cos(th);
-    out.sp = sin(ph);
-    out.cp = cos(ph);
-  } else {
-    // FP32 mode: the segment rotated into its frame in FP64 (a few FP64
-    // operations per segment), then the basis from its components, which
-    // keeps each of sin/cos theta, phi to a few FP32 ulps even for
-    // directions near the frame's axis, where an FP32 rotation or sin(theta)
-    // of theta near 0 or pi loses most of their relative precision
-    const double* fr = i == 0 ? txcs : frames[i - 1];
-    double w64[3];
-    float w[3];
-    for (int j = 0; j < 3; ++j) {
-      const double r0 = fr ? fr[3 * j] : (j == 0 ? 1.0 : 0.0);
-      const double r1 = fr ? fr[3 * j + 1] : (j == 1 ? 1.0 : 0.0);
-      const double r2 = fr ? fr[3 * j + 2] : (j == 2 ? 1.0 : 0.0);
-      w64[j] = (r0 * vg64[0] + r1 * vg64[1]) + r2 * vg64[2];
-      w[j] = float(w64[j]);
-    }
-    // the segment length as the FP64 mode (and the reference) takes it: of
-    // the vector rotated by the FP64 frame, which a triangle's single-
-    // precision file normal leaves orthonormal only to ~1e-7, so the
-    // global length would move the phase k*L of a long path by ~1e-4 rad
-    out.r = sqrt((w64[0] * w64[0] + w64[1] * w64[1]) + w64[2] * w64[2]);
-    const float rho = sqrtf(w[0] * w[0] + w[1] * w[1]);
-    const float len = sqrtf(rho * rho + w[2] * w[2]);
-    if (len > 0.0f) {
-      out.st = double(rho / len);
-      out.ct = double(w[2] / len);
-    } else {  // the zero vector: theta = pi/2, phi = 0 (VecMatDef.h:132-155)
-      out.st = 1.0;
-      out.ct = 0.0;
-    }
-    out.sp = rho > 0.0f ? double(w[1] / rho) : 0.0;
-    out.cp = rho > 0.0f ? double(w[0] / rho) : 1.0;
-    th = atan2(rho, w[2]);  // the pattern's angles
-    if (len == 0.0f) th = R(K.pi_hi * 0.5);
-    ph = atan2(w[1], w[0]);
-    if (ph < R(0)) ph = R((double(ph) + 2.0 * K.pi_hi) + 2.0 * K.pi_lo);
-  }
-  for (int j = 0; j < 6; ++j) out.inc[j] = 0.0;
-  out.fp64_fresnel = 0;
-  out.pad = 0;
-  if (i == 0) {
-    Cx<R> inc[3] = {cx(R(0)), cx(R(0)), cx(R(0))};
+  if (part != kSegInteraction) {
+    const M3<R> cur = start_frame<R>(i, frames, txcs);
+    R vg[3] = {R(vg64[0]), R(vg64[1]), R(vg64[2])};
+    R vl[3];
+    mv(cur, vg, vl);
+    // CartesianToSpherical (VecMatDef.h:132-155); r is kept in FP64, the length
+    // of the vector rotated by the FP64 frame, as in the reference (the FP32
+    // mode forms it the same way below).
     if constexpr (sizeof(R) == sizeof(double)) {
-      if (antenna == 0) inc[0] = cx(R(0), R(sqrt(60.0 * pt)));
-      if (antenna == 1) inc[1] = cx(R(0), R(sqrt(60.0 * pt * 1.5)) * sin(th));
-      else if (antenna == 2)
-        inc[1] = cx(R(0), R(sqrt(60.0 * pt)) * (cos(R(K.pi_hi) * cos(th) / R(2)) / sin(th)));
+      double vl64[3];
+      for (int j = 0; j < 3; ++j)
+        vl64[j] = (cur.m[3 * j] * vg64[0] + cur.m[3 * j + 1] * vg64[1]) + cur.m[3 * j + 2] * vg64[2];
+      out.r = sqrt((vl64[0] * vl64[0] + vl64[1] * vl64[1]) + vl64[2] * vl64[2]);
+    }
+    R th, ph;
+    if (vl[0] == R(0) && vl[1] == R(0) && vl[2] == R(0)) th = R(K.pi_hi * 0.5);
+    else th = atan2(sqrt(vl[0] * vl[0] + vl[1] * vl[1]), vl[2]);
+    ph = atan2(vl[1], vl[0]);
+    if (ph < R(0)) ph = R((double(ph) + 2.0 * K.pi_hi) + 2.0 * K.pi_lo);
+    if constexpr (sizeof(R) == sizeof(double)) {
+      out.st = sin(th);
+      out.ct = cos(th);
+      out.sp = sin(ph);
+      out.cp = cos(ph);
     } else {
-      // FP32: sin and cos of theta from the segment's components (accurate
-      // to ulps, unlike sin(theta) near the dipole axis, where theta's own
-      // FP32 rounding is most of sin(theta)).  The half-wave pattern's
-      // cos(pi/2 cos th) is sin(pi s) with s = sin^2(th/2) = st^2 / (2 (1 + ct))
-      // or cos^2(th/2) = st^2 / (2 (1 - ct)), whichever is at most 1/2: no
-      // cancellation near the axis, where cos(pi/2 cos th) -> 0.
-      const float st = float(out.st), ct = float(out.ct);
-      if (antenna == 0) inc[0] = cx(R(0), R(sqrt(60.0 * pt)));
-      if (antenna == 1) inc[1] = cx(R(0), R(sqrt(60.0 * pt * 1.5)) * st);
-      else if (antenna == 2) {
-        const float h2 = (st * st) / (2.0f * (ct >= 0.0f ? 1.0f + ct : 1.0f - ct));
-        inc[1] = cx(R(0), R(sqrt(60.0 * pt)) * (sinf(float(K.pi_hi) * h2) / st));
+      // FP32 mode: the segment rotated into its frame in FP64 (a few FP64
+      // operations per segment), then the basis from its components, which
+      // keeps each of sin/cos theta, phi to a few FP32 ulps even for
+      // directions near the frame's axis, where an FP32 rotation or sin(theta)
+      // of theta near 0 or pi loses most of their relative precision
+      const double* fr = i == 0 ? txcs : frames[i - 1];
+      double w64[3];
+      float w[3];
+      for (int j = 0; j < 3; ++j) {
+        const double r0 = fr ? fr[3 * j] : (j == 0 ? 1.0 : 0.0);
+        const double r1 = fr ? fr[3 * j + 1] : (j == 1 ? 1.0 : 0.0);
+        const double r2 = fr ? fr[3 * j + 2] : (j == 2 ? 1.0 : 0.0);
+        w64[j] = (r0 * vg64[0] + r1 * vg64[1]) + r2 * vg64[2];
+        w[j] = float(w64[j]);
+      }
+      // the segment length as the FP64 mode (and the reference) takes it: of
+      // the vector rotated by the FP64 frame, which a triangle's single-
+      // precision file normal leaves orthonormal only to ~1e-7, so the
+      // global length would move the phase k*L of a long path by ~1e-4 rad
+      out.r = sqrt((w64[0] * w64[0] + w64[1] * w64[1]) + w64[2] * w64[2]);
+      const float rho = sqrtf(w[0] * w[0] + w[1] * w[1]);
+      const float len = sqrtf(rho * rho + w[2] * w[2]);
+      if (len > 0.0f) {
+        out.st = double(rho / len);
+        out.ct = double(w[2] / len);
+      } else {  // the zero vector: theta = pi/2, phi = 0 (VecMatDef.h:132-155)
+        out.st = 1.0;
+        out.ct = 0.0;
+      }
+      out.sp = rho > 0.0f ? double(w[1] / rho) : 0.0;
+      out.cp = rho > 0.0f ? double(w[0] / rho) : 1.0;
+      th = atan2(rho, w[2]);  // the pattern's angles
+      if (len == 0.0f) th = R(K.pi_hi * 0.5);
+      ph = atan2(w[1], w[0]);
+      if (ph < R(0)) ph = R((double(ph) + 2.0 * K.pi_hi) + 2.0 * K.pi_lo);
+    }
+    for (int j = 0; j < 6; ++j) out.inc[j] = 0.0;
+    if (i == 0) {
+      Cx<R> inc[3] = {cx(R(0)), cx(R(0)), cx(R(0))};
+      if constexpr (sizeof(R) == sizeof(double)) {
+        if (antenna == 0) inc[0] = cx(R(0), R(sqrt(60.0 * pt)));
+        if (antenna == 1) inc[1] = cx(R(0), R(sqrt(60.0 * pt * 1.5)) * sin(th));
+        else if (antenna == 2)
+          inc[1] = cx(R(0), R(sqrt(60.0 * pt)) * (cos(R(K.pi_hi) * cos(th) / R(2)) / sin(th)));
+      } else {
+        // FP32: sin and cos of theta from the segment's components (accurate
+        // to ulps, unlike sin(theta) near the dipole axis, where theta's own
+        // FP32 rounding is most of sin(theta)).  The half-wave pattern's
+        // cos(pi/2 cos th) is sin(pi s) with s = sin^2(th/2) = st^2 / (2 (1 + ct))
+        // or cos^2(th/2) = st^2 / (2 (1 - ct)), whichever is at most 1/2: no
+        // cancellation near the axis, where cos(pi/2 cos th) -> 0.
+        const float st = float(out.st), ct = float(out.ct);
+        if (antenna == 0) inc[0] = cx(R(0), R(sqrt(60.0 * pt)));
+        if (antenna == 1) inc[1] = cx(R(0), R(sqrt(60.0 * pt * 1.5)) * st);
+        else if (antenna == 2) {
+          const float h2 = (st * st) / (2.0f * (ct >= 0.0f ? 1.0f + ct : 1.0f - ct));
+          inc[1] = cx(R(0), R(sqrt(60.0 * pt)) * (sinf(float(K.pi_hi) * h2) / st));
+        }
+      }
+      if (antenna == 3 && pat) {
+        double a[4];
+        pattern_at(*pat, double(th) * (180.0 / K.pi_hi), double(ph) * (180.0 / K.pi_hi), a);
+        const double amp = sqrt(60.0 * pt);
+        inc[1] = cx(R(amp * a[0]), R(amp * a[1]));
+        inc[2] = cx(R(amp * a[2]), R(amp * a[3]));
+      }
+      for (int j = 0; j < 3; ++j) {
+        out.inc[2 * j] = double(inc[j].re);
+        out.inc[2 * j + 1] = double(inc[j].im);
       }
     }
-    if (antenna == 3 && pat) {
-      double a[4];
-      pattern_at(*pat, double(th) * (180.0 / K.pi_hi), double(ph) * (180.0 / K.pi_hi), a);
-      const double amp = sqrt(60.0 * pt);
-      inc[1] = cx(R(amp * a[0]), R(amp * a[1]));
-      inc[2] = cx(R(amp * a[2]), R(amp * a[3]));
-    }
-    for (int j = 0; j < 3; ++j) {
-      out.inc[2 * j] = double(inc[j].re);
-      out.inc[2 * j + 1] = double(inc[j].im);
-    }
   }
+  if (part == kSegDirection) return;
+  const double lam64 = 2.99792458e8 / freq;
+  out.fp64_fresnel = 0;
+  out.pad = 0;
   Cx<R> ctm = cx(R(1)), cte = cx(R(1));
   if (kind[i] != 0) {
     // AngleBetween(vecGlobal, current row 2) in radians (VecMatDef.h:56-77),

@@ -222,6 +222,10 @@ struct FieldArgs {
   double* path_pts;     // (kMaxDepth + 2) * 3 per survivor
   SegTerms* seg;        // (kMaxDepth + 1) per survivor
   int* path_mat;        // (kMaxDepth + 1) per survivor: material of each ray's start
+  // k_seg's tasks, path << 5 | segment: every segment's direction, every
+  // interaction (Counters::seg_tasks, int_tasks of them)
+  uint32_t* seg_list;
+  uint32_t* int_list;
   // FP32 field mode: bound on each component's absolute error per survivor
   // (0: computed in FP64; -1: no bound, the FP32-phase study mode)
   double* path_bound;
@@ -232,6 +236,8 @@ struct FieldArgs {
 // FP32 field mode: a path whose condition number (path_combine's kappa)
 // exceeds this is computed in FP64.
 constexpr float kKappaMax32 = 32.0f;
+// path_bound of a path whose FP64 field is still to come (k_escalate).
+constexpr double kBoundRedo = -2.0;
 
 // Barycentric distance of a point (on the triangle's plane) from the
 // triangle's edges is below tol: min(u, v, 1-u-v) < tol.
@@ -254,31 +260,58 @@ __device__ __forceinline__ int near_edge(const CorrTri& T, const double* p, doub
 // segment); k_combine carries each path's field along it.
 __global__ void k_path(FieldArgs A) {
   const unsigned long long ns = min(A.ctr->survivors, A.cap);
-  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < ns;
-       i += (unsigned long long)gridDim.x * blockDim.x) {
-    const Survivor sv = A.surv[i];
-    const TxParams& P = A.txp[A.rx_req[sv.rx]];
-    PathBuf pb;
-    class_path(A.cls_info, sv.cls, pb);
-    correct_path(A.sc, A.rank_to_id, P, A.rx + 3 * size_t(sv.rx), pb);
-    A.path_nray[i] = pb.n;
-    const size_t b = size_t(i) * (kMaxDepth + 1);
-    for (int r = 0; r < pb.n; ++r) {
-      const int t = pb.tri[r];
-      A.path_tri[b + r] = t >= 0 ? A.rank_to_id[t] : -1;
-      A.path_cop[b + r] = t >= 0 ? A.sc.tri64[t].cop : -1;
-      A.path_kind[b + r] = pb.kind[r];
-      // the hit triangle's own material (the ray's hit record carries it)
-      A.path_mat[b + r] = r > 0 ? A.sc.tri64[pb.tri[r - 1]].mat : 0;
+  const unsigned lane = threadIdx.x & 31u;
+  for (unsigned long long i0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) & ~31ull;
+       i0 < ns; i0 += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned long long i = i0 + lane;
+    int n = 0;
+    if (i < ns) {
+      const Survivor sv = A.surv[i];
+      const TxParams& P = A.txp[A.rx_req[sv.rx]];
+      PathBuf pb;
+      class_path(A.cls_info, sv.cls, pb);
+      correct_path(A.sc, A.rank_to_id, P, A.rx + 3 * size_t(sv.rx), pb);
+      A.path_nray[i] = n = pb.n;
+      const size_t b = size_t(i) * (kMaxDepth + 1);
+      for (int r = 0; r < pb.n; ++r) {
+        const int t = pb.tri[r];
+        A.path_tri[b + r] = t >= 0 ? A.rank_to_id[t] : -1;
+        A.path_cop[b + r] = t >= 0 ? A.sc.tri64[t].cop : -1;
+        A.path_kind[b + r] = pb.kind[r];
+        // the hit triangle's own material (the ray's hit record carries it)
+        A.path_mat[b + r] = r > 0 ? A.sc.tri64[pb.tri[r - 1]].mat : 0;
+      }
+      const size_t bp = size_t(i) * (kMaxDepth + 2) * 3;
+      for (int r = 0; r <= pb.n; ++r)
+        for (int a = 0; a < 3; ++a) A.path_pts[bp + 3 * r + a] = pb.pts[r][a];
+      // interaction point r+1 lies on the triangle the correction intersected
+      int near = 0;
+      for (int r = 0; r + 1 < pb.n; ++r)
+        near |= near_edge(A.sc.corr[A.rank_to_id[pb.tri[r]]], pb.pts[r + 1], 1e-6);
+      A.path_near_edge[i] = near;
     }
-    const size_t bp = size_t(i) * (kMaxDepth + 2) * 3;
-    for (int r = 0; r <= pb.n; ++r)
-      for (int a = 0; a < 3; ++a) A.path_pts[bp + 3 * r + a] = pb.pts[r][a];
-    // interaction point r+1 lies on the triangle the correction intersected
-    int near = 0;
-    for (int r = 0; r + 1 < pb.n; ++r)
-      near |= near_edge(A.sc.corr[A.rank_to_id[pb.tri[r]]], pb.pts[r + 1], 1e-6);
-    A.path_near_edge[i] = near;
+    __syncwarp();
+    // the path's segments and its interactions (all segments but the first)
+    int incl = n, m = n > 0 ? 1 : 0;  // segments; paths
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o), w = __shfl_up_sync(0xffffffffu, m, o);
+      if (int(lane) >= o) {
+        incl += v;
+        m += w;
+      }
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31), paths = __shfl_sync(0xffffffffu, m, 31);
+    unsigned long long bs = 0, bi = 0;
+    if (lane == 0) {
+      bs = atomicAdd(&A.ctr->seg_tasks, (unsigned long long)total);
+      bi = atomicAdd(&A.ctr->int_tasks, (unsigned long long)(total - paths));
+    }
+    bs = __shfl_sync(0xffffffffu, bs, 0) + (incl - n);
+    bi = __shfl_sync(0xffffffffu, bi, 0) + (incl - n) - (m - (n > 0 ? 1 : 0));
+    for (int r = 0; r < n; ++r) {
+      A.seg_list[bs + r] = uint32_t(i) << 5 | uint32_t(r);
+      if (r > 0) A.int_list[bi + r - 1] = uint32_t(i) << 5 | uint32_t(r);
+    }
   }
 }
 
@@ -292,11 +325,13 @@ struct PathView {
   int mat[kMaxDepth + 1];
 };
 
-__device__ __forceinline__ void path_view(const FieldArgs& A, unsigned long long i, PathView& v) {
+// (of its rays [from, to) where the caller reads no other).
+__device__ __forceinline__ void path_view(const FieldArgs& A, unsigned long long i, PathView& v,
+                                          int from = 0, int to = kMaxDepth + 1) {
   v.n = A.path_nray[i];
   v.pts = reinterpret_cast<const double(*)[3]>(A.path_pts + size_t(i) * (kMaxDepth + 2) * 3);
   const size_t b = size_t(i) * (kMaxDepth + 1);
-  for (int r = 0; r < v.n; ++r) {
+  for (int r = from; r < min(v.n, to); ++r) {
     // frames by the id's position in the caller's mesh vector, as the
     // reference looks them up (FieldCompute.cpp:107)
     const int id = A.path_tri[b + r];
@@ -306,28 +341,39 @@ __device__ __forceinline__ void path_view(const FieldArgs& A, unsigned long long
   }
 }
 
+// One thread per direction task, then one per interaction task.  Chains of
+// FP64 instructions (angles, complex functions), so the two parts of a segment
+// run side by side, and the tasks are dense: by (path, segment slot) a batch of
+// 9,567 paths kept 5 of 32 lanes busy.
 __global__ void k_seg(FieldArgs A) {
-  const unsigned long long ns = min(A.ctr->survivors, A.cap);
-  const unsigned long long n_slots = ns * (kMaxDepth + 1);
+  const unsigned long long ns_t = A.ctr->seg_tasks, ni_t = A.ctr->int_tasks;
+  const unsigned long long first_i = (ns_t + 31) & ~31ull;  // no warp holds both kinds
   for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-       k < n_slots; k += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long i = k / (kMaxDepth + 1);
-    const int r = int(k % (kMaxDepth + 1));
-    if (r >= A.path_nray[i]) continue;
+       k < first_i + ni_t; k += (unsigned long long)gridDim.x * blockDim.x) {
+    if (k >= ns_t && k < first_i) continue;
+    const bool inter = k >= first_i;
+    const uint32_t task = inter ? A.int_list[k - first_i] : A.seg_list[k];
+    const unsigned long long i = task >> 5;
+    const int r = int(task & 31u);
     const Survivor sv = A.surv[i];
     const TxParams& P = A.txp[A.rx_req[sv.rx]];
     PathView v;
-    path_view(A, i, v);
+    path_view(A, i, v, max(r - 1, 0), r + 1);
     const PatternTab pat{P.pat, P.pat_nt, P.pat_np, P.pat_dt, P.pat_dp};
     const int prec = A.precision < 0 ? P.precision : A.precision;
-    SegTerms t;
+    SegTerms& t = A.seg[i * (kMaxDepth + 1) + r];
+    const int part = inter ? kSegInteraction : kSegDirection;
+    if (!inter && r == 0) {  // no interaction at the start
+      t.fp64_fresnel = 0;
+      t.ctm[0] = t.cte[0] = 1.0;
+      t.ctm[1] = t.cte[1] = 0.0;
+    }
     if (prec != 0)
       seg_terms<float>(r, v.pts, v.frames, v.kind, v.mat, A.sc.mats, P.txcs, P.freq, P.pt,
-                       P.antenna, P.fresnel != 0, A.K, t, &pat);
+                       P.antenna, P.fresnel != 0, A.K, t, &pat, part);
     else
       seg_terms<double>(r, v.pts, v.frames, v.kind, v.mat, A.sc.mats, P.txcs, P.freq, P.pt,
-                        P.antenna, P.fresnel != 0, A.K, t, &pat);
-    A.seg[k] = t;
+                        P.antenna, P.fresnel != 0, A.K, t, &pat, part);
   }
 }
 
@@ -339,7 +385,7 @@ __global__ void k_combine(FieldArgs A) {
     const TxParams& P = A.txp[A.rx_req[sv.rx]];
     PathView v;
     path_view(A, i, v);
-    SegTerms* seg = A.seg + size_t(i) * (kMaxDepth + 1);
+    const SegTerms* seg = A.seg + size_t(i) * (kMaxDepth + 1);
     Cx<double> e[3];
     const int prec = A.precision < 0 ? P.precision : A.precision;
     double bound = 0.0;
@@ -352,13 +398,7 @@ __global__ void k_combine(FieldArgs A) {
       bool pole = false;
       for (int r = 0; r < v.n; ++r) pole |= seg[r].fp64_fresnel != 0;
       if (pole || !(kappa <= kKappaMax32)) {
-        // an ill-conditioned path: its terms and field again, in FP64
-        const PatternTab pat{P.pat, P.pat_nt, P.pat_np, P.pat_dt, P.pat_dp};
-        for (int r = 0; r < v.n; ++r)
-          seg_terms<double>(r, v.pts, v.frames, v.kind, v.mat, A.sc.mats, P.txcs, P.freq, P.pt,
-                            P.antenna, P.fresnel != 0, A.K, seg[r], &pat);
-        path_combine<double>(v.n, seg, v.pts, v.frames, v.kind, P.txcs, P.freq, A.K, e);
-        atomicAdd(&A.fstat[0], 1ull);
+        bound = kBoundRedo;  // an ill-conditioned path: k_escalate takes it in FP64
       } else {
         // each component errs by at most (7 kappa) ulps of |E| (measured on
         // every path of the urban canyon); the bound takes 16 kappa, plus
@@ -378,31 +418,41 @@ __global__ void k_combine(FieldArgs A) {
   }
 }
 
-// FP32 field mode, receivers k_rx_sum could not certify: every path of such
-// a receiver gets its terms and field again in FP64 (k_rx_sum then sums the
-// receiver in FP64).
-__global__ void k_escalate(FieldArgs A) {
+// FP32 field mode: terms and field again in FP64, first (receivers = false) for
+// the ill-conditioned paths k_combine marked, then for every path of the
+// receivers k_rx_sum could not certify (it then sums those in FP64).  One warp
+// per path, a lane per segment: one thread going through a path's segments
+// took 280 and 140 us in the canyon with slab walls (its whole field stage
+// 0.54 ms, now 0.30).
+__global__ void k_escalate(FieldArgs A, bool receivers) {
   const unsigned long long ns = min(A.ctr->survivors, A.cap);
-  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < ns;
-       i += (unsigned long long)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (unsigned long long i = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
+       i < ns; i += ((unsigned long long)gridDim.x * blockDim.x) >> 5) {
     const Survivor sv = A.surv[i];
-    if (!A.rx_flag[sv.rx] || A.path_bound[i] == 0.0) continue;  // taken in FP64 already
+    const double state = A.path_bound[i];
+    // (bound 0: taken in FP64 already)
+    if (receivers ? !A.rx_flag[sv.rx] || state == 0.0 : state != kBoundRedo) continue;
     const TxParams& P = A.txp[A.rx_req[sv.rx]];
     PathView v;
     path_view(A, i, v);
     SegTerms* seg = A.seg + size_t(i) * (kMaxDepth + 1);
     const PatternTab pat{P.pat, P.pat_nt, P.pat_np, P.pat_dt, P.pat_dp};
-    for (int r = 0; r < v.n; ++r)
-      seg_terms<double>(r, v.pts, v.frames, v.kind, v.mat, A.sc.mats, P.txcs, P.freq, P.pt,
-                        P.antenna, P.fresnel != 0, A.K, seg[r], &pat);
-    Cx<double> e[3];
-    path_combine<double>(v.n, seg, v.pts, v.frames, v.kind, P.txcs, P.freq, A.K, e);
-    for (int j = 0; j < 3; ++j) {
-      A.path_field[6 * i + 2 * j] = e[j].re;
-      A.path_field[6 * i + 2 * j + 1] = e[j].im;
+    if (lane < v.n)
+      seg_terms<double>(lane, v.pts, v.frames, v.kind, v.mat, A.sc.mats, P.txcs, P.freq, P.pt,
+                        P.antenna, P.fresnel != 0, A.K, seg[lane], &pat);
+    __syncwarp();
+    if (lane == 0) {
+      Cx<double> e[3];
+      path_combine<double>(v.n, seg, v.pts, v.frames, v.kind, P.txcs, P.freq, A.K, e);
+      for (int j = 0; j < 3; ++j) {
+        A.path_field[6 * i + 2 * j] = e[j].re;
+        A.path_field[6 * i + 2 * j + 1] = e[j].im;
+      }
+      A.path_bound[i] = 0.0;
+      atomicAdd(&A.fstat[0], 1ull);
     }
-    A.path_bound[i] = 0.0;
-    atomicAdd(&A.fstat[0], 1ull);
+    __syncwarp();
   }
 }
 
