@@ -797,7 +797,7 @@ static void sort_perm_by(DBuf<int>& perm, DBuf<int>& tmp, DBuf<int>& flags, DBuf
 // numbers the nodes depth-first as the host build does.  v: the device
 // copy of the vertices (9 floats per triangle).
 struct RefSort {
-  DBuf<double> key;
+  DBuf<refbvh::Key> key;
   DBuf<int> idx, lpos, rpos, tile_seg, cnt_l, cnt_r, off_l, off_r;
   DBuf<int2> totals;
   DBuf<refbvh::SortSeg> big, big_next, small, tiny, heap;
@@ -855,10 +855,11 @@ static void ref_sort(RefSort& R, const refbvh::RNode* nodes, const int* active, 
     std::swap(R.big.n, R.big_next.n);
   }
   if (h[kSmall])
-    k_small<kSmallMax><<<std::min(h[kSmall], R.sms * 8), 32, small_smem<kSmallMax>(), st>>>(
-        R.small.p, R.ctl.p + kSmall, 0, R.key.p, R.idx.p, R.ctl.p);
+    k_small<kSmallMax, kSmallWarps>
+        <<<std::min(h[kSmall], R.sms * 4), 32 * kSmallWarps, small_smem<kSmallMax>(), st>>>(
+            R.small.p, R.ctl.p + kSmall, 0, R.key.p, R.idx.p, R.ctl.p);
   if (h[kShort])
-    k_small<kShortMax><<<std::min(h[kShort], R.sms * 32), 32, small_smem<kShortMax>(), st>>>(
+    k_small<kShortMax, 1><<<std::min(h[kShort], R.sms * 32), 32, small_smem<kShortMax>(), st>>>(
         R.small.p, R.ctl.p + kShort, R.small_cap, R.key.p, R.idx.p, R.ctl.p);
   if (h[kSmall] + h[kShort] > R.small_cap)
     throw std::string("device reference BVH: small segment list overflow");
@@ -1148,10 +1149,12 @@ static void device_prepare(const float* v_host, const float* n_host, int nt, cud
   int n_segs = 1;
   for (int level = 0; n_segs > 0; ++level) {
     if (level > 200) throw std::string("device search BVH deeper than 200 levels");
-    prep::k_plan<<<n_segs, 256, 0, st>>>(segs.p, n_segs, ord.p, blo.p, bhi.p, cen.p, nodes.p,
+    // a block per segment, as wide as the level's segments are long on average
+    const int per = nt / n_segs, threads = per > 2048 ? 1024 : (per > 128 ? 256 : 32);
+    prep::k_plan<<<n_segs, threads, 0, st>>>(segs.p, n_segs, ord.p, blo.p, bhi.p, cen.p, nodes.p,
                                          ctl.p, plans.p, ctl.p + 2, ctl.p + 3, root_box.p);
-    prep::k_partition<<<n_segs, 256, 0, st>>>(segs.p, n_segs, plans.p, ord.p, otmp.p, cen.p);
-    prep::k_median<<<n_segs, 256, 0, st>>>(segs.p, n_segs, plans.p, ord.p, otmp.p, cen.p,
+    prep::k_partition<<<n_segs, threads, 0, st>>>(segs.p, n_segs, plans.p, ord.p, otmp.p, cen.p);
+    prep::k_median<<<n_segs, threads, 0, st>>>(segs.p, n_segs, plans.p, ord.p, otmp.p, cen.p,
                                            ctl.p + 4);
     CK(cudaMemsetAsync(ctl.p + 1, 0, sizeof(int), st));
     prep::k_children<<<grid_for(n_segs, 256), 256, 0, st>>>(segs.p, n_segs, plans.p, next.p,

@@ -284,14 +284,35 @@ __global__ void k_plan(const Seg* segs, int n_segs, const int* ord, const float*
     }
   }
   __syncthreads();
-  for (int i = S.b + threadIdx.x; i < S.e; i += blockDim.x) {
-    const int p = ord[i];
+  {  // bounds per thread, per warp, then one atomic each
+    int v[12];
     for (int a = 0; a < 3; ++a) {
-      atomicMin(&sbox[a], f2o(blo[3 * p + a]));
-      atomicMax(&sbox[3 + a], f2o(bhi[3 * p + a]));
-      atomicMin(&scb[a], f2o(cen[3 * p + a]));
-      atomicMax(&scb[3 + a], f2o(cen[3 * p + a]));
+      v[a] = v[6 + a] = INT_MAX;
+      v[3 + a] = v[9 + a] = INT_MIN;
     }
+    for (int i = S.b + threadIdx.x; i < S.e; i += blockDim.x) {
+      const int p = ord[i];
+      for (int a = 0; a < 3; ++a) {
+        const int c = f2o(cen[3 * p + a]);
+        v[a] = min(v[a], f2o(blo[3 * p + a]));
+        v[3 + a] = max(v[3 + a], f2o(bhi[3 * p + a]));
+        v[6 + a] = min(v[6 + a], c);
+        v[9 + a] = max(v[9 + a], c);
+      }
+    }
+    for (int a = 0; a < 3; ++a) {
+      v[a] = __reduce_min_sync(0xffffffffu, v[a]);
+      v[3 + a] = __reduce_max_sync(0xffffffffu, v[3 + a]);
+      v[6 + a] = __reduce_min_sync(0xffffffffu, v[6 + a]);
+      v[9 + a] = __reduce_max_sync(0xffffffffu, v[9 + a]);
+    }
+    if ((threadIdx.x & 31) == 0)
+      for (int a = 0; a < 3; ++a) {
+        atomicMin(&sbox[a], v[a]);
+        atomicMax(&sbox[3 + a], v[3 + a]);
+        atomicMin(&scb[a], v[6 + a]);
+        atomicMax(&scb[3 + a], v[9 + a]);
+      }
   }
   __syncthreads();
   const int n = S.e - S.b;
@@ -427,13 +448,14 @@ __global__ void k_partition(const Seg* segs, int n_segs, SegPlan* plans, int* or
     const unsigned bal = __ballot_sync(0xffffffffu, f);
     if (lane == 0) warp_sum[wid] = __popc(bal);
     __syncthreads();
-    int before = carry;
-    for (int w = 0; w < wid; ++w) before += warp_sum[w];
-    before += __popc(bal & ((1u << lane) - 1u));
+    int before = carry + __reduce_add_sync(0xffffffffu, lane < wid ? warp_sum[lane] : 0) +
+                 __popc(bal & ((1u << lane) - 1u));
     if (f) tmp[S.b + before] = p;
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < nw; ++w) carry += warp_sum[w];
+    if (wid == 0) {
+      const int all = __reduce_add_sync(0xffffffffu, lane < nw ? warp_sum[lane] : 0);
+      if (lane == 0) carry += all;
+    }
     __syncthreads();
   }
   const int n_left = carry;
@@ -448,13 +470,14 @@ __global__ void k_partition(const Seg* segs, int n_segs, SegPlan* plans, int* or
     const unsigned bal = __ballot_sync(0xffffffffu, f);
     if (lane == 0) warp_sum[wid] = __popc(bal);
     __syncthreads();
-    int before = carry;
-    for (int w = 0; w < wid; ++w) before += warp_sum[w];
-    before += __popc(bal & ((1u << lane) - 1u));
+    int before = carry + __reduce_add_sync(0xffffffffu, lane < wid ? warp_sum[lane] : 0) +
+                 __popc(bal & ((1u << lane) - 1u));
     if (f) tmp[S.b + n_left + before] = p;
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < nw; ++w) carry += warp_sum[w];
+    if (wid == 0) {
+      const int all = __reduce_add_sync(0xffffffffu, lane < nw ? warp_sum[lane] : 0);
+      if (lane == 0) carry += all;
+    }
     __syncthreads();
   }
   for (int i = S.b + threadIdx.x; i < S.e; i += blockDim.x) ord[i] = tmp[i];

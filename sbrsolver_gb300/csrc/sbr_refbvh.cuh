@@ -40,8 +40,9 @@ namespace refbvh {
 
 constexpr int kTile = 2048;        // elements per block of the partition rounds
 constexpr int kTileThreads = 256;  // 8 consecutive elements per thread
-constexpr int kSmallMax = 2048;    // longest segment one warp sorts in shared memory
-constexpr int kShortMax = 256;     // segments up to this long use the lighter warp sort
+constexpr int kSmallMax = 2048;    // longest segment one block sorts in shared memory
+constexpr int kShortMax = 256;     // segments up to this long take one warp
+constexpr int kSmallWarps = 8;     // warps for the longer ones
 constexpr int kInsertion = 16;     // segments this short wait for insertion sort
 
 struct __align__(16) SortSeg {
@@ -71,26 +72,64 @@ enum Ctl {
 __device__ __forceinline__ int floor_log2(int n) { return 31 - __clz(n); }
 
 
-// Box centre along axis a exactly as the reference computes it from the
-// box of float vertices: (min + max) / 2 in FP64.
-__device__ __forceinline__ double centre(const float4& lo, const float4& hi, int a) {
+// Sort keys: the reference sorts by box centres, (min + max) / 2 in FP64 of
+// the box of float vertices.  The sum orders like its half, and the integer
+// like the sum (-0 and +0 alike; the coordinates are finite), so the sort's
+// comparisons stay off the FP64 pipe, where each takes a warp ~76 cycles
+// (with the sweeps' integer products the canyon's tree 11.6 -> 10.2 ms).
+typedef long long Key;
+__device__ __forceinline__ Key centre_key(const float4& lo, const float4& hi, int a) {
   const float l = a == 0 ? lo.x : (a == 1 ? lo.y : lo.z);
   const float h = a == 0 ? hi.x : (a == 1 ? hi.y : hi.z);
-  return __ddiv_rn(__dadd_rn(double(l), double(h)), 2.0);
+  const long long b = __double_as_longlong(__dadd_rn(double(l), double(h)));
+  return b >= 0 ? b : -(b & 0x7fffffffffffffffll);
 }
 
 // Surface area of a box as the host computes it (sbr_host.cpp
 // surface_area): 0 for a box that is flat or empty along any axis, else
-// 2 (dx dy + dy dz + dz dx) with every operation rounded on its own.
+// 2 (dx dy + dy dz + dz dx) with every operation rounded on its own (products
+// and conversions in integer arithmetic where the extents allow).
 __device__ __forceinline__ double surface_area(float lx, float ly, float lz, float hx, float hy,
                                                float hz) {
   if (hx <= lx || hy <= ly || hz <= lz) return 0.0;
-  const double dx = __dsub_rn(double(hx), double(lx));
-  const double dy = __dsub_rn(double(hy), double(ly));
-  const double dz = __dsub_rn(double(hz), double(lz));
-  const double s = __dadd_rn(__dadd_rn(__dmul_rn(dx, dy), __dmul_rn(dy, dz)), __dmul_rn(dz, dx));
-  return __dmul_rn(2.0, s);
+  using soft64::from_f32;
+  const double dx = __dsub_rn(from_f32(hx), from_f32(lx));
+  const double dy = __dsub_rn(from_f32(hy), from_f32(ly));
+  const double dz = __dsub_rn(from_f32(hz), from_f32(lz));
+  double s;
+  if (soft64::safe(dx) && soft64::safe(dy) && soft64::safe(dz))
+    s = __dadd_rn(__dadd_rn(soft64::mul(dx, dy), soft64::mul(dy, dz)), soft64::mul(dz, dx));
+  else
+    s = __dadd_rn(__dadd_rn(__dmul_rn(dx, dy), __dmul_rn(dy, dz)), __dmul_rn(dz, dx));
+  return __dadd_rn(s, s);
 }
+
+// Cost of splitting n objects after the i-th, 2 + (i sa1 + (n - i) sa2) / sr
+// with each operation rounded on its own; sr = SA(node box).
+struct SplitCost {
+  double sr;
+  uint64_t x;  // its mantissa's reciprocal
+  bool soft;   // sr is nonzero and in range: areas of extents in soft64's range, and
+               // n times them, are too
+  __device__ __forceinline__ explicit SplitCost(double s) : sr(s), x(0) {
+    const uint32_t e = uint32_t(soft64::bits(s) >> 52) & 0x7ffu;
+    soft = e > 1023 - 300 && e < 1023 + 260;
+    if (soft) x = soft64::rcp_of(s);
+  }
+  __device__ __forceinline__ double operator()(int i, int n, double sa1, double sa2) const {
+    auto in_range = [](double v) {  // 0, or within [2^-300, 2^260)
+      const uint32_t e = uint32_t(soft64::bits(v) >> 52) & 0x7ffu;
+      return soft64::bits(v) == 0 || (e > 1023 - 300 && e < 1023 + 260);
+    };
+    if (soft && in_range(sa1) && in_range(sa2)) {
+      const double num = __dadd_rn(soft64::mul(soft64::from_int(i), sa1),
+                                   soft64::mul(soft64::from_int(n - i), sa2));
+      return __dadd_rn(2.0, soft64::div_by(num, sr, x));
+    }
+    const double num = __dadd_rn(__dmul_rn(double(i), sa1), __dmul_rn(double(n - i), sa2));
+    return __dadd_rn(2.0, __ddiv_rn(num, sr));
+  }
+};
 
 // ---- per-triangle boxes ----------------------------------------------------
 
@@ -118,7 +157,7 @@ __global__ void k_boxes(const float* v, int nt, float4* lo, float4* hi) {
 
 template <class K, class I>
 __device__ __forceinline__ void swap_pair(K* key, I* idx, int a, int b) {
-  const double k = key[a];
+  const K k = key[a];
   key[a] = key[b];
   key[b] = k;
   const int i = idx[a];
@@ -148,7 +187,7 @@ __device__ __forceinline__ void median_to_first(K* key, I* idx, int r, int a, in
 template <class K, class I>
 __device__ void insertion_sort(K* key, I* idx, int f, int l) {
   for (int i = f + 1; i < l; ++i) {
-    const double k = key[i];
+    const K k = key[i];
     const int x = idx[i];
     int j = i;
     while (j > f && k < key[j - 1]) {
@@ -166,7 +205,7 @@ __device__ void insertion_sort(K* key, I* idx, int f, int l) {
 // (the hole goes down to the larger child, the right one on ties, to the
 // bottom, then the value climbs back), then the root is popped n - 1 times.
 template <class K, class I>
-__device__ void heap_push(K* key, I* idx, long hole, long top, double v, int vi) {
+__device__ void heap_push(K* key, I* idx, long hole, long top, K v, int vi) {
   long parent = (hole - 1) / 2;
   while (hole > top && key[parent] < v) {
     key[hole] = key[parent];
@@ -178,7 +217,7 @@ __device__ void heap_push(K* key, I* idx, long hole, long top, double v, int vi)
   idx[hole] = vi;
 }
 template <class K, class I>
-__device__ void heap_adjust(K* key, I* idx, long hole, long len, double v, int vi) {
+__device__ void heap_adjust(K* key, I* idx, long hole, long len, K v, int vi) {
   const long top = hole;
   long child = hole;
   while (child < (len - 1) / 2) {
@@ -205,7 +244,7 @@ __device__ void heap_sort(K* key, I* idx, long n) {
     }
   for (long last = n; last > 1;) {
     --last;
-    const double v = key[last];
+    const K v = key[last];
     const int vi = idx[last];
     key[last] = key[0];
     idx[last] = idx[0];
@@ -263,7 +302,7 @@ __global__ void k_tile_map(const SortSeg* big, const int* n_big, int* tile_seg) 
 }
 
 // Round step 1: the median of three to the front of every big segment.
-__global__ void k_pivot(const SortSeg* big, int n_big, double* key, int* idx) {
+__global__ void k_pivot(const SortSeg* big, int n_big, Key* key, int* idx) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n_big) return;
   const SortSeg g = big[s];
@@ -272,11 +311,11 @@ __global__ void k_pivot(const SortSeg* big, int n_big, double* key, int* idx) {
 
 // Stop flags of position p of segment g around pivot key pk: left stops in
 // [f + 1, l), right stops in [f, l).
-__device__ __forceinline__ void stop_flags(const double* key, const SortSeg& g, double pk, int p,
+__device__ __forceinline__ void stop_flags(const Key* key, const SortSeg& g, Key pk, int p,
                                            int& lf, int& rf) {
   lf = rf = 0;
   if (p >= g.l) return;
-  const double k = key[p];
+  const Key k = key[p];
   lf = p > g.f && !(k < pk);
   rf = !(pk < k);
 }
@@ -309,12 +348,12 @@ __device__ __forceinline__ int block_exclusive(int v, int& excl, int* sh) {
 
 // Round step 2: stop counts per tile.
 __global__ void __launch_bounds__(kTileThreads) k_count(const SortSeg* big, const int* tile_seg,
-                                                        const double* key, int* cnt_l,
+                                                        const Key* key, int* cnt_l,
                                                         int* cnt_r) {
   __shared__ int sh[64];
   const int tile = blockIdx.x;
   const SortSeg g = big[tile_seg[tile]];
-  const double pk = key[g.f];
+  const Key pk = key[g.f];
   const int base = g.f + (tile - g.tile0) * kTile + threadIdx.x * (kTile / kTileThreads);
   int nl = 0, nr = 0;
   for (int j = 0; j < kTile / kTileThreads; ++j) {
@@ -352,14 +391,14 @@ __global__ void k_tile_offsets(const SortSeg* big, int n_big, const int* cnt_l, 
 // Round step 4: the stops' positions, left stops ascending in lpos[f ..],
 // right stops descending in rpos[f ..].
 __global__ void __launch_bounds__(kTileThreads) k_stops(const SortSeg* big, const int* tile_seg,
-                                                        const double* key, const int* off_l,
+                                                        const Key* key, const int* off_l,
                                                         const int* off_r, const int2* totals,
                                                         int* lpos, int* rpos) {
   __shared__ int sh[64];
   const int tile = blockIdx.x;
   const int s = tile_seg[tile];
   const SortSeg g = big[s];
-  const double pk = key[g.f];
+  const Key pk = key[g.f];
   const int base = g.f + (tile - g.tile0) * kTile + threadIdx.x * (kTile / kTileThreads);
   int lf[kTile / kTileThreads], rf[kTile / kTileThreads];
   int nl = 0, nr = 0;
@@ -384,7 +423,7 @@ __global__ void __launch_bounds__(kTileThreads) k_stops(const SortSeg* big, cons
 __global__ void __launch_bounds__(kTileThreads) k_exchange(const SortSeg* big,
                                                            const int* tile_seg,
                                                            const int2* totals, const int* lpos,
-                                                           const int* rpos, double* key,
+                                                           const int* rpos, Key* key,
                                                            int* idx) {
   const int tile = blockIdx.x;
   const int s = tile_seg[tile];
@@ -424,122 +463,139 @@ __global__ void k_cut(const SortSeg* big, int n_big, const int2* totals, const i
                kTilesNext);
 }
 
-// A warp per segment of at most kSmallMax: the segment is sorted in shared
-// memory (partition by the warp, exchanges spread over its lanes), then the
-// leftover segments of at most 16 are insertion sorted, one per lane.
-template <int kCap>
+// A block per segment of at most kCap, sorted in shared memory: the segments a
+// partition leaves are independent, so the block's warps take one each, round
+// by round (a partition by the warp, its exchanges spread over the lanes);
+// segments of at most 16 wait for the end, when they are insertion sorted,
+// one per thread.  A chain of shared-memory passes: with one warp for all of
+// a segment's partitions the canyon's tree spent 4.3 ms here, with eight 2.1.
+struct SortPart {
+  short f, l, d, pad;
+};
+template <int kCap>  // at most kCap / kInsertion parts at one time
 constexpr size_t small_smem() {
-  return size_t(kCap) * (8 + 4 + 2 + 2 + 4);
+  return size_t(kCap) * (8 + 4 + 2 + 2 + 4) + 2 * sizeof(SortPart) * (kCap / kInsertion);
 }
 
 // segs: the list; n_segs: its count; from_end > 0: the list is read from
 // its end (entry from_end - 1 - s, from_end being the list's capacity).
-template <int kCap>
-__global__ void __launch_bounds__(32) k_small(const SortSeg* segs, const int* n_segs,
-                                              int from_end, double* key, int* idx, int* ctl) {
+template <int kCap, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) k_small(const SortSeg* segs, const int* n_segs,
+                                                       int from_end, Key* key, int* idx,
+                                                       int* ctl) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double* sk = reinterpret_cast<double*>(smem);
+  Key* sk = reinterpret_cast<Key*>(smem);
   int* si = reinterpret_cast<int*>(sk + kCap);
-  short* lp = reinterpret_cast<short*>(si + kCap);
-  short* rp = lp + kCap;
-  int* tiny = reinterpret_cast<int*>(rp + kCap);
-  __shared__ int3 stack[64];
-  const int lane = threadIdx.x;
+  int* tiny = si + kCap;
+  short* lps = reinterpret_cast<short*>(tiny + kCap);
+  short* rps = lps + kCap;
+  SortPart* parts[2];
+  parts[0] = reinterpret_cast<SortPart*>(rps + kCap);
+  parts[1] = parts[0] + kCap / kInsertion;
+  __shared__ int n_parts[2], n_tiny, bad;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   const int n = *n_segs;
   for (int s = blockIdx.x; s < n; s += gridDim.x) {
     const SortSeg g = segs[from_end > 0 ? from_end - 1 - s : s];
     const int len = g.l - g.f;
-    for (int i = lane; i < len; i += 32) {
+    for (int i = threadIdx.x; i < len; i += blockDim.x) {
       sk[i] = key[g.f + i];
       si[i] = idx[g.f + i];
     }
-    if (lane == 0) stack[0] = make_int3(0, len, g.d);
-    int sp = 1, n_tiny = 0;
-    __syncwarp();
-    while (sp > 0) {
-      const int3 t = stack[--sp];
-      __syncwarp();
-      const int f = t.x, l = t.y, d = t.z;
-      if (l - f <= kInsertion) {
-        if (l - f >= 2) {
-          if (lane == 0) tiny[n_tiny] = f | ((l - f) << 16);
-          ++n_tiny;
-        }
-        continue;
-      }
-      if (d == 0) {
-        if (lane == 0) heap_sort(sk + f, si + f, l - f);
-        __syncwarp();
-        continue;
-      }
-      if (lane == 0) median_to_first(sk, si, f, f + 1, f + (l - f) / 2, l - 1);
-      __syncwarp();
-      const double pk = sk[f];
-      int nl = 0, nr = 0;
-      for (int b = f + 1; b < l; b += 32) {
-        const int p = b + lane;
-        const bool fl = p < l && !(sk[p] < pk);
-        const unsigned m = __ballot_sync(0xffffffffu, fl);
-        if (fl) lp[nl + __popc(m & below)] = short(p);
-        nl += __popc(m);
-      }
-      for (int b = l - 1; b >= f; b -= 32) {
-        const int p = b - lane;
-        const bool fr = p >= f && !(pk < sk[p]);
-        const unsigned m = __ballot_sync(0xffffffffu, fr);
-        if (fr) rp[nr + __popc(m & below)] = short(p);
-        nr += __popc(m);
-      }
-      __syncwarp();
-      const int mk = min(nl, nr);
-      int K = 0;
-      for (int b = 0; b < mk; b += 32) {
-        const int k = b + lane;
-        const unsigned m = __ballot_sync(0xffffffffu, k < mk && lp[k] < rp[k]);
-        K += __popc(m);
-        if (m != 0xffffffffu) break;
-      }
-      for (int k = lane; k < K; k += 32) swap_pair(sk, si, lp[k], rp[k]);
-      int cut = K < nl ? int(lp[K]) : l;
-      if (K >= 1) cut = min(cut, int(rp[K - 1]));
-      __syncwarp();
-      if (cut <= f || cut >= l || sp + 2 > 64) {
-        if (lane == 0) atomicOr(ctl + kError, 2);
-        sp = 0;
-        n_tiny = 0;
-        break;
-      }
-      if (lane == 0) {
-        stack[sp] = make_int3(f, cut, d - 1);
-        stack[sp + 1] = make_int3(cut, l, d - 1);
-      }
-      sp += 2;
-      __syncwarp();
+    if (threadIdx.x == 0) {
+      parts[0][0] = SortPart{0, short(len), short(g.d), 0};
+      n_parts[0] = 1;
+      n_parts[1] = 0;
+      n_tiny = 0;
+      bad = 0;
     }
-    __syncwarp();
-    for (int j = lane; j < n_tiny; j += 32) {
+    __syncthreads();
+    // a segment's part is longer than kInsertion; a depth budget of at most
+    // 2 log2 n ends the rounds
+    for (int cur = 0; n_parts[cur] > 0; cur ^= 1) {
+      for (int q = warp; q < n_parts[cur]; q += kWarps) {
+        const SortPart t = parts[cur][q];
+        const int f = t.f, l = t.l, d = t.d;
+        if (d == 0) {
+          if (lane == 0) heap_sort(sk + f, si + f, l - f);
+          __syncwarp();
+          continue;
+        }
+        short *lp = lps + f, *rp = rps + f;  // the parts' ranges are disjoint
+        if (lane == 0) median_to_first(sk, si, f, f + 1, f + (l - f) / 2, l - 1);
+        __syncwarp();
+        const Key pk = sk[f];
+        int nl = 0, nr = 0;
+        for (int b = f + 1; b < l; b += 32) {
+          const int p = b + lane;
+          const bool fl = p < l && !(sk[p] < pk);
+          const unsigned m = __ballot_sync(0xffffffffu, fl);
+          if (fl) lp[nl + __popc(m & below)] = short(p);
+          nl += __popc(m);
+        }
+        for (int b = l - 1; b >= f; b -= 32) {
+          const int p = b - lane;
+          const bool fr = p >= f && !(pk < sk[p]);
+          const unsigned m = __ballot_sync(0xffffffffu, fr);
+          if (fr) rp[nr + __popc(m & below)] = short(p);
+          nr += __popc(m);
+        }
+        __syncwarp();
+        const int mk = min(nl, nr);
+        int K = 0;
+        for (int b = 0; b < mk; b += 32) {
+          const int k = b + lane;
+          const unsigned m = __ballot_sync(0xffffffffu, k < mk && lp[k] < rp[k]);
+          K += __popc(m);
+          if (m != 0xffffffffu) break;
+        }
+        for (int k = lane; k < K; k += 32) swap_pair(sk, si, lp[k], rp[k]);
+        int cut = K < nl ? int(lp[K]) : l;
+        if (K >= 1) cut = min(cut, int(rp[K - 1]));
+        if (lane == 0) {
+          if (cut <= f || cut >= l) {  // the sentinel argument guarantees both parts
+            bad = 1;
+          } else {
+            for (int h = 0; h < 2; ++h) {
+              const int pf = h == 0 ? f : cut, pl = h == 0 ? cut : l;
+              if (pl - pf > kInsertion)
+                parts[cur ^ 1][atomicAdd(&n_parts[cur ^ 1], 1)] =
+                    SortPart{short(pf), short(pl), short(d - 1), 0};
+              else if (pl - pf >= 2)
+                tiny[atomicAdd(&n_tiny, 1)] = pf | ((pl - pf) << 16);
+            }
+          }
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) n_parts[cur] = 0;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0 && bad) atomicOr(ctl + kError, 2);
+    for (int j = threadIdx.x; j < n_tiny; j += blockDim.x) {
       const int f = tiny[j] & 0xffff, c = tiny[j] >> 16;
       insertion_sort(sk, si, f, f + c);
     }
-    __syncwarp();
-    for (int i = lane; i < len; i += 32) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < len; i += blockDim.x) {
       key[g.f + i] = sk[i];
       idx[g.f + i] = si[i];
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
 // Insertion sort of the short segments the partition rounds left.
-__global__ void k_tiny(const SortSeg* segs, const int* n_segs, double* key, int* idx) {
+__global__ void k_tiny(const SortSeg* segs, const int* n_segs, Key* key, int* idx) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= *n_segs) return;
   insertion_sort(key, idx, segs[s].f, segs[s].l);
 }
 
 // Heap sort of the segments the partition rounds ran out of depth on.
-__global__ void k_heap(const SortSeg* segs, const int* n_segs, double* key, int* idx) {
+__global__ void k_heap(const SortSeg* segs, const int* n_segs, Key* key, int* idx) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= *n_segs) return;
   heap_sort(key + segs[s].f, idx + segs[s].f, segs[s].l - segs[s].f);
@@ -551,7 +607,7 @@ __global__ void k_heap(const SortSeg* segs, const int* n_segs, double* key, int*
 // sort) gets its box centre along the axis; every position starts as itself
 // in the permutation.
 __global__ void k_keys(const float4* lo, const float4* hi, const int* node_of,
-                       const NodeBest* best, int axis, int n, double* key, int* idx) {
+                       const NodeBest* best, int axis, int n, Key* key, int* idx) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   idx[p] = p;
@@ -559,7 +615,7 @@ __global__ void k_keys(const float4* lo, const float4* hi, const int* node_of,
   if (a < 0) return;
   const int ax = best ? best[a].axis : axis;
   if (ax < 0) return;
-  key[p] = centre(lo[p], hi[p], ax);
+  key[p] = centre_key(lo[p], hi[p], ax);
 }
 
 // The build order after a sort: records moved along the permutation.
@@ -732,10 +788,9 @@ __global__ void k_small_node_sweep(const RNode* nodes, const int* active, const 
     sa2[i] = surface_area(run.l[0], run.l[1], run.l[2], run.h[0], run.h[1], run.h[2]);
   }
   NodeBest b = best[a];
-  const double sr = sa_root[a];
+  const SplitCost split(sa_root[a]);
   for (int i = 1; i < n - 1; ++i) {
-    const double num = __dadd_rn(__dmul_rn(double(i), sa1[i]), __dmul_rn(double(n - i), sa2[i]));
-    const double cost = __dadd_rn(2.0, __ddiv_rn(__dmul_rn(num, 1.0), sr));
+    const double cost = split(i, n, sa1[i], sa2[i]);
     if (cost < b.cost) b = NodeBest{cost, axis, i};
   }
   best[a] = b;
@@ -895,7 +950,8 @@ __global__ void k_tile_sweep(const RNode* nodes, const int* active, const int2* 
     run = box_merge(run, bx[j]);
     sa1[j] = surface_area(run.l[0], run.l[1], run.l[2], run.h[0], run.h[1], run.h[2]);
   }
-  const double sr = sa_root[a], leaf = double(n);
+  const SplitCost split(sa_root[a]);
+  const double leaf = double(n);
   double bc = INFINITY;
   int bi = INT_MAX;
   run = box_merge(post[tile], after);
@@ -904,8 +960,7 @@ __global__ void k_tile_sweep(const RNode* nodes, const int* active, const int2* 
     const int i = i0 + j;
     if (i >= 1 && i <= n - 2) {
       const double sa2 = surface_area(run.l[0], run.l[1], run.l[2], run.h[0], run.h[1], run.h[2]);
-      const double num = __dadd_rn(__dmul_rn(double(i), sa1[j]), __dmul_rn(double(n - i), sa2));
-      const double cost = __dadd_rn(2.0, __ddiv_rn(__dmul_rn(num, 1.0), sr));
+      const double cost = split(i, n, sa1[j], sa2);
       if (cost < leaf && (cost < bc || (cost == bc && i < bi))) {
         bc = cost;
         bi = i;

@@ -231,5 +231,32 @@ SBR_HD float to_f32(double x) {
   return float(x);
 }
 
+// double(x) and double(n) (n in [0, 2^31)), exact; subnormal, infinite and NaN
+// floats are left to the hardware.
+SBR_HD double from_f32(float x) {
+#ifdef __CUDA_ARCH__
+  const uint32_t u = __float_as_uint(x);
+#else
+  uint32_t u;
+  std::memcpy(&u, &x, 4);
+#endif
+  const uint32_t e = (u >> 23) & 0xffu;
+  if (e - 1u < 254u)
+    return from_bits(uint64_t((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))) << 32 |
+                     uint64_t(u << 29));
+  if ((u << 1) == 0) return from_bits(uint64_t(u) << 32);
+  return double(x);
+}
+SBR_HD double from_int(int n) {
+  if (n == 0) return 0.0;
+#ifdef __CUDA_ARCH__
+  const int lead = __clz(n);
+#else
+  const int lead = __builtin_clz(unsigned(n));
+#endif
+  const uint64_t m = uint64_t(n) << (lead + 21);  // leading bit at 52
+  return from_bits((uint64_t(1023 + 30 - lead) << 52) + m);  // its carry makes the exponent
+}
+
 }  // namespace soft64
 }  // namespace sbr
