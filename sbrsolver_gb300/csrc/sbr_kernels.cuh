@@ -704,30 +704,46 @@ __device__ __forceinline__ SlabRay slab_ray(const float3& o, const float3& d, fl
   return r;
 }
 
+// Four planes of an axis take two packed FP32 operations, each product and sum
+// rounded as fmaf rounds it: the search is bound by instruction issue (79 % of
+// the issue slots; level-9 canyon 4.27 -> 4.13 ms, level-10 terrain 8.87 ->
+// 8.63).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r, x = *reinterpret_cast<unsigned long long*>(&a),
+                        y = *reinterpret_cast<unsigned long long*>(&b),
+                        z = *reinterpret_cast<unsigned long long*>(&c);
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+  return *reinterpret_cast<float2*>(&r);
+}
 // The children of a four-wide node that the ray's slab test keeps within
-// [0, tcut], nearest first; returns how many (c[0..n)).
+// [0, tcut], nearest first; returns how many (c[0..n), entered at t[0..n)).
 __device__ __forceinline__ int visit_node4(const Node4* node, const SlabRay& r, float tcut,
-                                           int c[4]) {
+                                           int c[4], float t[4]) {
   const float4* p = reinterpret_cast<const float4*>(node);
   const int sx = r.near & 1 ? 3 : 0, sy = r.near & 2 ? 3 : 0, sz = r.near & 4 ? 3 : 0;
-  const float4 nx = __ldg(p + sx), ny = __ldg(p + 1 + sy), nz = __ldg(p + 2 + sz);
-  const float4 fx = __ldg(p + 3 - sx), fy = __ldg(p + 4 - sy), fz = __ldg(p + 5 - sz);
+  const float4 bnx = __ldg(p + sx), bny = __ldg(p + 1 + sy), bnz = __ldg(p + 2 + sz);
+  const float4 bfx = __ldg(p + 3 - sx), bfy = __ldg(p + 4 - sy), bfz = __ldg(p + 5 - sz);
   const int4 cr = __ldg(reinterpret_cast<const int4*>(p + 6));
   auto visit = [&](float ax, float ay, float az, float bx, float by, float bz, int child,
                    float& t) -> int {
-    const float tn = fmaxf(fmaxf(fmaf(ax, r.inv[0], r.off_near[0]), fmaf(ay, r.inv[1], r.off_near[1])),
-                           fmaxf(fmaf(az, r.inv[2], r.off_near[2]), 0.0f));
-    const float tf = fminf(fminf(fmaf(bx, r.inv[0], r.off_far[0]), fmaf(by, r.inv[1], r.off_far[1])),
-                           fminf(fmaf(bz, r.inv[2], r.off_far[2]), tcut));
+    const float tn = fmaxf(fmaxf(ax, ay), fmaxf(az, 0.0f));
+    const float tf = fminf(fminf(bx, by), fminf(bz, tcut));
     const bool h = tn <= tf;  // an absent child's planes are at infinity the wrong way round
     t = h ? tn : INFINITY;
     return h ? child : kEmptyChild;
   };
-  float t0, t1, t2, t3;
-  c[0] = visit(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, cr.x, t0);
-  c[1] = visit(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, cr.y, t1);
-  c[2] = visit(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, cr.z, t2);
-  c[3] = visit(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, cr.w, t3);
+  auto planes = [](const float4& b, float inv, float off) {
+    const float2 i2 = make_float2(inv, inv), o2 = make_float2(off, off);
+    const float2 l = fma2(make_float2(b.x, b.y), i2, o2), h = fma2(make_float2(b.z, b.w), i2, o2);
+    return make_float4(l.x, l.y, h.x, h.y);
+  };
+  const float4 nx = planes(bnx, r.inv[0], r.off_near[0]), ny = planes(bny, r.inv[1], r.off_near[1]),
+               nz = planes(bnz, r.inv[2], r.off_near[2]), fx = planes(bfx, r.inv[0], r.off_far[0]),
+               fy = planes(bfy, r.inv[1], r.off_far[1]), fz = planes(bfz, r.inv[2], r.off_far[2]);
+  c[0] = visit(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, cr.x, t[0]);
+  c[1] = visit(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, cr.y, t[1]);
+  c[2] = visit(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, cr.z, t[2]);
+  c[3] = visit(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, cr.w, t[3]);
   auto order = [](float& ta, int& ca, float& tb, int& cb) {
     if (tb < ta) {
       const float t = ta;
@@ -738,11 +754,11 @@ __device__ __forceinline__ int visit_node4(const Node4* node, const SlabRay& r, 
       cb = x;
     }
   };
-  order(t0, c[0], t1, c[1]);  // sorting network for four
-  order(t2, c[2], t3, c[3]);
-  order(t0, c[0], t2, c[2]);
-  order(t1, c[1], t3, c[3]);
-  order(t1, c[1], t2, c[2]);
+  order(t[0], c[0], t[1], c[1]);  // sorting network for four
+  order(t[2], c[2], t[3], c[3]);
+  order(t[0], c[0], t[2], c[2]);
+  order(t[1], c[1], t[3], c[3]);
+  order(t[1], c[1], t[2], c[2]);
   return int(c[0] != kEmptyChild) + int(c[1] != kEmptyChild) + int(c[2] != kEmptyChild) +
          int(c[3] != kEmptyChild);
 }

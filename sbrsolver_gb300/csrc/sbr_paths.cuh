@@ -113,7 +113,8 @@ __device__ bool direct_blocked(const DevScene& sc, const double* o, const double
     const int ni = stack[--sp];
     if (ni >= 0) {
       int c[4];
-      const int n = visit_node4(sc.snode4 + ni, slab, tcut, c);
+      float t[4];
+      const int n = visit_node4(sc.snode4 + ni, slab, tcut, c, t);
       if (sp + n > kStack) {  // a deep stack: the one-pass search
         const Hit h = closest_call(sc, o[0], o[1], o[2], d[0], d[1], d[2], ctr);
         return h.rank != INT_MAX && !(x64::norm(d) < h.dist);

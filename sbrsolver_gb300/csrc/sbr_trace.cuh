@@ -385,8 +385,8 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
   float3 o32 = make_float3(0, 0, 0), d32 = o32;
   SlabRay slab = {};
   float no = 0.0f, nd = 0.0f, tcut = INFINITY;
-  int stack[kStack];
-  int sp = 0, pending = -1, nc = 0, orank = -1;
+  int2 stack[kStack];  // child ref, entry distance (bits)
+  int sp = 0, cur = 0, nc = 0, orank = -1;
   bool fail = false, safe = false;
   uint2* out = nullptr;
   while (true) {
@@ -434,10 +434,9 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
         slab = slab_ray(o32, d32, A.sc.box_margin + kBoxK * no);
         tcut = INFINITY;
         sp = 0;
-        pending = -1;
+        cur = 0;  // the search root is always a node
         nc = 0;
         fail = false;
-        stack[sp++] = 0;  // the search root is always a node
         out = A.cand + size_t(k) * kCand;
       }
       __syncwarp();
@@ -447,20 +446,20 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
     bool done = false;
     for (int it = 0; it < A.steps && !done; ++it) {
       // A step is either a node visit or leaf tests, for all lanes: leaves are
-      // tested when a third of the lanes hold one, and every fourth step.
-      // Taking both kinds in each step ran the triangle test with 11 lanes,
-      // the node visit with 21 (level-9 canyon search 4.55 ms, now 4.28;
-      // level-10 terrain 9.3, now 8.8; half of the lanes or every second
-      // step: 4.28 and 9.1).
+      // tested when half of the lanes hold one, and every fourth step.  Taking
+      // both kinds in each step ran the triangle test with 11 lanes, the node
+      // visit with 21: level-9 canyon search 4.55 ms against 3.80, level-10
+      // terrain 9.3 against 8.0 (a third of the lanes: 3.86 and 8.1; every
+      // eighth step: 3.93 and 7.9).
       const unsigned active = __activemask();
-      const unsigned leaves = __ballot_sync(active, pending >= 0);
-      const bool leaf_step = leaves && (3 * __popc(leaves) >= __popc(active) || (it & 3) == 3);
-      if (leaf_step != (pending >= 0)) continue;
+      const unsigned leaves = __ballot_sync(active, cur < 0);
+      const bool leaf_step = leaves && (2 * __popc(leaves) >= __popc(active) || (it & 3) == 3);
+      if (leaf_step != (cur < 0)) continue;
       if (leaf_step) {
-        // up to tris_per_step triangles of the pending leaf per step
-        for (int q = 0; q < A.tris_per_step && pending >= 0; ++q) {
-          const int j = pending >> 3, left = (pending & 7) - 1;
-          pending = left > 0 ? ((j + 1) << 3 | left) : -1;
+        // up to tris_per_step triangles of the leaf per step
+        for (int q = 0; q < A.tris_per_step && cur != kEmptyChild; ++q) {
+          const int j = ~cur >> 3, left = (~cur & 7) - 1;
+          cur = left > 0 ? ~((j + 1) << 3 | left) : kEmptyChild;
           float tlo, thi;
           const Tri32 T = A.sc.stri[j];
           const int k = tri_classify(T, o32, d32, no, nd, tlo, thi);
@@ -478,32 +477,34 @@ __global__ void __launch_bounds__(128, 8) k_find(FindArgs A) {
                                  __float_as_uint(tlo));
           if (k & kSureHit) tcut = fminf(tcut, thi * (1.0f + kTieSlack) + 1e-30f);
         }
-        continue;
+      } else {
+        // a four-wide node: the children the ray's slab test keeps (within
+        // tcut), nearest first; it goes on with the nearest, the farther ones
+        // go on the stack
+        int c[4];
+        float t[4];
+        const int need = visit_node4(A.sc.snode4 + cur, slab, tcut, c, t);
+        if (sp + need > kStack) {
+          fail = done = true;
+          break;
+        }
+        if (need > 3) stack[sp++] = make_int2(c[3], __float_as_int(t[3]));
+        if (need > 2) stack[sp++] = make_int2(c[2], __float_as_int(t[2]));
+        if (need > 1) stack[sp++] = make_int2(c[1], __float_as_int(t[1]));
+        cur = c[0];
       }
-      if (sp == 0) {
-        done = true;
-        break;
-      }
-      const int ni = stack[--sp];
-      if (ni < 0) {  // a leaf deferred as the farther child
-        pending = ~ni;
-        continue;
-      }
-      // a four-wide node: the children the ray's slab test keeps (within
-      // tcut), nearest first; the farther ones go on the stack, the nearest
-      // on top (a leaf as the nearest becomes the pending leaf at once)
-      int c[4];
-      const int need = visit_node4(A.sc.snode4 + ni, slab, tcut, c);
-      if (sp + need > kStack) {
-        fail = done = true;
-        break;
-      }
-      if (need > 3) stack[sp++] = c[3];  // node, or ~leaf code
-      if (need > 2) stack[sp++] = c[2];
-      if (need > 1) stack[sp++] = c[1];
-      if (need > 0) {
-        if (c[0] < 0) pending = ~c[0];
-        else stack[sp++] = c[0];
+      // The next child off the stack that a hit found since has not cut off,
+      // taken in this step: a lane starts each step with a node or a leaf in
+      // hand.  A cut-off child cost a node visit before, a postponed leaf a
+      // step of its own (level-9 canyon search 4.13 ms, now 3.96; level-10
+      // terrain 8.6, now 8.35).
+      while (cur == kEmptyChild) {
+        if (sp == 0) {
+          done = true;
+          break;
+        }
+        const int2 e = stack[--sp];
+        if (__int_as_float(e.y) <= tcut) cur = e.x;
       }
     }
     if (done) {
