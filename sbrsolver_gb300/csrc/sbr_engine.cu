@@ -183,6 +183,7 @@ struct Workspace {
   DBuf<unsigned char> direct_ok;
   DBuf<Survivor> surv;
   DBuf<int> s_counts, s_starts, s_cursor, s_order;
+  DBuf<unsigned> ray_offset;
   DBuf<double> path_field, path_pts, field;
   DBuf<SegTerms> seg;                  // field terms per path segment
   DBuf<uint32_t> seg_list, int_list;   // k_seg's tasks
@@ -753,12 +754,12 @@ static void swap_buf(DBuf<T>& a, DBuf<T>& b) {
 // launches over many blocks (sums: a tile total each); returns the launches.
 // (One block over the level-10 terrain's 400,000 cells took 361 us, the three
 // launches 14; at 4,096 items one block takes 4 us and the three 9.)
-static int scan_ints(const int* in, int* out, int n, int* sums, cudaStream_t st) {
+static int scan_ints(const int* in, int* out, long long n, int* sums, cudaStream_t st) {
   if (n <= kScanOne) {
-    k_scan_exclusive<<<1, 1024, 0, st>>>(in, out, n);
+    k_scan_exclusive<<<1, 1024, 0, st>>>(in, out, int(n));
     return 1;
   }
-  const int nb = (n + kScanTile - 1) / kScanTile;
+  const int nb = int((n + kScanTile - 1) / kScanTile);
   k_tile_sums<<<nb, kScanThreads, 0, st>>>(in, n, sums);
   k_sums_scan<<<1, 1024, 0, st>>>(sums, nb, out + n);
   k_tile_scan<<<nb, kScanThreads, 0, st>>>(in, n, sums, out);
@@ -1284,7 +1285,7 @@ static std::string pipeline_key(const SceneImpl& S, const Workspace& W, const sb
                         W.nodes.p, W.nodes_cold.p, W.cls_keys.p, W.cop_keys.p, W.dd_keys.p,
                         W.dd_rank.p, W.cc_keys.p, W.cls_list.p, W.cc_val.p, W.cls_info.p,
                         W.cls_cap.p, W.corr_list.p, W.pairs.p, W.direct_ok.p, W.surv.p,
-                        W.s_counts.p, W.s_starts.p, W.s_cursor.p, W.s_order.p, W.path_field.p,
+                        W.s_counts.p, W.s_starts.p, W.s_cursor.p, W.s_order.p, W.ray_offset.p, W.path_field.p,
                         W.path_pts.p, W.field.p, W.seg.p, W.seg_list.p, W.int_list.p, W.path_mat.p, W.path_field64.p,
                         W.field64.p, W.path_nray.p, W.path_tri.p, W.path_cop.p, W.path_kind.p,
                         W.path_near.p, W.ctr.p, W.seg_tx.p, W.cand.p, W.ncand.p, W.find_work.p,
@@ -1500,8 +1501,14 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     // Tables from the occupancy ratios learned so far (hash tables half
     // full), each limited to 2% of free device memory: past that the solve
     // grows the table on overflow instead.
+    // The free memory is asked for only when one grows (6 us of each solve).
+    const bool grows = 2.2 * W.r_cls * nodes > W.cap_cls || 2.2 * W.r_cop * nodes > W.cap_cop ||
+                       2.2 * W.r_dd * nodes > W.cap_dd || 2.2 * W.r_cc * nodes > W.cap_cc ||
+                       1.2 * W.r_corr * nodes > double(W.cap_corr) ||
+                       1.2 * W.r_surv * nodes > double(W.cap_surv) ||
+                       1.3 * W.r_pairs * nodes > double(W.cap_pairs);
     size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
+    if (grows) CK(cudaMemGetInfo(&free_b, &total_b));
     const double cap_bytes = 0.02 * double(free_b);
     auto pow2 = [](double x, double entry_bytes, double limit) {
       x = std::min(x, limit / entry_bytes);
@@ -1551,7 +1558,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       g->base.ensure(n_req + 1);
       g->counts.ensure(2 * cell_cap);
       g->starts.ensure(cell_cap + 1);
-      g->sums.ensure(std::max(cell_cap, size_t(rx_total)) / kScanTile + 1);
+      g->sums.ensure(std::max(cell_cap, 2 * size_t(rx_total)) / kScanTile + 1);
       g->rx32.ensure(std::max(1, rx_total));
     }
     W.rx_bad.ensure(1);
@@ -1591,8 +1598,9 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       W.int_list.ensure(nsa * kMaxDepth);
       W.path_mat.ensure(nsa * (kMaxDepth + 1));
       W.field.ensure(std::max(1, 6 * rx_total));
-      W.s_counts.ensure(rx_total + 1);
-      W.s_starts.ensure(rx_total + 2);
+      W.s_counts.ensure(2 * size_t(rx_total) + 1);  // paths, then rays, per receiver
+      W.s_starts.ensure(2 * size_t(rx_total) + 2);
+      W.ray_offset.ensure(nsa);
       W.s_cursor.ensure(rx_total + 1);
       W.s_order.ensure(nsa);
       W.path_bound.ensure(nsa);
@@ -1604,6 +1612,38 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
         W.field64.ensure(std::max(1, 6 * rx_total));
       }
     }
+    // ---- the result, written by the device into the workspace's pinned staging
+    ResultArgs ra;
+    ra.order = W.s_order.p;
+    ra.ray_offset = W.ray_offset.p;
+    ra.ray_starts = W.s_starts.p + rx_total;
+    ra.seg_tx = W.seg_tx.p;
+    ra.field = W.field.p;
+    ra.bound = W.field_bound.p;
+    ra.field64 = field_check ? W.field64.p : nullptr;
+    ra.rx_bad = W.rx_bad.p;
+    ra.n_req = n_req;
+    ra.rx_total = rx_total;
+    size_t fixed = 0;
+    auto at = [&fixed](size_t bytes) {
+      const size_t o = fixed;
+      fixed += (bytes + 15) & ~size_t(15);
+      return o;
+    };
+    at(sizeof(ResultHead));
+    ra.at.seg = at(sizeof(unsigned long long) * n_req);
+    const size_t b_field = sizeof(double) * 6 * size_t(rx_total);
+    ra.at.field = at(b_field);
+    ra.at.bound = at(sizeof(double) * size_t(rx_total));
+    ra.at.field64 = at(field_check ? b_field : 0);
+    ra.at.paths = fixed;
+    // (nothing may be in flight while staging is replaced: it fits or is grown here,
+    // or below after a synchronisation)
+    auto staging = [&](size_t bytes) {
+      if (bytes > W.h_res.n)  // pinning is slow
+        W.h_res.ensure(bytes + bytes / 4 + (size_t(64) << 10));
+    };
+    staging(fixed);
     (void)resolved(tu);  // the occupancy queries run before any recording
     // ---- the device pipeline: a fixed sequence of stream operations
     const long long nl_before = nl;
@@ -1619,6 +1659,34 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       else
         CK(cudaEventRecord(e, st));
     };
+    FieldArgs fa;  // of the field stage and the result
+    fa.sc = S.dev;
+    fa.txp = d_txp;
+    fa.rx = d_rx;
+    fa.rx_req = d_req;
+    fa.cls_info = W.cls_info.p;
+    fa.rank_to_id = S.rank_to_id.p;
+    fa.surv = W.surv.p;
+    fa.ctr = W.ctr.p;
+    fa.cap = W.cap_surv;
+    fa.K = K;
+    fa.precision = -1;
+    fa.path_field = W.path_field.p;
+    fa.path_nray = W.path_nray.p;
+    fa.path_tri = W.path_tri.p;
+    fa.path_cop = W.path_cop.p;
+    fa.path_kind = W.path_kind.p;
+    fa.path_near_edge = W.path_near.p;
+    fa.path_pts = W.path_pts.p;
+    fa.seg = W.seg.p;
+    fa.path_mat = W.path_mat.p;
+    fa.seg_list = W.seg_list.p;
+    fa.int_list = W.int_list.p;
+    fa.path_bound = W.path_bound.p;
+    fa.rx_flag = W.rx_flag.p;
+    fa.fstat = W.fstat.p;
+    bool any_fp32 = false;  // a request in the FP32 field mode (error bounds, escalation)
+    for (int r = 0; r < n_req; ++r) any_fp32 |= tp[r].precision == 1;
     auto record = [&]() {
   mark(W.ev[0]);
   CK(cudaMemcpyAsync(W.up.p, W.h_up.p, host_rx ? up_bytes : up_rx, cudaMemcpyHostToDevice, st));
@@ -1649,7 +1717,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     fill(W.cc_val.p, W.cap_cc, 0);
     fill(W.rx_flag.p, sizeof(int) * std::max(1, rx_total), 0);
     fill(W.fstat.p, 2 * sizeof(unsigned long long), 0);
-    fill(W.s_counts.p, sizeof(int) * (rx_total + 1), 0);
+    fill(W.s_counts.p, sizeof(int) * (2 * size_t(rx_total) + 1), 0);
     fill(W.s_cursor.p, sizeof(int) * (rx_total + 1), 0);
     size_t fill_bytes = 0;
     for (int k = 0; k < fl.n; ++k) fill_bytes = std::max<size_t>(fill_bytes, fl.r[k].bytes);
@@ -1796,46 +1864,21 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     // (the kernels take the count from the device), so the whole solve runs
     // without a host round trip until its results are read
     const unsigned long long ns_cap = W.cap_surv;
-    FieldArgs fa;
-    fa.sc = S.dev;
-    fa.txp = d_txp;
-    fa.rx = d_rx;
-    fa.rx_req = d_req;
-    fa.cls_info = W.cls_info.p;
-    fa.rank_to_id = S.rank_to_id.p;
-    fa.surv = W.surv.p;
-    fa.ctr = W.ctr.p;
-    fa.cap = W.cap_surv;
-    fa.K = K;
-    fa.precision = -1;
-    fa.path_field = W.path_field.p;
-    fa.path_nray = W.path_nray.p;
-    fa.path_tri = W.path_tri.p;
-    fa.path_cop = W.path_cop.p;
-    fa.path_kind = W.path_kind.p;
-    fa.path_near_edge = W.path_near.p;
-    fa.path_pts = W.path_pts.p;
-    fa.seg = W.seg.p;
-    fa.path_mat = W.path_mat.p;
-    fa.seg_list = W.seg_list.p;
-    fa.int_list = W.int_list.p;
-    bool any_fp32 = false;  // a request in the FP32 field mode (error bounds, escalation)
-    for (int r = 0; r < n_req; ++r) any_fp32 |= tp[r].precision == 1;
-    fa.path_bound = W.path_bound.p;
-    fa.rx_flag = W.rx_flag.p;
-    fa.fstat = W.fstat.p;
     ++nl, k_path<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
     ++nl, k_seg<<<grid_for(ns_cap * (kMaxDepth + 1), 64), 64, 0, st>>>(fa);
     ++nl, k_combine<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
     if (any_fp32) ++nl, k_escalate<<<grid_for(ns_cap * 32, 64), 64, 0, st>>>(fa, false);
-    ++nl, k_surv_hist<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv, W.s_counts.p);
-    nl += scan_ints(W.s_counts.p, W.s_starts.p, rx_total, W.all.sums.p, st);
+    ++nl, k_surv_hist<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv,
+                                                       W.path_nray.p, W.s_counts.p,
+                                                       W.s_counts.p + rx_total);
+    nl += scan_ints(W.s_counts.p, W.s_starts.p, 2LL * rx_total, W.all.sums.p, st);
     ++nl, k_surv_scatter<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv,
                                                           W.s_starts.p, W.s_cursor.p, W.s_order.p);
     if (rx_total)
       ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(
           W.surv.p, W.s_starts.p, W.s_order.p, rx_total, W.path_field.p, -1, d_req, d_txp,
-          W.field.p, W.path_bound.p, W.field_bound.p, W.rx_flag.p, W.fstat.p);
+          W.field.p, W.path_bound.p, W.field_bound.p, W.rx_flag.p, W.fstat.p, nullptr,
+          W.path_nray.p, W.s_starts.p + rx_total, W.ray_offset.p);
     if (any_fp32 && rx_total) {  // receivers the FP32 bound could not certify, in FP64
       ++nl, k_escalate<<<grid_for(ns_cap * 32, 64), 64, 0, st>>>(fa, true);
       ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(
@@ -1869,12 +1912,22 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     W.pipeline_kernels = nl - nl_before;
     n_tr = n_launch_pairs;
     const int graph_run = how == kEager ? 0 : 1;
-    Counters c;
-    int rx_bad = 0;
-    CK(cudaMemcpyAsync(&c, W.ctr.p, sizeof c, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&rx_bad, W.rx_bad.p, sizeof rx_bad, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (rx_bad) throw std::string("receiver coordinates must be finite");
+    ra.f = fa;
+    for (;;) {
+      ra.out = W.h_res.p;
+      ra.room = W.h_res.n;
+      ++nl, k_result<<<device_sms() * 2, 256, 0, st>>>(ra);
+      CK(cudaGetLastError());
+      CK(cudaEventRecord(W.ev[7], st));
+      CK(cudaStreamSynchronize(st));
+      const ResultHead h = *reinterpret_cast<const ResultHead*>(W.h_res.p);
+      if (h.fits || h.c.overflow) break;
+      staging(ra.at.end(h.c.survivors, size_t(h.rays)));
+    }
+    const unsigned char* const hr = W.h_res.p;
+    const ResultHead& head = *reinterpret_cast<const ResultHead*>(hr);
+    const Counters& c = head.c;
+    if (head.rx_bad) throw std::string("receiver coordinates must be finite");
     if (c.overflow & kOvStack) throw std::string("BVH deeper than the traversal stack");
     // keep every hash table at most half full for the next solve
     auto grow = [](uint32_t& cap, unsigned long long used) {
@@ -1920,105 +1973,25 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       upd(W.r_pairs, c.pairs / n);
     }
     const unsigned long long ns = c.survivors;
-    // ---- results to the host, through the workspace's pinned staging (every
-    // array copied by DMA into one area, one synchronisation)
-    size_t need = 0;
-    auto at = [&need](size_t bytes) {
-      const size_t o = need;
-      need += (bytes + 15) & ~size_t(15);
-      return o;
+    const size_t n_rays = size_t(head.rays);
+    auto take = [hr](auto& v, size_t o, size_t n) {
+      using T = typename std::remove_reference_t<decltype(v)>::value_type;
+      const T* p = reinterpret_cast<const T*>(hr + o);
+      v.assign(p, p + n);
     };
-    const size_t nrs = size_t(ns) * (kMaxDepth + 1), nps = size_t(ns) * (kMaxDepth + 2) * 3;
-    const size_t b_field = sizeof(double) * 6 * size_t(rx_total);
-    const size_t o_field = at(b_field), o_fb = at(sizeof(double) * size_t(rx_total));
-    const size_t o_fst = at(2 * sizeof(unsigned long long));
-    const size_t o_f64 = at(field_check ? b_field : 0);
-    const size_t o_order = at(sizeof(int) * ns), o_nray = at(sizeof(int) * ns);
-    const size_t o_near = at(sizeof(int) * ns), o_sv = at(sizeof(Survivor) * ns);
-    const size_t o_pf = at(sizeof(double) * 6 * ns);
-    const size_t o_tri = at(sizeof(int) * nrs), o_cop = at(sizeof(int) * nrs);
-    const size_t o_kind = at(sizeof(int) * nrs), o_pts = at(sizeof(double) * nps);
-    if (need > W.h_res.n) W.h_res.ensure(need + need / 4 + (size_t(64) << 10));  // pinning is slow
-    unsigned char* hr = W.h_res.p;
-    auto get = [&](size_t o, const void* src, size_t bytes) {
-      if (bytes) CK(cudaMemcpyAsync(hr + o, src, bytes, cudaMemcpyDeviceToHost, st));
-    };
-    get(o_field, W.field.p, b_field);
-    get(o_fb, W.field_bound.p, sizeof(double) * size_t(rx_total));
-    get(o_fst, W.fstat.p, 2 * sizeof(unsigned long long));
-    if (field_check) get(o_f64, W.field64.p, b_field);
-    if (ns) {
-      get(o_order, W.s_order.p, sizeof(int) * ns);
-      get(o_nray, W.path_nray.p, sizeof(int) * ns);
-      get(o_near, W.path_near.p, sizeof(int) * ns);
-      get(o_sv, W.surv.p, sizeof(Survivor) * ns);
-      get(o_pf, W.path_field.p, sizeof(double) * 6 * ns);
-      get(o_tri, W.path_tri.p, sizeof(int) * nrs);
-      get(o_cop, W.path_cop.p, sizeof(int) * nrs);
-      get(o_kind, W.path_kind.p, sizeof(int) * nrs);
-      get(o_pts, W.path_pts.p, sizeof(double) * nps);
-    }
-    CK(cudaEventRecord(W.ev[7], st));
-    CK(cudaStreamSynchronize(st));
-    const double* hfield = reinterpret_cast<const double*>(hr + o_field);
-    out.field.assign(hfield, hfield + 6 * size_t(rx_total));
-    const double* hfb = reinterpret_cast<const double*>(hr + o_fb);
-    out.field_bound.assign(hfb, hfb + size_t(rx_total));
-    unsigned long long fst[2];
-    std::memcpy(fst, hr + o_fst, sizeof fst);
-    out.field64.clear();
-    if (field_check) {
-      const double* h64 = reinterpret_cast<const double*>(hr + o_f64);
-      out.field64.assign(h64, h64 + 6 * size_t(rx_total));
-    }
-    const int* order = reinterpret_cast<const int*>(hr + o_order);
-    const int* nray = reinterpret_cast<const int*>(hr + o_nray);
-    const int* pnear = reinterpret_cast<const int*>(hr + o_near);
-    const Survivor* sv = reinterpret_cast<const Survivor*>(hr + o_sv);
-    const double* pf = reinterpret_cast<const double*>(hr + o_pf);
-    const int* ptri = reinterpret_cast<const int*>(hr + o_tri);
-    const int* pcop = reinterpret_cast<const int*>(hr + o_cop);
-    const int* pkind = reinterpret_cast<const int*>(hr + o_kind);
-    const double* pts = reinterpret_cast<const double*>(hr + o_pts);
-    // assemble paths in receiver order, then (launch, BFS) order
-    std::vector<int> req_of(rx_total);
-    for (int r = 0; r < n_req; ++r)
-      for (int i = 0; i < tp[r].n_rx; ++i) req_of[tp[r].rx_first + i] = r;
-    out.paths.clear();
-    out.tri.clear();
-    out.cop.clear();
-    out.kind.clear();
-    out.points.clear();
-    for (size_t k = 0; k < ns; ++k) {
-      const int i = order[k];
-      sbr_path p;
-      p.receiver = int(sv[i].rx) - tp[req_of[sv[i].rx]].rx_first;
-      p.request = req_of[sv[i].rx];
-      p.n_rays = nray[i];
-      p.launch = (long long)(sv[i].rank >> kHeapBits);
-      p.heap = int(sv[i].rank & ((1u << kHeapBits) - 1));
-      p.ray_offset = (long long)out.tri.size();
-      for (int j = 0; j < 6; ++j) p.field[j] = pf[6 * size_t(i) + j];
-      p.near_edge = pnear[i];
-      p.reserved = 0;
-      for (int r = 0; r < p.n_rays; ++r) {
-        const size_t b = size_t(i) * (kMaxDepth + 1) + r;
-        out.tri.push_back(ptri[b]);
-        out.cop.push_back(pcop[b]);
-        out.kind.push_back(pkind[b]);
-        const size_t q = size_t(i) * (kMaxDepth + 2) * 3 + 3 * r;
-        for (int a = 0; a < 6; ++a) out.points.push_back(pts[q + a]);
-      }
-      out.paths.push_back(p);
-    }
-    // paths are ordered by survivor order within a receiver; receivers ascend
-    // because s_order is grouped by receiver index.
+    take(out.field, ra.at.field, 6 * size_t(rx_total));
+    take(out.field_bound, ra.at.bound, size_t(rx_total));
+    take(out.field64, ra.at.field64, field_check ? 6 * size_t(rx_total) : 0);
+    // paths in receiver order, then (launch, BFS) order
+    take(out.paths, ra.at.paths, ns);
+    take(out.points, ra.at.points(ns), 6 * n_rays);
+    take(out.tri, ra.at.tri(ns, n_rays), n_rays);
+    take(out.cop, ra.at.tri(ns, n_rays) + n_rays * sizeof(int), n_rays);
+    take(out.kind, ra.at.tri(ns, n_rays) + 2 * n_rays * sizeof(int), n_rays);
     out.counts.segments = (long long)c.nodes;
     {
-      std::vector<unsigned long long> spt(n_req);
-      CK(cudaMemcpy(spt.data(), W.seg_tx.p, sizeof(unsigned long long) * n_req,
-                    cudaMemcpyDeviceToHost));
-      out.segments_per_request.assign(spt.begin(), spt.end());
+      const unsigned long long* spt = reinterpret_cast<const unsigned long long*>(hr + ra.at.seg);
+      out.segments_per_request.assign(spt, spt + n_req);
       out.rx_per_request.resize(n_req);
       out.launches_per_request.resize(n_req);
       for (int r = 0; r < n_req; ++r) {
@@ -2043,8 +2016,8 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     for (const sbr_path& p : out.paths) out.counts.near_edge_paths += p.near_edge;
     out.counts.gpu_kernels = nl;
     out.counts.pipeline_graph = graph_run;
-    out.counts.fp64_field_paths = (long long)fst[0];
-    out.counts.fp64_field_receivers = (long long)fst[1];
+    out.counts.fp64_field_paths = (long long)head.fstat[0];
+    out.counts.fp64_field_receivers = (long long)head.fstat[1];
     float ms[8] = {};
     for (int i = 1; i < 8; ++i) CK(cudaEventElapsedTime(&ms[i], W.ev[i - 1], W.ev[i]));
     out.timing.h2d_ms = ms[1];
@@ -2544,11 +2517,16 @@ sbr_status sbr_solve_batch(sbr_scene* scene, const sbr_request* requests, int n_
       }
     } give_back{pool, dev, W};
     // Split the batch into device passes whose estimated footprint (node
-    // records, queues, receivers) fits in 60% of the free device memory.
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    const double budget = std::max(2e9, 0.45 * double(free_b));
+    // records, queues, receivers) fits in 45% of the free device memory, at
+    // least 2 GB (a batch below that needs no asking, which took 24 us a solve).
     auto est = [](const sbr_request& q) { return request_bytes(q); };
+    double all_bytes = 0, budget = 2e9;
+    for (int r = 0; r < n_requests; ++r) all_bytes += est(requests[r]);
+    if (n_requests > 1 && !(all_bytes <= budget)) {
+      size_t free_b = 0, total_b = 0;
+      CK(cudaMemGetInfo(&free_b, &total_b));
+      budget = std::max(budget, 0.45 * double(free_b));
+    }
     bool batch_check = false;  // every pass carries the FP64 shadow if any request wants it
     for (int r = 0; r < n_requests; ++r)
       batch_check |= requests[r].field_check && requests[r].field_precision != SBR_FIELD_FP64;

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(const int* in, int* out
 // consecutive items.
 constexpr int kScanThreads = 512, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
 
-__global__ void __launch_bounds__(kScanThreads) k_tile_sums(const int* in, int n, int* sums) {
+__global__ void __launch_bounds__(kScanThreads) k_tile_sums(const int* in, long long n, int* sums) {
   __shared__ int sh[32];
   const long long base = (long long)blockIdx.x * kScanTile;
   int s = 0;
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(1024) k_sums_scan(int* sums, int nb, int* tota
   if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_tile_scan(const int* in, int n, const int* sums,
+__global__ void __launch_bounds__(kScanThreads) k_tile_scan(const int* in, long long n, const int* sums,
                                                             int* out) {
   __shared__ int sh[32];
   const long long base = (long long)blockIdx.x * kScanTile + threadIdx.x * kScanItems;
