@@ -47,6 +47,7 @@
 #include "sbr_trace.cuh"
 #include "sbr_capture.cuh"
 #include "sbr_paths.cuh"
+#include "sbr_dirs.cuh"
 #include "sbr_prep.cuh"
 #include "sbr_refbvh.cuh"
 
@@ -582,6 +583,29 @@ static void upload_mesh_order(SceneImpl& S, const std::vector<int>& order) {
   CK(cudaStreamSynchronize(S.stream));
 }
 
+static int device_sms();
+static long long n_launch_of(int level);
+
+// The launch directions of a level into b, on the device.  False if there is no
+// room for the scratch: the host's
+// subdivision needs none.
+static bool device_dirs(int level, double* v) {
+  DBuf<int> scratch;
+  try {
+    scratch.ensure(dirs::scratch_ints(level));
+  } catch (const CudaError& e) {
+    if (e.e != cudaErrorMemoryAllocation) throw;
+    return false;
+  }
+  std::vector<double> v0;
+  std::vector<int> from, mate;
+  icosahedron(v0, from, mate);
+  dirs::subdivide(level, v0.data(), from.data(), mate.data(), v, scratch.p, device_sms(), 0);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(0));
+  return true;
+}
+
 static void ensure_dirs(SceneImpl& S, int level) {
   if (level < 0 || level > 12) throw std::string("tessellation level must be 0..12");
   std::lock_guard<std::mutex> lock(S.dirs_mu);
@@ -591,11 +615,15 @@ static void ensure_dirs(SceneImpl& S, int level) {
     CK(cudaMemset(S.dir_table.p, 0, 13 * sizeof(const double*)));
   }
   if (!S.dirs[level]) {
-    std::vector<double> d;
-    icosphere(level, d);
     auto b = std::make_unique<DBuf<double>>();
-    b->ensure(d.size());
-    CK(cudaMemcpy(b->p, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice));
+    b->ensure(3 * size_t(n_launch_of(level)));
+    // (the first solve at level 3 takes 0.260 ms with the host's subdivision,
+    // 0.273 with the device's; at level 4 0.423 and 0.298)
+    if (level < 4 || !device_dirs(level, b->p)) {
+      std::vector<double> d;
+      icosphere(level, d);
+      CK(cudaMemcpy(b->p, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice));
+    }
     const double* ptr = b->p;
     CK(cudaMemcpy(S.dir_table.p + level, &ptr, sizeof ptr, cudaMemcpyHostToDevice));
     S.dirs[level] = std::move(b);
@@ -750,21 +778,6 @@ static void swap_buf(DBuf<T>& a, DBuf<T>& b) {
 
 // Exclusive scan of in[0, n) into out[0, n], out[n] = total, over many
 // blocks; sums: scratch of at least n / kScanTile + 1 ints.
-// Exclusive scan of a solve's counts: one block up to kScanOne items, else three
-// launches over many blocks (sums: a tile total each); returns the launches.
-// (One block over the level-10 terrain's 400,000 cells took 361 us, the three
-// launches 14; at 4,096 items one block takes 4 us and the three 9.)
-static int scan_ints(const int* in, int* out, long long n, int* sums, cudaStream_t st) {
-  if (n <= kScanOne) {
-    k_scan_exclusive<<<1, 1024, 0, st>>>(in, out, int(n));
-    return 1;
-  }
-  const int nb = int((n + kScanTile - 1) / kScanTile);
-  k_tile_sums<<<nb, kScanThreads, 0, st>>>(in, n, sums);
-  k_sums_scan<<<1, 1024, 0, st>>>(sums, nb, out + n);
-  k_tile_scan<<<nb, kScanThreads, 0, st>>>(in, n, sums, out);
-  return 3;
-}
 static void scan_exclusive(const int* in, int* out, int n, int* sums, cudaStream_t st) {
   const int nb = std::max(1, (n + kScanTile - 1) / kScanTile);
   k_tile_sums<<<nb, kScanThreads, 0, st>>>(in, n, sums);

@@ -750,13 +750,24 @@ void build_search_bvh(HostScene& H) {
   for (int& o : H.search.order) o = rank_of[size_t(o)];
 }
 
-void icosphere(int level, std::vector<double>& dirs) {
+void icosahedron(std::vector<double>& v, std::vector<int>& from, std::vector<int>& mate) {
   const double X = .525731112119133606, Z = .850650808352039932, N = 0.0;
-  std::vector<double> v = {-X, N, Z, X, N, Z,  -X, N, -Z, X, N, -Z, N, Z, X,  N, Z, -X,
+  v = {-X, N, Z, X, N, Z,  -X, N, -Z, X, N, -Z, N, Z, X,  N, Z, -X,
                            N,  -Z, X, N, -Z, -X, Z,  X, N, -Z, X,  N, Z, -X, N, -Z, -X, N};
-  std::vector<int> f = {0, 4, 1,  0, 9, 4,  9, 5, 4,  4, 5, 8,  4, 8, 1,  8, 10, 1, 8, 3, 10,
+  from = {0, 4, 1,  0, 9, 4,  9, 5, 4,  4, 5, 8,  4, 8, 1,  8, 10, 1, 8, 3, 10,
                         5, 3, 8,  5, 2, 3,  2, 7, 3,  7, 10, 3, 7, 6, 10, 7, 11, 6, 11, 0, 6,
                         0, 1, 6,  6, 1, 10, 9, 0, 11, 9, 11, 2, 9, 2, 5,  7, 2, 11};
+  mate.resize(from.size());
+  auto to = [&from](int h) { return from[size_t(h % 3 == 2 ? h - 2 : h + 1)]; };
+  for (int h = 0; h < int(from.size()); ++h)
+    for (int o = 0; o < int(from.size()); ++o)
+      if (from[size_t(o)] == to(h) && to(o) == from[size_t(h)]) mate[size_t(h)] = o;
+}
+
+void icosphere(int level, std::vector<double>& dirs) {
+  std::vector<double> v;
+  std::vector<int> f, mate;
+  icosahedron(v, f, mate);
   for (int l = 0; l < level; ++l) {
     std::unordered_map<uint64_t, int> lookup;
     lookup.reserve(f.size());

@@ -79,6 +79,9 @@ void map_search_order(HostScene& H);
 // Builds H.search from the triangles in depth-first rank order.
 void build_search_bvh(HostScene& H);
 
+// The icosahedron's vertices, and its faces as half-edges: start vertices and,
+// for each, the half-edge of the face across it.
+void icosahedron(std::vector<double>& v, std::vector<int>& from, std::vector<int>& mate);
 // Icosahedron launch directions at a subdivision level, in the reference's
 // vertex order (Icosahedron.cpp:3-109), 3 doubles per direction.
 void icosphere(int level, std::vector<double>& dirs);
