@@ -812,8 +812,8 @@ static void sort_perm_by(DBuf<int>& perm, DBuf<int>& tmp, DBuf<int>& flags, DBuf
 // copy of the vertices (9 floats per triangle).
 struct RefSort {
   DBuf<refbvh::Key> key;
-  DBuf<int> idx, lpos, rpos, tile_seg, cnt_l, cnt_r, off_l, off_r;
-  DBuf<int2> totals;
+  DBuf<int> idx, lpos, rpos, tile_seg;
+  DBuf<int2> totals, cnt;
   DBuf<refbvh::SortSeg> big, big_next, small, tiny, heap;
   DBuf<int> ctl;
   int sms = 1;
@@ -841,32 +841,31 @@ static void ref_sort(RefSort& R, const refbvh::RNode* nodes, const int* active, 
                                                  R.small_cap, R.tiny.p, R.heap.p, R.ctl.p);
   CK(cudaGetLastError());
   read_ctl(R, h, st);
-  int n_big = h[kBig], n_tiles = h[kTiles];
-  for (int round = 0; n_big > 0; ++round) {
-    if (round > 64) throw std::string("device reference BVH: too many partition rounds");
-    k_tile_map<<<n_big, 256, 0, st>>>(R.big.p, R.ctl.p + kBig, R.tile_seg.p);
-    k_pivot<<<grid_all(n_big, 128), 128, 0, st>>>(R.big.p, n_big, R.key.p, R.idx.p);
-    k_count<<<n_tiles, kTileThreads, 0, st>>>(R.big.p, R.tile_seg.p, R.key.p, R.cnt_l.p,
-                                              R.cnt_r.p);
-    k_tile_offsets<<<grid_all(n_big, 128), 128, 0, st>>>(R.big.p, n_big, R.cnt_l.p, R.cnt_r.p,
-                                                         R.off_l.p, R.off_r.p, R.totals.p);
-    k_stops<<<n_tiles, kTileThreads, 0, st>>>(R.big.p, R.tile_seg.p, R.key.p, R.off_l.p,
-                                              R.off_r.p, R.totals.p, R.lpos.p, R.rpos.p);
-    k_exchange<<<n_tiles, kTileThreads, 0, st>>>(R.big.p, R.tile_seg.p, R.totals.p, R.lpos.p,
-                                                 R.rpos.p, R.key.p, R.idx.p);
-    CK(cudaMemsetAsync(R.ctl.p + kBigNext, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(R.ctl.p + kTilesNext, 0, sizeof(int), st));
-    k_cut<<<grid_all(n_big, 128), 128, 0, st>>>(R.big.p, n_big, R.totals.p, R.lpos.p, R.rpos.p,
-                                                R.big_next.p, R.small.p, R.small_cap, R.tiny.p,
-                                                R.heap.p, R.ctl.p);
+  // Rounds of partitions, the counts read back after as many as segments of the
+  // average length need if they halve, then after every fourth (a round that
+  // finds nothing to do costs four empty launches).
+  int par = 0, round = 0;
+  while (h[kBig + par] > 0) {
+    const int n_big = h[kBig + par];
+    int rounds = 4;
+    if (round == 0)
+      rounds = int(std::log2(double(h[kTiles + par]) * kTile / n_big / kSmallMax)) + 2;
+    for (int r = 0; r < rounds; ++r, par ^= 1, ++round) {
+      const int segs = int(std::min<size_t>(R.big.n, size_t(R.sms) * 4));
+      const int tiles = int(std::min<size_t>(R.tile_seg.n, size_t(R.sms) * 4));
+      SortSeg* const big = par ? R.big_next.p : R.big.p;
+      SortSeg* const next = par ? R.big.p : R.big_next.p;
+      k_pivot<<<segs, 128, 0, st>>>(big, R.ctl.p, par, R.key.p, R.idx.p, R.tile_seg.p);
+      k_count<<<tiles, kTileThreads, 0, st>>>(big, R.ctl.p, par, R.tile_seg.p, R.key.p, R.cnt.p);
+      k_stops<<<tiles, kTileThreads, 0, st>>>(big, R.ctl.p, par, R.tile_seg.p, R.key.p, R.cnt.p,
+                                              R.totals.p, R.lpos.p, R.rpos.p);
+      k_cut<<<tiles, kTileThreads, 0, st>>>(big, R.ctl.p, par, R.tile_seg.p, R.totals.p, R.lpos.p,
+                                            R.rpos.p, R.key.p, R.idx.p, next, R.small.p,
+                                            R.small_cap, R.tiny.p, R.heap.p);
+    }
     CK(cudaGetLastError());
+    if (round > 128) throw std::string("device reference BVH: too many partition rounds");
     read_ctl(R, h, st);
-    n_big = h[kBigNext];
-    n_tiles = h[kTilesNext];
-    CK(cudaMemcpyAsync(R.ctl.p + kBig, R.ctl.p + kBigNext, sizeof(int), cudaMemcpyDeviceToDevice,
-                       st));
-    std::swap(R.big.p, R.big_next.p);
-    std::swap(R.big.n, R.big_next.n);
   }
   if (h[kSmall])
     k_small<kSmallMax, kSmallWarps>
@@ -902,10 +901,7 @@ static void device_ref_bvh(const float* v, int nt, cudaStream_t st, DeviceTables
   R.rpos.ensure(nz);
   const size_t tiles = nz / (kTile / 2) + 16, lists = nz / 2 + 16;
   R.tile_seg.ensure(tiles);
-  R.cnt_l.ensure(tiles);
-  R.cnt_r.ensure(tiles);
-  R.off_l.ensure(tiles);
-  R.off_r.ensure(tiles);
+  R.cnt.ensure(tiles);
   R.totals.ensure(nz / kSmallMax + 16);
   R.big.ensure(nz / kSmallMax + 16);
   R.big_next.ensure(nz / kSmallMax + 16);
