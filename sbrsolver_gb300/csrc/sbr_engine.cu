@@ -48,6 +48,7 @@
 #include "sbr_capture.cuh"
 #include "sbr_paths.cuh"
 #include "sbr_dirs.cuh"
+#include "sbr_tables.cuh"
 #include "sbr_prep.cuh"
 #include "sbr_refbvh.cuh"
 
@@ -340,111 +341,82 @@ static void pattern_params(const sbr_pattern* p, int scene_device, TxParams& P) 
   P.pat = reinterpret_cast<const float4*>(dev);
 }
 
-// Runs f(b, e) over slices of [0, n) on the host's cores.
-static void host_parallel(size_t n, const std::function<void(size_t, size_t)>& f) {
-  const size_t T = std::max<size_t>(1, std::min<size_t>(std::thread::hardware_concurrency(), 32));
-  if (n < 8192 || T == 1) {
-    f(0, n);
-    return;
+static int grid_all(long long n, int block);
+
+// The triangle tables (sbr_tables.cuh): those by rank if by_rank, and corr[id] =
+// the triangle at mesh position id (what triangleMesh[id] returns).
+static void upload_triangles(SceneImpl& S, bool by_rank, const std::vector<int>& mesh_order) {
+  using namespace tables;
+  const HostScene& H = S.host;
+  const int nt = int(H.tris.size());
+  cudaStream_t st = S.stream;
+  DBuf<HostTri> chunk;
+  chunk.ensure(size_t(std::min(nt, kTableChunk)));
+  DBuf<int> perm, rank_of, position_of, found;
+  auto invert = [&](const std::vector<int>& p, DBuf<int>& inverse) {
+    perm.upload(p.data(), size_t(nt), st);
+    inverse.ensure(size_t(nt));
+    k_invert<<<grid_all(nt, 256), 256, 0, st>>>(perm.p, nt, inverse.p);
+  };
+  invert(mesh_order, position_of);
+  S.corr.ensure(size_t(nt));
+  S.corr32.ensure(size_t(nt));
+  if (by_rank) {
+    invert(H.dfs_tris, rank_of);
+    S.tri64.ensure(size_t(nt));
+    S.tri32.ensure(size_t(nt));
+    S.tri_cop.ensure(size_t(nt));
+    S.rank_to_id.ensure(size_t(nt));
+    found.ensure(2);
+    CK(cudaMemsetAsync(found.p, 0, 2 * sizeof(int), st));
   }
-  std::vector<std::thread> pool;
-  for (size_t k = 1; k < T; ++k) pool.emplace_back(f, n * k / T, n * (k + 1) / T);
-  f(0, n / T);
-  for (auto& t : pool) t.join();
+  for (int b = 0; b < nt; b += kTableChunk) {
+    const int n = std::min(nt - b, kTableChunk);
+    chunk.upload(H.tris.data() + b, size_t(n), st);
+    if (by_rank)
+      k_rank_tables<<<grid_all(n, 256), 256, 0, st>>>(chunk.p, b, n, rank_of.p, S.tri64.p,
+                                                      S.tri32.p, S.tri_cop.p, S.rank_to_id.p,
+                                                      found.p);
+    k_mesh_tables<<<grid_all(n, 256), 256, 0, st>>>(chunk.p, b, n, position_of.p, S.corr.p,
+                                                    S.corr32.p);
+  }
+  CK(cudaGetLastError());
+  int f[2] = {0, 0};
+  if (by_rank) CK(cudaMemcpyAsync(f, found.p, sizeof f, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (by_rank) {
+    S.dev.soft = f[0] ? 0 : 1;
+    S.n_cop = f[1];
+  }
+  S.dev.corr = S.corr.p;
+  S.dev.corr32 = S.corr32.p;
 }
 
-static void upload_scene(SceneImpl& S) {
+static void upload_scene(SceneImpl& S, const std::vector<int>& mesh_order) {
+  using namespace tables;
   const HostScene& H = S.host;
   const int nt = int(H.tris.size()), nn = int(H.nodes.size());
-  std::vector<Node32> n32(nn);
-  std::vector<RefNode> ref(nn);
   const double margin_m = std::ldexp(H.extent + 1.0, -14);
-  host_parallel(size_t(nn), [&](size_t b, size_t e) {
-    for (int i = int(b); i < int(e); ++i) {
-      const HostNode& h = H.nodes[i];
-      RefNode& r = ref[i];
-      std::memcpy(r.bb, h.bb, sizeof r.bb);
-      r.flat = 0;
-      for (int a = 0; a < 6; ++a) r.fb[a] = float(h.bb[a]);
-      for (int a = 0; a < 3; ++a) {
-        // boxes of float vertices are floats; a non-float bound (empty box
-        // sentinel) disables the FP32 decision for that node
-        if (double(r.fb[a]) != h.bb[a] || double(r.fb[3 + a]) != h.bb[3 + a]) r.flat |= 8;
-        if (h.bb[a] == h.bb[3 + a]) r.flat |= 1 << a;
-      }
-      r.c0 = h.c0;
-      r.c1 = h.c1;
-      r.first = h.first;
-      r.count = h.count;
-      r.parent = h.parent;
-      Node32& m = n32[i];
-      std::memset(&m, 0, sizeof m);
-      if (h.c0 >= 0) {
-        const int cs[2] = {h.c0, h.c1};
-        for (int k = 0; k < 2; ++k) {
-          const HostNode& c = H.nodes[cs[k]];
-          float* lo = k == 0 ? m.lo0 : m.lo1;
-          float* hi = k == 0 ? m.hi0 : m.hi1;
-          for (int a = 0; a < 3; ++a) {
-            // outward rounding keeps the FP32 box around the FP64 one
-            lo[a] = std::nextafter(float(c.bb[a]), -INFINITY);
-            hi[a] = std::nextafter(float(c.bb[3 + a]), INFINITY);
-          }
-          m.child[k] = c.c0 >= 0 ? cs[k] : ~cs[k];
-        }
-      }
+  cudaStream_t st = S.stream;
+  upload_triangles(S, true, mesh_order);
+  {
+    DBuf<HostNode> chunk;
+    chunk.ensure(size_t(std::min(nn, kTableChunk)));
+    S.ref.ensure(size_t(nn));
+    S.node32.ensure(size_t(nn));
+    for (int b = 0; b < nn; b += kTableChunk) {
+      const int n = std::min(nn - b, kTableChunk);
+      chunk.upload(H.nodes.data() + b, size_t(n), st);
+      k_ref_nodes<<<grid_all(n, 256), 256, 0, st>>>(chunk.p, b, n, S.ref.p, S.tri64.p);
     }
-  });
-  std::vector<Tri32> t32(nt);
-  std::vector<Tri64> t64(nt);
-  std::vector<int> cop(nt), r2i(nt);
-  std::atomic<bool> soft{true};
-  host_parallel(size_t(nt), [&](size_t b, size_t e) {
-    bool ok = true;
-    for (int r = int(b); r < int(e); ++r) {
-      const HostTri& t = H.tris[H.dfs_tris[r]];
-      Tri64& d = t64[r];
-      Tri32& f = t32[r];
-      for (int a = 0; a < 3; ++a) {
-        d.v1[a] = t.v1[a];
-        d.e1[a] = t.v2[a] - t.v1[a];
-        d.e2[a] = t.v3[a] - t.v1[a];
-        d.n[a] = t.n[a];
-        f.v1[a] = float(d.v1[a]);
-        f.e1[a] = float(d.e1[a]);
-        f.e2[a] = float(d.e2[a]);
-        ok &= soft64::safe(d.v1[a]) && soft64::safe(d.e1[a]) && soft64::safe(d.e2[a]) &&
-              soft64::safe(d.n[a]);
-      }
-      f.nv1 = float(std::sqrt(d.v1[0] * d.v1[0] + d.v1[1] * d.v1[1] + d.v1[2] * d.v1[2])) * 1.0001f;
-      f.ne1 = float(std::sqrt(d.e1[0] * d.e1[0] + d.e1[1] * d.e1[1] + d.e1[2] * d.e1[2])) * 1.0001f;
-      f.ne2 = float(std::sqrt(d.e2[0] * d.e2[0] + d.e2[1] * d.e2[1] + d.e2[2] * d.e2[2])) * 1.0001f;
-      d.id = t.id;
-      d.cop = t.cop;
-      d.mat = t.mat;
-      d.node = -1;
-      cop[r] = t.cop;
-      r2i[r] = t.id;
-    }
-    if (!ok) soft = false;
-  });
-  host_parallel(size_t(nn), [&](size_t b, size_t e) {
-    for (int i = int(b); i < int(e); ++i)
-      if (H.nodes[i].c0 < 0)
-        for (int r = H.nodes[i].first; r < H.nodes[i].first + H.nodes[i].count; ++r)
-          t64[r].node = i;
-  });
-  S.n_cop = 0;
-  for (auto& t : H.tris) S.n_cop = std::max(S.n_cop, t.cop + 1);
+    k_node32<<<grid_all(nn, 256), 256, 0, st>>>(S.ref.p, nn, S.node32.p);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));  // chunk goes
+  }
   std::vector<Material> mats(S.materials.size());
   for (size_t i = 0; i < mats.size(); ++i)
     mats[i] = Material{S.materials[i].rel_permittivity_re, S.materials[i].rel_conductivity,
                        S.materials[i].width};
-  cudaStream_t st = S.stream;
-  S.node32.upload(n32.data(), n32.size(), st);
-  S.ref.upload(ref.data(), ref.size(), st);
-  S.tri32.upload(t32.data(), t32.size(), st);
-  S.tri64.upload(t64.data(), t64.size(), st);
   S.mats.upload(mats.data(), mats.size(), st);
   {  // search BVH, collapsed to four-wide nodes
     const SearchBVH& B = H.search;
@@ -509,20 +481,17 @@ static void upload_scene(SceneImpl& S) {
       return me;
     };
     build4(0);
-    std::vector<Tri32> st32(B.order.size());
-    host_parallel(B.order.size(), [&](size_t lo, size_t hi) {
-      for (size_t j = lo; j < hi; ++j) st32[j] = t32[B.order[j]];
-    });
     S.snode4.upload(sn.data(), sn.size(), st);
-    S.stri.upload(st32.data(), st32.size(), st);
     S.srank.upload(B.order.data(), B.order.size(), st);
+    S.stri.ensure(B.order.size());
+    k_search_tris<<<grid_all((long long)B.order.size(), 256), 256, 0, st>>>(
+        S.tri32.p, S.srank.p, int(B.order.size()), S.stri.p);
+    CK(cudaGetLastError());
     S.dev.snode4 = S.snode4.p;
     S.dev.stri = S.stri.p;
     S.dev.srank = S.srank.p;
     CK(cudaStreamSynchronize(st));  // the host vectors above go out of scope
   }
-  S.tri_cop.upload(cop.data(), cop.size(), st);
-  S.rank_to_id.upload(r2i.data(), r2i.size(), st);
   S.dev.node32 = S.node32.p;
   S.dev.ref = S.ref.p;
   S.dev.tri32 = S.tri32.p;
@@ -533,54 +502,13 @@ static void upload_scene(SceneImpl& S) {
   S.dev.n_nodes = nn;
   S.dev.n_mats = int(mats.size());
   S.dev.root_leaf = H.nodes[0].c0 < 0 ? 1 : 0;
-  S.dev.soft = soft.load() ? 1 : 0;
   S.dev.box_margin = float(margin_m);
-  S.dev_bytes = (long long)(n32.size() * sizeof(Node32) + ref.size() * sizeof(RefNode) +
-                            t32.size() * sizeof(Tri32) + t64.size() * sizeof(Tri64) +
-                            2 * nt * sizeof(int) + nt * sizeof(CorrTri) +
+  S.dev_bytes = (long long)(nn * (sizeof(Node32) + sizeof(RefNode)) +
+                            nt * (sizeof(Tri32) + sizeof(Tri64) + 2 * sizeof(int) +
+                                  sizeof(CorrTri)) +
                             S.snode4.n * sizeof(Node4) + S.stri.n * sizeof(Tri32) +
                             S.srank.n * sizeof(int));
   CK(cudaStreamSynchronize(st));
-}
-
-// corr[id] = the triangle at mesh position id (what triangleMesh[id] returns).
-static void upload_mesh_order(SceneImpl& S, const std::vector<int>& order) {
-  const HostScene& H = S.host;
-  const int nt = int(H.tris.size());
-  std::vector<CorrTri> c(nt);
-  std::vector<Tri32> c32(nt);
-  host_parallel(size_t(nt), [&](size_t lo, size_t hi) {
-    for (int i = int(lo); i < int(hi); ++i) {
-      const HostTri& t = H.tris[order[i]];
-      CorrTri& d = c[i];
-      for (int a = 0; a < 3; ++a) {
-        d.v1[a] = t.v1[a];
-        d.e1[a] = t.v2[a] - t.v1[a];
-        d.e2[a] = t.v3[a] - t.v1[a];
-        d.n[a] = t.n[a];
-      }
-      std::memcpy(d.cs, t.cs, sizeof d.cs);
-      d.mat = t.mat;
-      d.pad = 0;
-    }
-    for (int i = int(lo); i < int(hi); ++i) {
-      Tri32& f = c32[i];
-      for (int a = 0; a < 3; ++a) {
-        f.v1[a] = float(c[i].v1[a]);
-        f.e1[a] = float(c[i].e1[a]);
-        f.e2[a] = float(c[i].e2[a]);
-      }
-      auto n3 = [](const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]); };
-      f.nv1 = float(n3(c[i].v1)) * 1.0001f;
-      f.ne1 = float(n3(c[i].e1)) * 1.0001f;
-      f.ne2 = float(n3(c[i].e2)) * 1.0001f;
-    }
-  });
-  S.corr.upload(c.data(), c.size(), S.stream);
-  S.corr32.upload(c32.data(), c32.size(), S.stream);
-  S.dev.corr = S.corr.p;
-  S.dev.corr32 = S.corr32.p;
-  CK(cudaStreamSynchronize(S.stream));
 }
 
 static int device_sms();
@@ -2257,8 +2185,7 @@ static sbr_status scene_common(std::vector<float>& v, std::vector<float>& n, con
           " exceeds the traversal stack (" + std::to_string(kStack) + ")";
     S.materials.assign(materials, materials + n_materials);
     const auto t_up = std::chrono::steady_clock::now();
-    upload_scene(S);
-    upload_mesh_order(S, S.host.mesh_order);
+    upload_scene(S, S.host.mesh_order);
     CK(cudaStreamSynchronize(S.stream));
     S.prep_ms[5] = ms_since(t_up);
     S.prep_ms[0] = ms_since(t_start);
@@ -2416,7 +2343,7 @@ sbr_status sbr_scene_set_mesh_order(sbr_scene* scene, const int* order) {
     // not to be called while solves on this scene are in flight
     std::lock_guard<std::mutex> lock(scene->impl.pool_mu);
     scene->impl.host.mesh_order = o;
-    upload_mesh_order(scene->impl, o);
+    upload_triangles(scene->impl, false, o);
     return SBR_OK;
   })
 }
@@ -2443,8 +2370,7 @@ sbr_status sbr_scene_set_materials(sbr_scene* scene, const int* material_ids,
     std::lock_guard<std::mutex> lock(S.pool_mu);
     for (int i = 0; i < nt; ++i) S.host.tris[i].mat = material_ids ? material_ids[i] : 0;
     S.materials.assign(materials, materials + n_materials);
-    upload_scene(S);
-    upload_mesh_order(S, S.host.mesh_order);
+    upload_scene(S, S.host.mesh_order);
     return SBR_OK;
   })
 }
