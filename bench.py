@@ -38,7 +38,7 @@ EVENT_BYTES = 16     # per capture event (group-table rank + count update)
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of k_trace's
 # first launch of the level-9 urban solve (its 2,621,442 launch rays), from
 # one ncu capture of that launch alone: profiles/k_trace_urban_L9_first_launch.md
-TRACE_FIRST_LAUNCH_DRAM_BYTES = 277407488 + 698306816
+TRACE_FIRST_LAUNCH_DRAM_BYTES = 273808896 + 646486016
 
 
 def _env_int(k, d):
@@ -449,7 +449,7 @@ def main():
     ap.add_argument("--no-serving", action="store_true")
     ap.add_argument("--no-precision", action="store_true")
     ap.add_argument("--tuning", default="",
-                    help="launch shapes of the benchmark scene, e.g. trace_kernel=2,find_steps=16 "
+                    help="launch shapes of the benchmark scene, e.g. find_steps=16,trace_chunk_log2=24 "
                          "(sbr_tuning field names; default: the library's)")
     ap.add_argument("--scene-prep", action="store_true",
                     help="only time the scene preparation of the large terrain (580,484 "
