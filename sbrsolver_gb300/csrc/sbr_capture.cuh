@@ -684,6 +684,53 @@ struct StagedNode {
   uint32_t cls, grid;  // grid: its receivers' grid (CaptureArgs::grids)
 };
 
+// The correction prefilter of a node's class as a candidate needs it: the image
+// source, the last triangle's edges, tri_from's terms and the margins' factors
+// (tri_filter_from's, the ones that depend on the class alone multiplied
+// beforehand).  Five 16-byte loads a candidate instead of 23 words of two
+// records, and the cones an odd number of words apart: the kernel is bound by
+// issue and L1 (level-9 canyon 5.05 -> 4.89 ms, 24 requests 2.53 -> 2.45, level-10
+// terrain 5.25 -> 5.15).  Seven blocks an SM, with 48 pairs gathered instead of
+// 64 to fit, took 5.01 ms in the canyon and 0.155 for 0.141 ms on a line of
+// receivers.
+struct __align__(16) LineFilter {
+  float img[3], W, e1[3], ka, e2[3], ku, s[3], kv, q[3], kw;
+};
+__device__ __forceinline__ LineFilter line_filter(const ClassCap& c, const Tri32& T) {
+  LineFilter L;
+  const float ns = c.F[7];
+  for (int a = 0; a < 3; ++a) {
+    L.img[a] = c.img[a];
+    L.e1[a] = T.e1[a];
+    L.e2[a] = T.e2[a];
+    L.s[a] = c.F[a];
+    L.q[a] = c.F[3 + a];
+  }
+  L.W = c.F[6];
+  L.ka = kCorrK * T.ne1 * T.ne2;
+  L.ku = kCorrK * ns * T.ne2;
+  L.kv = kCorrK * ns * T.ne1;
+  L.kw = kCorrK * ns * T.ne1 * T.ne2;
+  return L;
+}
+// tri_filter_from of the line from the image source to c.
+__device__ __forceinline__ bool line_may_cross(const LineFilter& L, const float3& c) {
+  const float dx = c.x - L.img[0], dy = c.y - L.img[1], dz = c.z - L.img[2];
+  const float nd = sqrt_up(dx * dx + dy * dy + dz * dz);
+  const float hx = dy * L.e2[2] - dz * L.e2[1];
+  const float hy = dz * L.e2[0] - dx * L.e2[2];
+  const float hz = dx * L.e2[1] - dy * L.e2[0];
+  const float a = L.e1[0] * hx + L.e1[1] * hy + L.e1[2] * hz;
+  const float sg = copysignf(1.0f, a), A = fabsf(a);
+  const float U = sg * (L.s[0] * hx + L.s[1] * hy + L.s[2] * hz);
+  const float V = sg * (dx * L.q[0] + dy * L.q[1] + dz * L.q[2]);
+  const float W = sg * L.W;
+  const float ea = L.ka * nd, eU = L.ku * nd, eV = L.kv * nd;
+  const bool parallel = A <= kEps32 + ea;  // the FP64 test decides
+  return parallel || (U >= -eU && V >= -eV && U <= A + ea + eU && U + V <= A + ea + eU + eV &&
+                      W + L.kw > (kEps32 * 0.5f) * (A - ea));
+}
+
 // Pairs for k_capture_finish, gathered per warp so that one atomic on the pair
 // counter (which every warp of the grid adds to) serves more than 32 of them.
 constexpr int kPairBuf = 64;
@@ -710,12 +757,10 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
   __shared__ StagedNode s_nh[kCapWarps][B];
   __shared__ uint2 s_pr[kCapWarps][kPairBuf];
   int n_pr = 0;  // pairs gathered (the same on every lane)
-  __shared__ Tri32 s_tl[kCapWarps][B];      // the class's last triangle
-  __shared__ float s_fl[kCapWarps][B][12];  // image source + correction filter terms
-  __shared__ float s_cn[kCapWarps][B][16];  // loosened correction cone
-  __shared__ NodeSpan s_sp[kCapWarps][B];   // clipped span and chunking
+  __shared__ LineFilter s_lf[kCapWarps][B];  // the class's correction prefilter
+  __shared__ float s_cn[kCapWarps][B][15];   // loosened correction cone (odd: no bank conflicts)
+  __shared__ NodeSpan s_sp[kCapWarps][B];    // clipped span and chunking
   __shared__ ChunkBox s_ck[kCapWarps][32];  // the current 32 (node, chunk) items
-  __shared__ int s_ckn[kCapWarps][32];      // their node (batch index) | chunk << 8
   // fewer nodes than the grid's lanes: fewer nodes per warp, so that each
   // node's chunks still find a warp of their own (184 nodes of up to 250
   // chunks on 6 warps took 1.9 ms)
@@ -739,10 +784,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
         int cone_ok = 0;
         if (!is_root_class(h.cls)) {
           const ClassCap c = A.cls_cap[h.cls];
-          s_tl[warp][lane] = A.sc.corr32[c.tpos];
-          float* fl = s_fl[warp][lane];
-          for (int q = 0; q < 3; ++q) fl[q] = c.img[q];
-          for (int q = 0; q < 8; ++q) fl[3 + q] = c.F[q];
+          s_lf[warp][lane] = line_filter(c, A.sc.corr32[c.tpos]);
           // the cone's planes loosened by 2 m, m = 2^-21 |n| (cmax + |img| + |T| + 1)
           float* cn = s_cn[warp][lane];
           cone_ok = 1;
@@ -777,9 +819,9 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
         const RxGrid& g = A.grids[nd.grid];
         const ChunkBox cb = chunk_box(nd, g, sp, ch, g.cmax, g.tanb, sp.use_cone != 0,
                                       s_cn[warp][j]);
-        s_ck[warp][lane] = cb;
-        s_ckn[warp][lane] = j | ch << 8;
         nrows = cb.nrows;
+        s_ck[warp][lane] = cb;
+        s_ck[warp][lane].nrows = j | ch << 8;  // node (batch index), chunk
       }
       __syncwarp();
       const int r_incl = warp_incl_scan(nrows, lane);
@@ -794,7 +836,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
         if (r < n_r) {
           const int ridx = r - (ci_incl - ci_n);
           const ChunkBox& cb = s_ck[warp][ci];
-          const int jn = s_ckn[warp][ci] & 0xff;
+          const int jn = cb.nrows & 0xff;
           const StagedNode& nd = s_nh[warp][jn];
           const RxGrid& g = A.grids[nd.grid];
           const int ar = g.ax[0], am = g.ax[1], al = g.ax[2];
@@ -855,7 +897,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
           uint2 pair = make_uint2(0, 0);
           auto passes = [&]() -> bool {
             if (q >= n_c) return false;
-            const int ckn = s_ckn[warp][rci];
+            const int ckn = s_ck[warp][rci].nrows;
             const int jn = ckn & 0xff, ch = ckn >> 8;
             const StagedNode& nd = s_nh[warp][jn];
             const NodeSpan& sp = s_sp[warp][jn];
@@ -871,16 +913,9 @@ __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast
             if (ch < sp.nchunk - 1 && lam >= b) return false;    // owned by a later chunk
             const int gi = __float_as_int(c4.w);
             ++cand;
-            if (!is_root_class(nd.cls)) {
-              // MultiPathCorrection's last step must cross the class's last
-              // triangle: FP32 filter from the image source towards the receiver
-              const float* fl = s_fl[warp][jn];
-              const TriFrom Fl{fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10]};
-              const float3 dd = make_float3(c.x - fl[0], c.y - fl[1], c.z - fl[2]);
-              if (!tri_filter_from(s_tl[warp][jn], Fl, dd,
-                                   sqrt_up(dd.x * dd.x + dd.y * dd.y + dd.z * dd.z)))
-                return false;
-            }
+            // MultiPathCorrection's last step must cross the class's last
+            // triangle: FP32 filter from the image source towards the receiver
+            if (!is_root_class(nd.cls) && !line_may_cross(s_lf[warp][jn], c)) return false;
             const float tanb = g.tanb;
             const float len = nd.len, S = nd.S;
             int v;
