@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -215,16 +216,44 @@ struct Workspace {
   std::vector<std::string> seen;  // keys that ran eagerly, most recent last
   unsigned long long graph_tick = 0;
   long long pipeline_kernels = 0;  // kernels the last pipeline ran
-  // capacities (grown from occupancy and on overflow)
-  unsigned long long cap_nodes = 1 << 20, cap_queue = 1 << 19, cap_surv = 1 << 14;
-  unsigned long long cap_corr = 1 << 16, cap_pairs = 1 << 20;
-  uint32_t cap_cls = 1 << 16, cap_cop = 1 << 14, cap_dd = 1 << 14, cap_cc = 1 << 14;
-  // occupancy seen per executed segment in earlier solves, used to size the
-  // tables of the next solve before it runs
-  // (first solve: values typical of the urban canyon, so most first solves
-  // need no retry)
-  double r_cls = 0.01, r_cop = 0.004, r_corr = 0.01, r_dd = 5e-4, r_surv = 5e-4, r_pairs = 0.1,
-         r_cc = 0.01;
+  // Capacities (grown from occupancy and on overflow) and the occupancy seen per
+  // executed segment in earlier solves, which sizes the tables of the next one
+  // before it runs, kept by the solve's size: floor(log2) of its ray trees'
+  // nodes.  A solve clears its tables, so their size is time: when all solves
+  // shared one set, 500 nodes with 3,000 receivers taught a level-9 canyon
+  // solve tables of gigabytes (1.4 of its 17.1 ms to clear), and small solves
+  // after large ones cleared the large ones' tables.
+  struct Sizing {
+    bool used = false;
+    unsigned long long cap_nodes = 1 << 20, cap_queue = 1 << 19, cap_surv = 1 << 14;
+    unsigned long long cap_corr = 1 << 16, cap_pairs = 1 << 20;
+    uint32_t cap_cls = 1 << 16, cap_cop = 1 << 14, cap_dd = 1 << 14, cap_cc = 1 << 14;
+    // (first solve: values typical of the urban canyon, so most first solves
+    // need no retry)
+    double r_cls = 0.01, r_cop = 0.004, r_corr = 0.01, r_dd = 5e-4, r_surv = 5e-4, r_pairs = 0.1,
+           r_cc = 0.01;
+  };
+  std::array<Sizing, 64> sizing;
+  // The set for a solve of `nodes`; a new one starts from the occupancy of the
+  // nearest within a factor of four.
+  Sizing& sizing_for(double nodes) {
+    const int k = std::min(63, std::max(0, int(std::log2(std::max(1.0, nodes)))));
+    Sizing& z = sizing[size_t(k)];
+    for (int d : {1, -1, 2, -2}) {
+      if (z.used || k + d < 0 || k + d > 63 || !sizing[size_t(k + d)].used) continue;
+      const Sizing& o = sizing[size_t(k + d)];
+      z.r_cls = o.r_cls;
+      z.r_cop = o.r_cop;
+      z.r_corr = o.r_corr;
+      z.r_dd = o.r_dd;
+      z.r_surv = o.r_surv;
+      z.r_pairs = o.r_pairs;
+      z.r_cc = o.r_cc;
+      break;
+    }
+    z.used = true;
+    return z;
+  }
   ~Workspace() {
     for (auto& g : graphs) {
       if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -1182,7 +1211,8 @@ static FieldConsts field_consts() {
 // receiver counts and offsets, field precisions, device receiver pointers),
 // the capacities, every buffer and scene pointer, the launch shapes and the
 // solve's flags.  Two solves with the same key run the same operations.
-static std::string pipeline_key(const SceneImpl& S, const Workspace& W, const sbr_request* reqs,
+static std::string pipeline_key(const SceneImpl& S, const Workspace& W,
+                                const Workspace::Sizing& Z, const sbr_request* reqs,
                                 const std::vector<TxParams>& tp, int n_req, int rx_total,
                                 long long launches, int max_depth, size_t cell_cap,
                                 long long chunk, const Tuning& tu, int stage_counts,
@@ -1211,8 +1241,8 @@ static std::string pipeline_key(const SceneImpl& S, const Workspace& W, const sb
     put_v(tp[r].precision);
     put_v(reqs[r].rx_on_device ? reqs[r].rx : nullptr);
   }
-  const unsigned long long caps[9] = {W.cap_nodes, W.cap_queue, W.cap_cls, W.cap_cop, W.cap_dd,
-                                      W.cap_cc,    W.cap_corr,  W.cap_surv, W.cap_pairs};
+  const unsigned long long caps[9] = {Z.cap_nodes, Z.cap_queue, Z.cap_cls, Z.cap_cop, Z.cap_dd,
+                                      Z.cap_cc,    Z.cap_corr,  Z.cap_surv, Z.cap_pairs};
   put(caps, sizeof caps);
   const void* ptrs[] = {W.up.p, W.rx_bad.p, W.path_bound.p, W.field_bound.p, W.rx_flag.p,
                         W.fstat.p, W.grids.p, W.all.base.p, W.all.counts.p, W.all.starts.p,
@@ -1424,26 +1454,27 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       g.n = 0;
     }
   const FieldConsts K = field_consts();
+  double nodes = 0, width = 0;
+  for (int r = 0; r < n_req; ++r) {
+    const double L = double(tp[r].n_launch);
+    nodes += L * tree_nodes(tp[r].R, tp[r].T);
+    width += L * tree_width(tp[r].R, tp[r].T);
+  }
+  Workspace::Sizing& Z = W.sizing_for(nodes);
   {
     // Size node pool and queues at the ray-tree bounds so a pass needs no
     // re-run (the batch splitter keeps each pass within the memory budget).
-    double nodes = 0, width = 0;
-    for (int r = 0; r < n_req; ++r) {
-      const double L = double(tp[r].n_launch);
-      nodes += L * tree_nodes(tp[r].R, tp[r].T);
-      width += L * tree_width(tp[r].R, tp[r].T);
-    }
-    W.cap_nodes = std::max<unsigned long long>(W.cap_nodes, (unsigned long long)nodes + 1024);
-    W.cap_queue = std::max<unsigned long long>(W.cap_queue, (unsigned long long)width + 1024);
+    Z.cap_nodes = std::max<unsigned long long>(Z.cap_nodes, (unsigned long long)nodes + 1024);
+    Z.cap_queue = std::max<unsigned long long>(Z.cap_queue, (unsigned long long)width + 1024);
     // Tables from the occupancy ratios learned so far (hash tables half
     // full), each limited to 2% of free device memory: past that the solve
     // grows the table on overflow instead.
     // The free memory is asked for only when one grows (6 us of each solve).
-    const bool grows = 2.2 * W.r_cls * nodes > W.cap_cls || 2.2 * W.r_cop * nodes > W.cap_cop ||
-                       2.2 * W.r_dd * nodes > W.cap_dd || 2.2 * W.r_cc * nodes > W.cap_cc ||
-                       1.2 * W.r_corr * nodes > double(W.cap_corr) ||
-                       1.2 * W.r_surv * nodes > double(W.cap_surv) ||
-                       1.3 * W.r_pairs * nodes > double(W.cap_pairs);
+    const bool grows = 2.2 * Z.r_cls * nodes > Z.cap_cls || 2.2 * Z.r_cop * nodes > Z.cap_cop ||
+                       2.2 * Z.r_dd * nodes > Z.cap_dd || 2.2 * Z.r_cc * nodes > Z.cap_cc ||
+                       1.2 * Z.r_corr * nodes > double(Z.cap_corr) ||
+                       1.2 * Z.r_surv * nodes > double(Z.cap_surv) ||
+                       1.3 * Z.r_pairs * nodes > double(Z.cap_pairs);
     size_t free_b = 0, total_b = 0;
     if (grows) CK(cudaMemGetInfo(&free_b, &total_b));
     const double cap_bytes = 0.02 * double(free_b);
@@ -1453,36 +1484,36 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       while (p < x && p < (1u << 30)) p <<= 1;
       return p;
     };
-    W.cap_cls = std::max(W.cap_cls, pow2(2.2 * W.r_cls * nodes, 8 + sizeof(ClassInfo) + sizeof(ClassCap), cap_bytes));
-    W.cap_cop = std::max(W.cap_cop, pow2(2.2 * W.r_cop * nodes, 8, cap_bytes));
-    W.cap_dd = std::max(W.cap_dd, pow2(2.2 * W.r_dd * nodes, 16, cap_bytes));
-    W.cap_cc = std::max(W.cap_cc, pow2(2.2 * W.r_cc * nodes, 9, cap_bytes));
-    W.cap_corr = std::max<unsigned long long>(
-        W.cap_corr, (unsigned long long)std::min(1.2 * W.r_corr * nodes, cap_bytes / sizeof(Corrected)));
-    W.cap_surv = std::max<unsigned long long>(
-        W.cap_surv, (unsigned long long)std::min(1.2 * W.r_surv * nodes, cap_bytes / 640.0));
-    W.cap_pairs = std::max<unsigned long long>(
-        W.cap_pairs, (unsigned long long)std::min(1.3 * W.r_pairs * nodes, cap_bytes / sizeof(uint2)));
+    Z.cap_cls = std::max(Z.cap_cls, pow2(2.2 * Z.r_cls * nodes, 8 + sizeof(ClassInfo) + sizeof(ClassCap), cap_bytes));
+    Z.cap_cop = std::max(Z.cap_cop, pow2(2.2 * Z.r_cop * nodes, 8, cap_bytes));
+    Z.cap_dd = std::max(Z.cap_dd, pow2(2.2 * Z.r_dd * nodes, 16, cap_bytes));
+    Z.cap_cc = std::max(Z.cap_cc, pow2(2.2 * Z.r_cc * nodes, 9, cap_bytes));
+    Z.cap_corr = std::max<unsigned long long>(
+        Z.cap_corr, (unsigned long long)std::min(1.2 * Z.r_corr * nodes, cap_bytes / sizeof(Corrected)));
+    Z.cap_surv = std::max<unsigned long long>(
+        Z.cap_surv, (unsigned long long)std::min(1.2 * Z.r_surv * nodes, cap_bytes / 640.0));
+    Z.cap_pairs = std::max<unsigned long long>(
+        Z.cap_pairs, (unsigned long long)std::min(1.3 * Z.r_pairs * nodes, cap_bytes / sizeof(uint2)));
   }
   for (int attempt = 0;; ++attempt) {
     if (attempt > 6) throw std::string("capacity: tables kept overflowing");
     W.ctr.ensure(1);
-    W.nodes.ensure(W.cap_nodes);
-    W.nodes_cold.ensure(W.cap_nodes);
-    W.q0.ensure(W.cap_queue);
-    W.q1.ensure(W.cap_queue);
-    W.cls_keys.ensure(W.cap_cls);
-    W.cls_info.ensure(W.cap_cls);
-    W.cls_cap.ensure(W.cap_cls);
-    W.cls_list.ensure(W.cap_cls);
-    W.cop_keys.ensure(W.cap_cop);
-    W.corr_list.ensure(W.cap_corr);
-    W.pairs.ensure(W.cap_pairs);
-    W.dd_keys.ensure(W.cap_dd);
-    W.cc_keys.ensure(W.cap_cc);
-    W.cc_val.ensure(W.cap_cc);
-    W.dd_rank.ensure(W.cap_dd);
-    W.surv.ensure(W.cap_surv);
+    W.nodes.ensure(Z.cap_nodes);
+    W.nodes_cold.ensure(Z.cap_nodes);
+    W.q0.ensure(Z.cap_queue);
+    W.q1.ensure(Z.cap_queue);
+    W.cls_keys.ensure(Z.cap_cls);
+    W.cls_info.ensure(Z.cap_cls);
+    W.cls_cap.ensure(Z.cap_cls);
+    W.cls_list.ensure(Z.cap_cls);
+    W.cop_keys.ensure(Z.cap_cop);
+    W.corr_list.ensure(Z.cap_corr);
+    W.pairs.ensure(Z.cap_pairs);
+    W.dd_keys.ensure(Z.cap_dd);
+    W.cc_keys.ensure(Z.cap_cc);
+    W.cc_val.ensure(Z.cap_cc);
+    W.dd_rank.ensure(Z.cap_dd);
+    W.surv.ensure(Z.cap_surv);
     W.seg_tx.ensure(n_req);
     // receivers and their grid
     W.up.ensure(up_bytes);
@@ -1502,7 +1533,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     // trace chunks: each depth runs in chunks of at most kTraceChunk rays
     const long long kTraceChunk =
         1LL << (tu.chunk_log2 > 0 ? std::min(tu.chunk_log2, 26) : kTraceChunkLog2);
-    const long long max_width = std::max<long long>(launches, (long long)W.cap_queue);
+    const long long max_width = std::max<long long>(launches, (long long)Z.cap_queue);
     const long long chunk = std::max<long long>(1, std::min(kTraceChunk, max_width));
     W.cand.ensure(size_t(chunk) * kCand);
     W.ncand.ensure(size_t(chunk));
@@ -1510,7 +1541,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     size_t n_launch_pairs = 0;  // k_find / k_trace launch pairs of the trace
     {
       for (int d = 0; d <= max_depth; ++d) {
-        const long long bound = d == 0 ? launches : (long long)W.cap_queue;
+        const long long bound = d == 0 ? launches : (long long)Z.cap_queue;
         n_launch_pairs += size_t((bound + chunk - 1) / chunk);
       }
       W.find_work.ensure(2 * n_launch_pairs + 1);
@@ -1522,7 +1553,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     }
     // the field stage, sized by the survivor capacity
     {
-      const size_t nsa = std::max<size_t>(1, W.cap_surv);
+      const size_t nsa = std::max<size_t>(1, Z.cap_surv);
       W.path_field.ensure(6 * nsa);
       W.path_nray.ensure(nsa);
       W.path_tri.ensure(nsa * (kMaxDepth + 1));
@@ -1605,7 +1636,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     fa.rank_to_id = S.rank_to_id.p;
     fa.surv = W.surv.p;
     fa.ctr = W.ctr.p;
-    fa.cap = W.cap_surv;
+    fa.cap = Z.cap_surv;
     fa.K = K;
     fa.precision = -1;
     fa.path_field = W.path_field.p;
@@ -1646,12 +1677,12 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     fill(W.seg_tx.p, sizeof(unsigned long long) * n_req, 0);
     fill(W.find_work.p, sizeof(unsigned long long) * (2 * n_launch_pairs + 1), 0);
     static_assert(kEmptyKey == ~0ull, "tables are cleared byte by byte");
-    fill(W.cls_keys.p, sizeof(unsigned long long) * W.cap_cls, 0xFF);
-    fill(W.cop_keys.p, sizeof(unsigned long long) * W.cap_cop, 0xFF);
-    fill(W.dd_keys.p, sizeof(unsigned long long) * W.cap_dd, 0xFF);
-    fill(W.dd_rank.p, sizeof(unsigned long long) * W.cap_dd, 0xFF);
-    fill(W.cc_keys.p, sizeof(unsigned long long) * W.cap_cc, 0xFF);
-    fill(W.cc_val.p, W.cap_cc, 0);
+    fill(W.cls_keys.p, sizeof(unsigned long long) * Z.cap_cls, 0xFF);
+    fill(W.cop_keys.p, sizeof(unsigned long long) * Z.cap_cop, 0xFF);
+    fill(W.dd_keys.p, sizeof(unsigned long long) * Z.cap_dd, 0xFF);
+    fill(W.dd_rank.p, sizeof(unsigned long long) * Z.cap_dd, 0xFF);
+    fill(W.cc_keys.p, sizeof(unsigned long long) * Z.cap_cc, 0xFF);
+    fill(W.cc_val.p, Z.cap_cc, 0);
     fill(W.rx_flag.p, sizeof(int) * std::max(1, rx_total), 0);
     fill(W.fstat.p, 2 * sizeof(unsigned long long), 0);
     fill(W.s_counts.p, sizeof(int) * (2 * size_t(rx_total) + 1), 0);
@@ -1696,10 +1727,10 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ta.dirs = S.dir_table.p;
     ta.nodes = W.nodes.p;
     ta.nodes_cold = W.nodes_cold.p;
-    ta.node_cap = W.cap_nodes;
-    ta.out_cap = W.cap_queue;
-    ta.cls_tab = HashTable{W.cls_keys.p, W.cap_cls - 1};
-    ta.cop_tab = HashTable{W.cop_keys.p, W.cap_cop - 1};
+    ta.node_cap = Z.cap_nodes;
+    ta.out_cap = Z.cap_queue;
+    ta.cls_tab = HashTable{W.cls_keys.p, Z.cap_cls - 1};
+    ta.cop_tab = HashTable{W.cop_keys.p, Z.cap_cop - 1};
     ta.cls_info = W.cls_info.p;
     ta.cls_cap = W.cls_cap.p;
     ta.cls_list = W.cls_list.p;
@@ -1717,7 +1748,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     fnd.n_tx = n_req;
     fnd.dirs = S.dir_table.p;
     fnd.ctr = W.ctr.p;
-    fnd.in_cap = W.cap_queue;
+    fnd.in_cap = Z.cap_queue;
     fnd.n_root = launches;
     fnd.cand = W.cand.p;
     fnd.ncand = W.ncand.p;
@@ -1733,7 +1764,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       ta.depth = fnd.depth = d;
       ta.in = fnd.in = (d % 2 == 0) ? W.q1.p : W.q0.p;
       ta.out = (d % 2 == 0) ? W.q0.p : W.q1.p;
-      const long long bound = d == 0 ? launches : (long long)W.cap_queue;
+      const long long bound = d == 0 ? launches : (long long)Z.cap_queue;
       for (long long lo = 0; lo < bound; lo += chunk) {
         ta.lo = fnd.lo = lo;
         ta.hi = fnd.hi = std::min(bound, lo + chunk);
@@ -1749,8 +1780,8 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       }
     }
     // correction cones of the classes the trace interned
-    ++nl, k_class_cones<<<grid_for(W.cap_cls / 2, 128), 128, 0, st>>>(
-        W.cls_list.p, W.ctr.p, W.cap_cls, W.cls_info.p, S.dev, W.cls_cap.p);
+    ++nl, k_class_cones<<<grid_for(Z.cap_cls / 2, 128), 128, 0, st>>>(
+        W.cls_list.p, W.ctr.p, Z.cap_cls, W.cls_info.p, S.dev, W.cls_cap.p);
     CK(cudaGetLastError());
     mark(W.ev[3]);
     // ---- capture
@@ -1767,13 +1798,13 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ca.cls_cap = W.cls_cap.p;
     ca.direct_ok = W.direct_ok.p;
     ca.corr_list = W.corr_list.p;
-    ca.corr_cap = W.cap_corr;
+    ca.corr_cap = Z.cap_corr;
     ca.ctr = W.ctr.p;
-    ca.node_cap = W.cap_nodes;
+    ca.node_cap = Z.cap_nodes;
     ca.stage_counts = stage_counts;
     ca.pairs = W.pairs.p;
-    ca.pair_cap = W.cap_pairs;
-    ca.corr_cache = HashTable{W.cc_keys.p, W.cap_cc - 1};
+    ca.pair_cap = Z.cap_pairs;
+    ca.corr_cache = HashTable{W.cc_keys.p, Z.cap_cc - 1};
     ca.corr_val = W.cc_val.p;
     ca.work = W.find_work.p + 2 * n_launch_pairs;
     CK(cudaStreamWaitEvent(st, W.join, 0));
@@ -1789,27 +1820,27 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     CK(cudaGetLastError());
     mark(W.ev[4]);
     // ---- duplicate removal over the corrected captures
-    const HashTable dd{W.dd_keys.p, W.cap_dd - 1};
-    ++nl, k_dedup<<<grid_for(W.cap_corr, 256), 256, 0, st>>>(W.corr_list.p, W.cap_corr, W.cls_info.p,
+    const HashTable dd{W.dd_keys.p, Z.cap_dd - 1};
+    ++nl, k_dedup<<<grid_for(Z.cap_corr, 256), 256, 0, st>>>(W.corr_list.p, Z.cap_corr, W.cls_info.p,
                                                        dd, W.dd_rank.p, W.ctr.p);
-    ++nl, k_select<<<grid_for(W.cap_corr, 256), 256, 0, st>>>(W.corr_list.p, W.cap_corr, W.cls_info.p,
-                                                        dd, W.dd_rank.p, W.surv.p, W.cap_surv,
+    ++nl, k_select<<<grid_for(Z.cap_corr, 256), 256, 0, st>>>(W.corr_list.p, Z.cap_corr, W.cls_info.p,
+                                                        dd, W.dd_rank.p, W.surv.p, Z.cap_surv,
                                                         W.ctr.p);
     CK(cudaGetLastError());
     mark(W.ev[5]);
     // ---- field + ordered per-receiver sum, sized by the survivor capacity
     // (the kernels take the count from the device), so the whole solve runs
     // without a host round trip until its results are read
-    const unsigned long long ns_cap = W.cap_surv;
+    const unsigned long long ns_cap = Z.cap_surv;
     ++nl, k_path<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
     ++nl, k_seg<<<grid_for(ns_cap * (kMaxDepth + 1), 64), 64, 0, st>>>(fa);
     ++nl, k_combine<<<grid_for(ns_cap, 64), 64, 0, st>>>(fa);
     if (any_fp32) ++nl, k_escalate<<<grid_for(ns_cap * 32, 64), 64, 0, st>>>(fa, false);
-    ++nl, k_surv_hist<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv,
+    ++nl, k_surv_hist<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, Z.cap_surv,
                                                        W.path_nray.p, W.s_counts.p,
                                                        W.s_counts.p + rx_total);
     nl += scan_ints(W.s_counts.p, W.s_starts.p, 2LL * rx_total, W.all.sums.p, st);
-    ++nl, k_surv_scatter<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, W.cap_surv,
+    ++nl, k_surv_scatter<<<grid_for(ns_cap, 256), 256, 0, st>>>(W.surv.p, W.ctr.p, Z.cap_surv,
                                                           W.s_starts.p, W.s_cursor.p, W.s_order.p);
     if (rx_total)
       ++nl, k_rx_sum<<<grid_for(rx_total, 128), 128, 0, st>>>(
@@ -1841,7 +1872,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     Workspace::PipelineGraph* graph = nullptr;
     const PipelineRun how =
         run_pipeline(W, st, record,
-                     pipeline_key(S, W, reqs, tp, n_req, rx_total, launches, max_depth, cell_cap,
+                     pipeline_key(S, W, Z, reqs, tp, n_req, rx_total, launches, max_depth, cell_cap,
                                   chunk, tu, stage_counts, field_check),
                      resolved(tu).graph > 0, &graph);
     if (how == kReplayed) nl = nl_before + graph->kernels;
@@ -1870,16 +1901,16 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     auto grow = [](uint32_t& cap, unsigned long long used) {
       while (used * 2 > cap && cap < (1u << 30)) cap *= 2;
     };
-    grow(W.cap_cls, c.used_cls);
-    grow(W.cap_cop, c.used_cop);
-    grow(W.cap_dd, c.used_dd);
-    grow(W.cap_cc, c.used_cc);  // a full cache only costs recomputation
+    grow(Z.cap_cls, c.used_cls);
+    grow(Z.cap_cop, c.used_cop);
+    grow(Z.cap_dd, c.used_dd);
+    grow(Z.cap_cc, c.used_cc);  // a full cache only costs recomputation
     if (c.overflow) {
-      if (c.overflow & kOvNodes) W.cap_nodes = std::max(W.cap_nodes * 2, c.nodes + c.nodes / 8);
+      if (c.overflow & kOvNodes) Z.cap_nodes = std::max(Z.cap_nodes * 2, c.nodes + c.nodes / 8);
       if (c.overflow & kOvQueue) {
         unsigned long long mx = 0;
         for (auto v : c.queue) mx = std::max(mx, v);
-        W.cap_queue = std::max(W.cap_queue * 2, mx + mx / 8);
+        Z.cap_queue = std::max(Z.cap_queue * 2, mx + mx / 8);
       }
       // at least 4x, and twice what the refused inserts say was needed (the
       // trace stops at the overflow, so later depths are not counted)
@@ -1887,12 +1918,12 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
         const unsigned long long need = std::max<unsigned long long>(4ull * cap, 2 * (used + lost));
         while (cap < need && cap < (1u << 30)) cap *= 2;
       };
-      if (c.overflow & kOvClass) regrow(W.cap_cls, c.used_cls, c.lost_cls);
-      if (c.overflow & kOvCop) regrow(W.cap_cop, c.used_cop, c.lost_cop);
-      if (c.overflow & kOvCorr) W.cap_corr = std::max(W.cap_corr * 2, c.corrected + c.corrected / 4);
-      if (c.overflow & kOvDedup) regrow(W.cap_dd, c.used_dd, c.lost_dd);
-      if (c.overflow & kOvSurv) W.cap_surv = next_pow2(c.survivors + c.survivors / 4);
-      if (c.overflow & kOvPairs) W.cap_pairs = std::max(W.cap_pairs * 2, c.pairs + c.pairs / 4);
+      if (c.overflow & kOvClass) regrow(Z.cap_cls, c.used_cls, c.lost_cls);
+      if (c.overflow & kOvCop) regrow(Z.cap_cop, c.used_cop, c.lost_cop);
+      if (c.overflow & kOvCorr) Z.cap_corr = std::max(Z.cap_corr * 2, c.corrected + c.corrected / 4);
+      if (c.overflow & kOvDedup) regrow(Z.cap_dd, c.used_dd, c.lost_dd);
+      if (c.overflow & kOvSurv) Z.cap_surv = next_pow2(c.survivors + c.survivors / 4);
+      if (c.overflow & kOvPairs) Z.cap_pairs = std::max(Z.cap_pairs * 2, c.pairs + c.pairs / 4);
       continue;
     }
     if (c.nodes) {
@@ -1901,13 +1932,13 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
       for (int r = 0; r < n_req; ++r) bound += double(tp[r].n_launch) * tree_nodes(tp[r].R, tp[r].T);
       const double n = std::max(1.0, bound);
       auto upd = [](double& r, double v) { r = std::max(0.9 * r, v); };
-      upd(W.r_cls, c.used_cls / n);
-      upd(W.r_cop, c.used_cop / n);
-      upd(W.r_dd, c.used_dd / n);
-      upd(W.r_cc, c.used_cc / n);
-      upd(W.r_corr, c.corrected / n);
-      upd(W.r_surv, c.survivors / n);
-      upd(W.r_pairs, c.pairs / n);
+      upd(Z.r_cls, c.used_cls / n);
+      upd(Z.r_cop, c.used_cop / n);
+      upd(Z.r_dd, c.used_dd / n);
+      upd(Z.r_cc, c.used_cc / n);
+      upd(Z.r_corr, c.corrected / n);
+      upd(Z.r_surv, c.survivors / n);
+      upd(Z.r_pairs, c.pairs / n);
     }
     const unsigned long long ns = c.survivors;
     const size_t n_rays = size_t(head.rays);
