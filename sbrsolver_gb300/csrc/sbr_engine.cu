@@ -235,11 +235,12 @@ struct Workspace {
   };
   std::array<Sizing, 64> sizing;
   // The set for a solve of `nodes`; a new one starts from the occupancy of the
-  // nearest within a factor of four.
+  // nearest within a factor of sixteen (with the defaults a first solve through
+  // slab walls ran twice, 4.1 instead of 2.5 ms).
   Sizing& sizing_for(double nodes) {
     const int k = std::min(63, std::max(0, int(std::log2(std::max(1.0, nodes)))));
     Sizing& z = sizing[size_t(k)];
-    for (int d : {1, -1, 2, -2}) {
+    for (int d : {1, -1, 2, -2, 3, -3, 4, -4}) {
       if (z.used || k + d < 0 || k + d > 63 || !sizing[size_t(k + d)].used) continue;
       const Sizing& o = sizing[size_t(k + d)];
       z.r_cls = o.r_cls;
