@@ -73,7 +73,17 @@ int main(int argc, char** argv) {
     if ((u >> 52 & 0x7ff) != 0x7ff) same_f(soft64::from_bits(u));
     same_tests(soft64::from_bits(rng()));
     same_tests(a);
+    const uint32_t f = uint32_t(rng());
+    float x;
+    std::memcpy(&x, &f, 4);
+    if (x == x) same("double of a float", soft64::from_f32(x), double(x));
+    const int k = int(rng() & 0x7fffffff) >> (rng() % 31);
+    same("double of a count", soft64::from_int(k), double(k));
   }
+  for (int k : {0, 1, 2, 3, 0x7fffffff, 0x7ffffffe, 0x40000000, 0x3fffffff})
+    same("double of a count", soft64::from_int(k), double(k));
+  for (float x : {0.0f, -0.0f, 1.0f, 1.17549435e-38f, 3.4028235e38f, 1e-45f, INFINITY})
+    same("double of a float", soft64::from_f32(x), double(x));
   for (double x : {0.0, -0.0, double(INFINITY), double(-INFINITY), double(NAN), -double(NAN), 1.0,
                    -1.0, 5e-324, -5e-324, 1.7e308, 1.1920928955078125e-07}) {
     same_tests(x);
