@@ -443,10 +443,10 @@ sbr_status sbr_fault_inject_alloc(long long after);
  * array's device address and must come before any stream capture.  A later
  * call on a stream that is being captured into a CUDA graph only enqueues its
  * kernels and returns SBR_OK: the host-side argument checks still apply, but
- * receiver indices outside [0, n_rx) and receivers over the per-receiver
- * limit are then skipped without a report (their fields stay zero).  Calls
- * share the array: calls (or graph launches) that overlap on the GPU race
- * and must be serialised by the caller. */
+ * paths whose receiver index lies outside [0, n_rx) are then left out and
+ * receivers over the per-receiver limit get a zero field, without a report.
+ * Calls share the array: calls (or graph launches) that overlap on the GPU
+ * race and must be serialised by the caller. */
 sbr_status sbr_receiver_field_sum_noalloc(const int* path_receiver, const long long* path_rank,
                                           const double* path_field, int n_paths, int n_rx,
                                           int field_precision, double* field_out,

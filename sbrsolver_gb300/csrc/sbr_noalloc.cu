@@ -128,7 +128,8 @@ struct Sum {
 // Receivers with at most kSmallRx paths, one warp each: every lane finds its
 // path's place among the others' (rank, path) by comparing with each, lays
 // its field down there, and six lanes add them up.  Larger ones are listed
-// for k_sum_large; more than kMaxPerRx raises an error flag.  (One thread per
+// for k_sum_large; more than kMaxPerRx give a zero field and raise an error
+// flag.  (One thread per
 // receiver, sorting by insertion through global memory, took 67 us for 20,011
 // receivers of 120,001 paths; this 14.)
 constexpr int kSumWarps = 8;
@@ -141,9 +142,11 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_sum(const long long* rank, c
   for (int r = blockIdx.x * kSumWarps + warp; r < n_rx; r += gridDim.x * kSumWarps) {
     const int n = s[kCounts + r], b = s[kCursor + r] - n;
     if (n > kSmallRx) {
-      if (lane == 0) {
-        if (n > kMaxPerRx) atomicOr(&s[kError], kErrPerRx);
-        else s[kLarge + atomicAdd(&s[kLargeCount], 1)] = r;
+      if (n > kMaxPerRx) {
+        if (lane < 6) out[6 * size_t(r) + lane] = 0.0;
+        if (lane == 0) atomicOr(&s[kError], kErrPerRx);
+      } else if (lane == 0) {
+        s[kLarge + atomicAdd(&s[kLargeCount], 1)] = r;
       }
       continue;
     }
@@ -324,9 +327,9 @@ sbr_status sbr_receiver_field_sum_noalloc(const int* path_receiver, const long l
   // While the stream is being captured into a CUDA graph the call only
   // enqueues its kernels: a capture admits neither the pageable read-back
   // nor the synchronisation (nor, in the global capture mode, queries beyond
-  // the capture status).  The kernels still skip out-of-range receivers and
-  // over-long receivers (those fields stay zero); their flags are not
-  // reported then.
+  // the capture status).  The kernels still leave paths of out-of-range
+  // receivers out and give over-long receivers a zero field; their flags are
+  // not reported then.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   {
     const cudaError_t e = cudaStreamIsCapturing(cs, &cap);
