@@ -1105,7 +1105,9 @@ static void device_prepare(const float* v_host, const float* n_host, int nt, cud
   next.ensure(max_nodes * 2 + 2);
   plans.ensure(max_nodes * 2 + 2);
   nodes.ensure(max_nodes);
-  DBuf<int> ctl;  // [0] nodes, [1] next segments, [2] max depth, [3] root ref, [4] median too big
+  // [0] nodes, [1] next segments, [2] the longest of them, [3] max depth, [4] root ref,
+  // [5] median too big
+  DBuf<int> ctl;
   ctl.ensure(8);
   DBuf<float> root_box;
   root_box.ensure(6);
@@ -1114,21 +1116,20 @@ static void device_prepare(const float* v_host, const float* n_host, int nt, cud
     const prep::Seg root{0, nt, 1, -1, 0};
     segs.upload(&root, 1, st);
   }
-  int n_segs = 1;
-  for (int level = 0; n_segs > 0; ++level) {
+  int level_segs[2] = {1, nt};  // segments, the longest one's triangles
+  for (int level = 0; level_segs[0] > 0; ++level) {
     if (level > 200) throw std::string("device search BVH deeper than 200 levels");
-    // a block per segment, as wide as the level's segments are long on average
-    const int per = nt / n_segs, threads = per > 2048 ? 1024 : (per > 128 ? 256 : 32);
+    const int n_segs = level_segs[0], threads = prep::segment_threads(nt / n_segs, level_segs[1]);
     prep::k_plan<<<n_segs, threads, 0, st>>>(segs.p, n_segs, ord.p, blo.p, bhi.p, cen.p, nodes.p,
-                                         ctl.p, plans.p, ctl.p + 2, ctl.p + 3, root_box.p);
+                                             ctl.p, plans.p, ctl.p + 3, ctl.p + 4, root_box.p);
     prep::k_partition<<<n_segs, threads, 0, st>>>(segs.p, n_segs, plans.p, ord.p, otmp.p, cen.p);
     prep::k_median<<<n_segs, threads, 0, st>>>(segs.p, n_segs, plans.p, ord.p, otmp.p, cen.p,
-                                           ctl.p + 4);
-    CK(cudaMemsetAsync(ctl.p + 1, 0, sizeof(int), st));
+                                               ctl.p + 5);
+    CK(cudaMemsetAsync(ctl.p + 1, 0, 2 * sizeof(int), st));
     prep::k_children<<<grid_for(n_segs, 256), 256, 0, st>>>(segs.p, n_segs, plans.p, next.p,
                                                             ctl.p + 1);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&n_segs, ctl.p + 1, sizeof n_segs, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(level_segs, ctl.p + 1, sizeof level_segs, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     swap_buf(segs, next);
   }
@@ -1148,17 +1149,17 @@ static void device_prepare(const float* v_host, const float* n_host, int nt, cud
   CK(cudaStreamSynchronize(st));
   CK(cudaMemcpy(&T.degenerate, misc.p, sizeof(int), cudaMemcpyDeviceToHost));
   T.search_ms = ms_since(t0);
-  if (c[4]) throw std::string("device search BVH: a median split of more than 8192 triangles");
+  if (c[5]) throw std::string("device search BVH: a median split of more than 8192 triangles");
   const int n_nodes = c[0];
   std::vector<prep::BNode> bn(size_t(std::max(1, n_nodes)));
   if (n_nodes)
     CK(cudaMemcpy(bn.data(), nodes.p, sizeof(prep::BNode) * n_nodes, cudaMemcpyDeviceToHost));
   T.search.order.resize(nt);
   CK(cudaMemcpy(T.search.order.data(), ord.p, sizeof(int) * nt, cudaMemcpyDeviceToHost));
-  T.search.max_depth = c[2];
+  T.search.max_depth = c[3];
   // depth-first numbering (node 0 = a copy of the root), children[0] first
   T.search.nodes.assign(size_t(n_nodes) + 1, SearchNode{});
-  const int root_ref = c[3];
+  const int root_ref = c[4];
   if (root_ref >= 0) {
     std::vector<int> dfs(size_t(n_nodes), -1);
     std::vector<int> stack{root_ref};
