@@ -113,14 +113,11 @@ SBR_HD bool same(double a, double b) { return bits(a) == bits(b); }
 
 SBR_HD double mul(double a, double b) {
   const uint64_t ua = bits(a), ub = bits(b);
-  const uint32_t ah = uint32_t(ua >> 32), al = uint32_t(ua);
-  const uint32_t bh = uint32_t(ub >> 32), bl = uint32_t(ub);
+  const uint32_t ah = uint32_t(ua >> 32), bh = uint32_t(ub >> 32);
   // a's 53 bits at the top of 64, b's shifted up by one: bits 64.. of the
   // product are the result's mantissa with 0 (c = 0) or 1 (c = 1) bit more
   const uint64_t A = (ua << 11) | (1ull << 63);
   const uint64_t B = ((ub << 1) & 0x001fffffffffffffull) | (1ull << 53);
-  (void)al;
-  (void)bl;
   const uint32_t a0 = uint32_t(A), a1 = uint32_t(A >> 32);
   const uint32_t b0 = uint32_t(B), b1 = uint32_t(B >> 32);
   const uint64_t p = uint64_t(a0) * b0;
@@ -151,8 +148,8 @@ SBR_HD uint64_t rcp_q63(uint64_t M) {
   const float r = seed_rcp(f32_bits(0x3f800000u | ((mh >> 8) & 0x7fffffu)));
   const uint32_t x0 = uint32_t(r * 2147483648.0f);  // Q31
   const uint64_t t0 = uint64_t(mh) * x0 + (uint64_t(ml) * x0 >> 32);  // m x0, Q62
-  const int64_t e0 = int64_t((1ull << 62) - t0);                      // |e0| < 2^-21
-  const uint64_t x1 = (uint64_t(x0) << 32) + uint64_t((int64_t(x0) * int32_t(e0 >> 10)) >> 20);
+  const int64_t e0 = int64_t((1ull << 62) - t0);  // |e0| < 2^-21: half of the 32 bits' range
+  const uint64_t x1 = (uint64_t(x0) << 32) + uint64_t((int64_t(x0) * int32_t(e0 >> 11)) >> 19);
   const int32_t e1 = int32_t((1ull << 62) - mulhi(M, x1));  // |e1| < 2^-41
   return x1 + uint64_t((int64_t(x1 >> 32) * e1) >> 30);
 }
@@ -204,7 +201,7 @@ SBR_HD double sqrt(double z) {
   const float f = f32_bits((0x3f800000u + (odd << 23)) | ((wh >> 8) & 0x7fffffu));
   const uint32_t x0 = uint32_t(seed_rsqrt(f) * 2147483648.0f);          // 1/sqrt(w), Q31
   const int64_t e0 = int64_t((1ull << 60) - mulhi(W, uint64_t(x0) * x0));  // 1 - w x0^2, Q60
-  const uint64_t x1 = (uint64_t(x0) << 32) + uint64_t((int64_t(x0) * int32_t(e0 >> 9)) >> 20);
+  const uint64_t x1 = (uint64_t(x0) << 32) + uint64_t((int64_t(x0) * int32_t(e0 >> 10)) >> 19);
   const uint64_t s1 = mulhi(W, x1);  // Q61
   const int32_t r = int32_t((W >> 4) - mulhi(s1, s1));  // w - s1^2, Q58
   const uint64_t s2 = s1 + uint64_t((int64_t(x1 >> 32) * r) >> 29);
