@@ -37,7 +37,6 @@ struct CaptureArgs {
   unsigned long long corr_cap;
   Counters* ctr;
   unsigned long long node_cap;
-  int stage_counts;
   uint2* pairs;                // (node, receiver | unsure << 31) for k_capture_finish
   unsigned long long pair_cap;
   HashTable corr_cache;        // (class, receiver) -> its image correction's outcome
@@ -114,7 +113,7 @@ __device__ __forceinline__ float sqrt_up(float x) {
 // image source img towards c crosses the class's last triangle T
 // (MultiPathCorrection's first test for a capture at c; RTSolver.cpp:356).
 // Three planes through img and T's edges, n_k . p >= n_k . img, formed once
-// per class in FP64 and rounded to FP32 (k_class_cones); k_capture loosens
+// per class in FP64 and rounded to FP32 (k_class_cones); k_capture_fast loosens
 // each by 2 m_k, m_k = 2^-21 |n_k| (cmax + |img| + |T| + 1).  The FP32 test
 // of a point p (|p| <= cmax) or of a cell corner errs by under
 // 10 * 2^-24 |n_k| (cmax + |img| + |T|): the plane's rounding, the rounding
@@ -292,15 +291,9 @@ __device__ __forceinline__ unsigned long long next_batch(unsigned long long* wor
   return __shfl_sync(0xffffffffu, base, 0);
 }
 
-// kStage: stage counts requested (every capture counted, the plain order of
-// tests); otherwise the fast path with the correction prefilter and the
-// deferred FP64 pass.
-// Resident blocks per SM of the fast path (register budget 65536 / (128 x this)).
-#ifndef SBR_CAP_BLOCKS
-#define SBR_CAP_BLOCKS 6
-#endif
-template <bool kStage>
-__global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k_capture(CaptureArgs A) {
+// The capture stage of solves that count its stages: every capture is counted,
+// in the plain order of tests (k_capture_fast serves all others).
+__global__ void __launch_bounds__(32 * kCapWarps, 4) k_capture(CaptureArgs A) {
   __shared__ AncRec anc[kCapWarps][kMaxDepth];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
@@ -308,14 +301,10 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
   const unsigned long long n_nodes = min(A.ctr->nodes, A.node_cap);
   unsigned long long events = 0, cand = 0, anc_tests = 0;
   unsigned n64 = 0;
-  // Nodes are taken 32 at a time: each lane loads one node's record, its
-  // class record and last triangle, so the three dependent loads are paid
-  // once per 32 nodes; the warp then works through the 32 from shared memory.
+  // Nodes are taken B at a time: each lane loads one node's record and forms its
+  // span; the warp then works through them from shared memory.
   constexpr int B = kCapBatch;
   __shared__ NodeHot s_nh[kCapWarps][B];
-  __shared__ Tri32 s_tl[kCapWarps][B];      // the class's last triangle
-  __shared__ float s_fl[kCapWarps][B][12];  // image source + correction filter terms
-  __shared__ float s_cn[kCapWarps][B][16];  // loosened correction cone
   __shared__ NodeSpan s_sp[kCapWarps][B];   // clipped span and chunking
   __shared__ ChunkBox s_ck[kCapWarps][B];   // the span's first chunk
   // Batches of B nodes are handed out by a work counter, one atomic per warp
@@ -328,32 +317,11 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
         const NodeHot h = A.nodes[my];
         s_nh[warp][lane] = h;
         const float cmax = A.gb[h.tx].cmax;
-        const int ar = A.grids[h.tx].ax[0];
-        int cone_ok = 0;
-        if (!is_root_class(h.cls)) {
-          const ClassCap c = A.cls_cap[h.cls];
-          s_tl[warp][lane] = A.sc.corr32[c.tpos];
-          float* fl = s_fl[warp][lane];
-          for (int q = 0; q < 3; ++q) fl[q] = c.img[q];
-          for (int q = 0; q < 8; ++q) fl[3 + q] = c.F[q];
-          // the cone's planes loosened by 2 m, m = 2^-21 |n| (cmax + |img| + |T| + 1)
-          float* cn = s_cn[warp][lane];
-          cone_ok = !kStage;
-          for (int k = 0; k < 3; ++k) {
-            const float m = kConeK * (c.nn[k] * cmax + c.w[k]);
-            cone_ok &= (c.gc[k] > 0.0f && isfinite(m)) ? 1 : 0;
-            cn[4 * k + 0] = c.n[k][0];
-            cn[4 * k + 1] = c.n[k][1];
-            cn[4 * k + 2] = c.n[k][2];
-            cn[4 * k + 3] = c.n[k][3] - 2.0f * m;
-            cn[12 + k] = 1.0f / (ar == 0 ? c.n[k][0] : (ar == 1 ? c.n[k][1] : c.n[k][2]));
-          }
-        }
-        const NodeSpan sp = node_span(h, A.grids[h.tx], cone_ok);
+        const NodeSpan sp = node_span(h, A.grids[h.tx], 0);
         s_sp[warp][lane] = sp;
         if (sp.nchunk > 0)
           s_ck[warp][lane] = chunk_box(h, A.grids[h.tx], sp, 0, cmax, A.txp[h.tx].tan_beta32,
-                                       cone_ok != 0, s_cn[warp][lane]);
+                                       false, nullptr);
       }
       __syncwarp();
     }
@@ -375,11 +343,9 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
       const float ur = sn.u[ar], um = sn.u[am], ul = sn.u[al];
       const float inv_um = __frcp_rn(um), inv_ul = __frcp_rn(ul);
       const float inv_cell = g.inv_cell;
-      // Stage the ancestor chain when every capture is checked against it
-      // (stage counts); otherwise only corrected captures (~0.1% of captures)
-      // need it and they walk the chain themselves.
+      // Stage the ancestor chain: every capture is checked against it.
       int na = 0;
-      if (kStage && lane == 0) {
+      if (lane == 0) {
         for (uint32_t p = nd.parent; p != 0xFFFFFFFFu && p < A.node_cap && na < kMaxDepth;) {
           const NodeHot a = A.nodes[p];
           AncRec& r = anc[warp][na++];
@@ -391,24 +357,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
       }
       na = __shfl_sync(FULL, na, 0);
       __syncwarp();
-      // Image correction of this node's class must first cross the triangle
-      // the last ray reflected or passed on (MultiPathCorrection's last step):
-      // an FP32 filter from the class's image source towards each receiver
-      // rejects ~99.9% of receivers before the reception test.  Stage counts
-      // need every capture, so they keep the reception test first.
-      const bool root = is_root_class(nd.cls);
-      Tri32 Tl;
-      TriFrom Fl;
-      float3 img = make_float3(0.0f, 0.0f, 0.0f);
       const NodeSpan sp = s_sp[warp][jj];
-      const bool use_cone = sp.use_cone != 0;
-      const float* cone_w = s_cn[warp][jj];
-      if (!root) {
-        const float* fl = s_fl[warp][jj];
-        img = make_float3(fl[0], fl[1], fl[2]);
-        Tl = s_tl[warp][jj];
-        Fl = TriFrom{fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10]};
-      }
       if (sp.nchunk > 0) {
         const float tanb = P.tan_beta32;
         const float cmax = A.gb[nd.tx].cmax;
@@ -419,7 +368,7 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
         {
           for (int ch = 0; ch < nchunk; ++ch) {
             if (ch > 0) {  // every lane forms the same box
-              const ChunkBox next = chunk_box(nd, g, sp, ch, cmax, tanb, use_cone, cone_w);
+              const ChunkBox next = chunk_box(nd, g, sp, ch, cmax, tanb, false, nullptr);
               __syncwarp();
               if (lane == 0) s_ck[warp][jj] = next;
               __syncwarp();
@@ -459,8 +408,6 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
                   const float xa = sr + la * ur, xb = sr + lb * ur;
                   int x0 = max(cb.c0[ar], int(floorf((fminf(xa, xb) - rb - g.org[ar]) * inv_cell)));
                   int x1 = min(cb.c1[ar], int(floorf((fmaxf(xa, xb) + rb - g.org[ar]) * inv_cell)));
-                  if (use_cone && x0 <= x1)
-                    cone_cells(cone_w, g, inv_cell, im, il, x0, x1);
                   if (x0 <= x1) {
                     const int row = (il * g.dim[am] + im) * g.dim[ar];
                     beg = g.cell_start[row + x0];
@@ -497,16 +444,6 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
                 const int gi = __float_as_int(c4.w);
                 const double* c64 = A.rx + 3 * size_t(gi);
                 ++cand;
-                if (!kStage) {
-                  if (root) {
-                    if (!A.direct_ok[gi]) continue;
-                  } else {
-                    const float3 dd = make_float3(c.x - img.x, c.y - img.y, c.z - img.z);
-                    if (!tri_filter_from(Tl, Fl, dd,
-                                         sqrt_up(dd.x * dd.x + dd.y * dd.y + dd.z * dd.z)))
-                      continue;
-                  }
-                }
                 int v;
                 if (lam < a || lam > b) {
                   // outside the chunk's own range: full-margin test
@@ -525,18 +462,6 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
                   const float rh = rad + mr, rl2 = rad - mr;
                   v = d2 > rh * rh ? 0 : ((rl2 > 0.0f && d2 < rl2 * rl2) ? 1 : -1);
                 }
-                if (!kStage) {
-                  // everything after the FP32 tests (exact reception test,
-                  // image correction, ancestor suppression) runs densely in
-                  // k_capture_finish
-                  if (v == 0) continue;
-                  const unsigned long long slot = warp_reserve(&A.ctr->pairs, 1);
-                  if (slot < A.pair_cap)
-                    A.pairs[slot] = make_uint2(uint32_t(i), uint32_t(gi) | (v < 0 ? 0x80000000u : 0u));
-                  else
-                    atomicOr(&A.ctr->overflow, kOvPairs);
-                  continue;
-                }
                 if (v < 0) {
                   ++n64;
                   v = capture_exact(A.nodes_cold, uint32_t(i), c64, P.tan_beta);
@@ -545,44 +470,25 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
                 // RayCapture deletes a captured node's subtree, so an ancestor
                 // capturing the same receiver suppresses this one.
                 auto suppressed = [&]() {
-                  if constexpr (kStage) {
-                    for (int q = 0; q < na; ++q) {
-                      const AncRec& r = anc[warp][q];
-                      ++anc_tests;
-                      int w = reception32(make_float3(r.s[0], r.s[1], r.s[2]),
-                                          make_float3(r.u[0], r.u[1], r.u[2]), r.len, r.S, c, tanb);
-                      if (w < 0) {
-                        ++n64;
-                        w = capture_exact(A.nodes_cold, r.idx, c64, P.tan_beta);
-                      }
-                      if (w) return true;
+                  for (int q = 0; q < na; ++q) {
+                    const AncRec& r = anc[warp][q];
+                    ++anc_tests;
+                    int w = reception32(make_float3(r.s[0], r.s[1], r.s[2]),
+                                        make_float3(r.u[0], r.u[1], r.u[2]), r.len, r.S, c, tanb);
+                    if (w < 0) {
+                      ++n64;
+                      w = capture_exact(A.nodes_cold, r.idx, c64, P.tan_beta);
                     }
-                    return false;
-                  } else {
-                    for (uint32_t p = nd.parent; p != 0xFFFFFFFFu && p < A.node_cap;) {
-                      const NodeHot a = A.nodes[p];
-                      ++anc_tests;
-                      int w = reception32(make_float3(a.s[0], a.s[1], a.s[2]),
-                                          make_float3(a.u[0], a.u[1], a.u[2]), a.len, a.S, c, tanb);
-                      if (w < 0) {
-                        ++n64;
-                        w = capture_exact(A.nodes_cold, p, c64, P.tan_beta);
-                      }
-                      if (w) return true;
-                      p = a.parent;
-                    }
-                    return false;
+                    if (w) return true;
                   }
+                  return false;
                 };
-                if (kStage) {
-                  if (suppressed()) continue;
-                  ++events;
-                }
+                if (suppressed()) continue;
+                ++events;
                 const bool ok = is_root_class(nd.cls)
                                     ? A.direct_ok[gi] != 0
                                     : correct_event(A.sc, A.cls_info, nd.cls, c, c64, n64);
                 if (!ok) continue;
-                if (!kStage && suppressed()) continue;
                 const unsigned long long kk = atomicAdd(&A.ctr->corrected, 1ull);
                 if (kk < A.corr_cap)
                   A.corr_list[kk] = Corrected{uint32_t(gi), nd.cls,
@@ -614,12 +520,11 @@ __global__ void __launch_bounds__(32 * kCapWarps, kStage ? 4 : SBR_CAP_BLOCKS) k
 
 // Items of a work counter handed to a warp, a window at a time: every warp of
 // the grid asks the same counter, which serves an atomic in about 0.65 ns, so
-// a warp takes a part of what was left when it last asked (at least
-// `smallest`, a multiple of 32) and the windows shrink
-// towards the end, where an uneven last one would leave warps waiting.  At
-// most 64 items: costly nodes lie next to each other, and a warp that drew
-// 256 of them held up the level-10 terrain's capture (12.2 ms; 128: 8.0,
-// 64 and 32: 7.1).
+// a warp takes a part of what was left when it last asked (whole batches of 32,
+// or `smallest`, a caller's smaller batch) and the windows shrink towards the
+// end, where an uneven last one would leave warps waiting.  At most 64 items:
+// costly nodes lie next to each other, and a warp that drew 256 of them held up
+// the level-10 terrain's capture (12.2 ms; 128: 8.0, 64 and 32: 7.1).
 struct WorkWindow {
   unsigned long long* counter;
   long long next, end, n;  // the window's rest; items in all
@@ -645,8 +550,11 @@ struct WorkWindow {
 
 // ---- fast path, flattened over the nodes of a batch ------------------------
 //
-// The same tests as k_capture's fast path with the same chunks, cell boxes
-// and margins, so the same (node, receiver) pairs reach k_capture_finish.
+// Receivers are found as k_capture finds them (chunks, cell boxes, margins), but
+// the correction's first test comes before the reception test: the line from the
+// class's image source to the receiver must cross the class's last triangle, which
+// an FP32 filter refutes for ~99.9 % of receivers, and the loosened cone for whole
+// rows of cells.  The (node, receiver) pairs left go to k_capture_finish.
 // The warp stages B nodes (one lane each: node record, class record, last
 // triangle, loosened correction cone, clipped span), then works through the
 // whole batch at three flattened levels instead of node by node: the batch's
@@ -686,7 +594,7 @@ struct StagedNode {
 
 // The correction prefilter of a node's class as a candidate needs it: the image
 // source, the last triangle's edges, tri_from's terms and the margins' factors
-// (tri_filter_from's, the ones that depend on the class alone multiplied
+// (tri_filter's, the ones that depend on the class alone multiplied
 // beforehand).  Five 16-byte loads a candidate instead of 23 words of two
 // records, and the cones an odd number of words apart: the kernel is bound by
 // issue and L1 (level-9 canyon 5.05 -> 4.89 ms, 24 requests 2.53 -> 2.45, level-10
@@ -713,7 +621,7 @@ __device__ __forceinline__ LineFilter line_filter(const ClassCap& c, const Tri32
   L.kw = kCorrK * ns * T.ne1 * T.ne2;
   return L;
 }
-// tri_filter_from of the line from the image source to c.
+// tri_filter of the line from the image source to c, without its bound on t.
 __device__ __forceinline__ bool line_may_cross(const LineFilter& L, const float3& c) {
   const float dx = c.x - L.img[0], dy = c.y - L.img[1], dz = c.z - L.img[2];
   const float nd = sqrt_up(dx * dx + dy * dy + dz * dz);
@@ -747,6 +655,10 @@ __device__ __forceinline__ void flush_pairs(const CaptureArgs& A, const uint2* b
   __syncwarp();
 }
 
+// Resident blocks per SM (register budget 65536 / (128 x this)).
+#ifndef SBR_CAP_BLOCKS
+#define SBR_CAP_BLOCKS 6
+#endif
 __global__ void __launch_bounds__(32 * kCapWarps, SBR_CAP_BLOCKS) k_capture_fast(CaptureArgs A) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;

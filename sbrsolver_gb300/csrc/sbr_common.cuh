@@ -14,22 +14,6 @@ namespace sbr {
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
-// Warp-aggregated slot reservation: every active lane asks for `cnt` (0..2)
-// entries; one atomicAdd per warp.
-__device__ __forceinline__ unsigned long long warp_reserve(unsigned long long* ctr, unsigned cnt) {
-  const unsigned mask = __activemask();
-  const unsigned b1 = __ballot_sync(mask, cnt >= 1);
-  const unsigned b2 = __ballot_sync(mask, cnt >= 2);
-  const unsigned lt = (1u << lane_id()) - 1u;
-  const unsigned before = __popc(b1 & lt) + __popc(b2 & lt);
-  const unsigned total = __popc(b1) + __popc(b2);
-  const int leader = __ffs(mask) - 1;
-  unsigned long long base = 0;
-  if (lane_id() == unsigned(leader) && total) base = atomicAdd(ctr, (unsigned long long)total);
-  base = __shfl_sync(mask, base, leader);
-  return base + before;
-}
-
 // Open addressing with linear probing.  Tables are kept at most half full
 // (the host grows them between solves from the occupancy counters), so a
 // probe run longer than kMaxProbe means the table is too small: the insert

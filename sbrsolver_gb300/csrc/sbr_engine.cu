@@ -1803,7 +1803,6 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     ca.corr_cap = Z.cap_corr;
     ca.ctr = W.ctr.p;
     ca.node_cap = Z.cap_nodes;
-    ca.stage_counts = stage_counts;
     ca.pairs = W.pairs.p;
     ca.pair_cap = Z.cap_pairs;
     ca.corr_cache = HashTable{W.cc_keys.p, Z.cap_cc - 1};
@@ -1812,7 +1811,7 @@ static void solve_impl(SceneImpl& S, Workspace& W, const sbr_request* reqs, int 
     CK(cudaStreamWaitEvent(st, W.join, 0));
     mark(W.cap_ev[0]);
     if (stage_counts) {
-      ++nl, k_capture<true><<<capture_grid(tu), 32 * kCapWarps, 0, st>>>(ca);
+      ++nl, k_capture<<<capture_grid(tu), 32 * kCapWarps, 0, st>>>(ca);
       mark(W.cap_ev[1]);
     } else {
       ++nl, k_capture_fast<<<capture_grid(tu), 32 * kCapWarps, 0, st>>>(ca);

@@ -267,9 +267,8 @@ __device__ __forceinline__ bool tri_filter(const Tri32& T, const float3& o, cons
   return true;
 }
 
-// tri_filter for many rays from one origin o (an image source towards many
-// receivers): the terms that depend only on o and the triangle are formed
-// once.  Same arithmetic and margins as tri_filter.
+// tri_filter's terms that depend only on the origin o and the triangle, for many
+// rays from one image source towards many receivers (line_may_cross).
 struct TriFrom {
   float sx, sy, sz;  // o - v1
   float qx, qy, qz;  // (o - v1) x e1
@@ -288,33 +287,6 @@ __device__ __forceinline__ TriFrom tri_from(const Tri32& T, const float3& o, flo
   F.W = T.e2[0] * F.qx + T.e2[1] * F.qy + T.e2[2] * F.qz;
   F.ns = no + T.nv1;
   return F;
-}
-
-__device__ __forceinline__ bool tri_filter_from(const Tri32& T, const TriFrom& F,
-                                                const float3& d, float nd) {
-  const float hx = d.y * T.e2[2] - d.z * T.e2[1];
-  const float hy = d.z * T.e2[0] - d.x * T.e2[2];
-  const float hz = d.x * T.e2[1] - d.y * T.e2[0];
-  const float a = T.e1[0] * hx + T.e1[1] * hy + T.e1[2] * hz;
-  float U = F.sx * hx + F.sy * hy + F.sz * hz;
-  float V = d.x * F.qx + d.y * F.qy + d.z * F.qz;
-  float W = F.W;
-  const float ea = kCorrK * T.ne1 * T.ne2 * nd;
-  const float eU = kCorrK * F.ns * nd * T.ne2;
-  const float eV = kCorrK * F.ns * T.ne1 * nd;
-  const float eW = kCorrK * F.ns * T.ne1 * T.ne2;
-  const float A = fabsf(a);
-  if (A <= kEps32 + ea) return true;  // near-parallel: the FP64 test decides
-  if (a < 0.0f) {
-    U = -U;
-    V = -V;
-    W = -W;
-  }
-  if (U < -eU || V < -eV) return false;
-  if (U > A + ea + eU) return false;
-  if (U + V > A + ea + eU + eV) return false;
-  // thi = (W + eW) / (A - ea) > eps/2 with A - ea > 0, without the division
-  return W + eW > (kEps32 * 0.5f) * (A - ea);
 }
 
 // As tri_filter, also telling what the FP64 test certainly decides: 0 = it
