@@ -106,8 +106,8 @@ __device__ __forceinline__ void cross64(const double* a, const double* b, double
 
 // Triangle::RayIntersects (Triangle.cpp:80-124), FP64, reference operation
 // order.  uv_sure: the FP32 filter has shown that the reference's tests of u
-// and v accept (tri_classify), so they are not formed.  No early exit: a lane
-// that fails costs its warp nothing more, and the warp stays together.
+// and v accept (tri_classify), so they are not formed.  It returns early
+// for a parallel ray, for u and v together (formed side by side) and for t.
 // Comparisons are integer ones, which decide alike without the FP64 pipe.
 template <class A>
 __device__ __forceinline__ bool mt64_t(const Tri64& T, const double* o, const double* d,

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256)
     d.id = s.id;
     d.cop = s.cop;
     d.mat = s.mat;
-    d.node = -1;  // k_leaf_of
+    d.node = -1;  // its leaf: k_ref_nodes
     t32[r] = filter_copy(s.v1, e1, e2);
     cop[r] = s.cop;
     rank_to_id[r] = s.id;
